@@ -14,6 +14,7 @@
 #include <string>
 #include <unordered_map>
 #include <unordered_set>
+#include <queue>
 #include <vector>
 
 #include "lc_internal.cuh"
@@ -61,10 +62,10 @@ struct ClusterArgs {
     int chunk_cap;
     int contact_gather;      // scatter solver: contacts gathered per owned vertex (no remote atomics)
 };
-cudaError_t launch_solve_cluster(const DevPtrs &d, const ClusterArgs &a, int cs, bool scatter, int nclusters,
+cudaError_t launch_solve_cluster(const DevPtrs &d, const ClusterArgs &a, int cs, int bs, bool scatter, int nclusters,
                                  cudaStream_t st);
 int cluster_chunk_cap(bool scatter);
-int cluster_max_active(int cs, int chunk_cap, bool scatter);
+int cluster_max_active(int cs, int bs, int chunk_cap, bool scatter);
 }  // namespace lc
 
 using namespace lc;
@@ -349,6 +350,7 @@ struct lc_batch {
     // cluster-resident solver (lc_cluster.cu)
     bool use_cluster = false;
     int cluster_cs = 8;
+    int cluster_bs = 512;  // threads per CTA of the on-chip solvers
     int want_cs = 0;  // 0: pick; 4, 8 or 16: requested through lc_batch_set_tuning
     bool cluster_scatter = false;
     ClusterArgs ca{};
@@ -554,13 +556,46 @@ static lc_status enqueue_cluster_solver(lc_batch *b, cudaStream_t st) {
         d.dbg_sphere = nullptr;
         d.coll_act = nullptr;
     }
-    LC_CUDA(launch_solve_cluster(d, b->ca, b->cluster_cs, b->cluster_scatter, b->C, st));
+    LC_CUDA(launch_solve_cluster(d, b->ca, b->cluster_cs, b->cluster_bs, b->cluster_scatter, b->C, st));
     return LC_OK;
 }
 
 template <class T> static lc_status upload(T *dst, const std::vector<T> &src) {
     if (!src.empty()) LC_CUDA(cudaMemcpy(dst, src.data(), sizeof(T) * src.size(), cudaMemcpyHostToDevice));
     return LC_OK;
+}
+
+// Estimated time of one launch of the on-chip solver (us, 10 iterations):
+// clusters of cs CTAs of bs threads, act of them resident, taking the cloths
+// largest first.  One cluster's time is a latency floor plus its vertices per
+// CTA times a rate, fitted on one contact-free cloth per launch: 512 threads
+// 31, 33, 57, 104 and 332 us at 16, 36, 256, 638 and 2304 vertices per CTA,
+// 1024 threads 33, 35, 47, 80 and 244 us.  Two 512-thread CTAs on an SM share
+// its issue slots, so their rate is that of one of 1024 threads.  A cloth in
+// contact takes 1.5 to 2.5 times as long, and the launch waits for the largest
+// one: its time once and a half is added.  Estimates are within a tenth of
+// the measured times of flat batches.  So one 101x101
+// cloth takes 16 CTAs of 1024 threads (78 us, where 4 CTAs of 512 take 321),
+// 64 cloths of side 16..192 16 of 512 (1.32 ms, a third of them folded; 8 CTAs
+// 2.3) and 128 of side 16..32 small clusters (0.14 ms with 4 CTAs, 0.46 with 16).
+static double estimate_solve(const lc_batch &b, const std::vector<int> &largest_first, int cs, int bs, int act) {
+    const int n = (int)largest_first.size(), slots = std::min(act, n);
+    const bool shared = bs == kSolveSmallBlock && slots * cs > sm_count();
+    const double base = bs == kSolveSmallBlock ? 29.0 : 31.0, own = bs == kSolveSmallBlock ? 0.125 : 0.09;
+    const double rate = shared ? 0.18 : own;
+    auto per_cta = [&](int k) { return (double)cluster_chunk(b.hosts[largest_first[k]].V, cs); };
+    std::priority_queue<double, std::vector<double>, std::greater<double>> busy;  // when each slot is free again
+    double end = 0;
+    for (int k = 0; k < n; ++k) {
+        double t = base + rate * per_cta(k);
+        if (k >= slots) {
+            t += busy.top();
+            busy.pop();
+        }
+        busy.push(t);
+        end = std::max(end, t);
+    }
+    return end + 1.5 * own * per_cta(0);
 }
 
 // Cluster-resident solver: picks the cluster size for the largest cloth and
@@ -579,18 +614,28 @@ lc_status lc_batch::setup_cluster() {
         vmax = std::max(vmax, hosts[c].V);
         if (cds[c].F > 8) ok = false;
     }
-    // cluster size: the requested one (lc_tuning.cluster_size) if it fits,
-    // else the one that keeps the most CTAs resident (more warps per SM to
-    // hide the distributed-shared-memory latency), 8 on a tie
-    int cs = 0;
+    std::vector<int> order(C);
+    for (int c = 0; c < C; ++c) order[c] = c;
+    std::stable_sort(order.begin(), order.end(), [&](int x, int y) { return hosts[x].V > hosts[y].V; });
+    // Cluster size (the requested lc_tuning.cluster_size if it fits) and
+    // threads per CTA: the pair with the shortest estimated launch.
+    int cs = 0, bs = kSolveSmallBlock;
     if (ok) {
-        long best = 0;
+        double best = 0;
         for (int cand : {8, 16, 4}) {
             if (want_cs && cand != want_cs) continue;
-            const int cap = (vmax + cand - 1) / cand;
+            const int cap = cluster_chunk(vmax, cand);
             if (cap > dev_cap) continue;
-            const long act = (long)cluster_max_active(cand, cap, scatter) * cand;
-            if (act > best) { best = act; cs = cand; }
+            for (int block : {kSolveSmallBlock, kSolveLargeBlock}) {
+                if (!scatter && block != kSolveSmallBlock) continue;
+                const int act = cluster_max_active(cand, block, cap, scatter);
+                // large blocks only where every cloth's cluster is resident at
+                // once: a second wave waits for whole SMs, and beside other
+                // kernels (the batches of a group) the first one does too
+                if (act < (block == kSolveLargeBlock ? C : 1)) continue;
+                const double t = estimate_solve(*this, order, cand, block, act);
+                if (!cs || t < best) { best = t; cs = cand; bs = block; }
+            }
         }
     }
     if (!cs) {
@@ -598,16 +643,14 @@ lc_status lc_batch::setup_cluster() {
         return LC_OK;
     }
     cluster_cs = cs;
+    cluster_bs = bs;
     cluster_scatter = scatter;
-    std::vector<int> order(C);
-    for (int c = 0; c < C; ++c) order[c] = c;
-    std::stable_sort(order.begin(), order.end(), [&](int x, int y) { return hosts[x].V > hosts[y].V; });
     int *clc;
     LC_TRY(arena.alloc(clc, C, "cl_cloth"));
     LC_TRY(upload(clc, order));
     ca.cl_cloth = clc;
     ca.nvf = nvf;
-    ca.chunk_cap = (vmax + cs - 1) / cs;
+    ca.chunk_cap = cluster_chunk(vmax, cs);
     use_cluster = true;
     return LC_OK;
 }

@@ -24,8 +24,6 @@ namespace cg = cooperative_groups;
 
 namespace lc {
 
-constexpr int kClusterBlock = 512;
-
 // Shared memory per vertex: two position buffers (32) + ground plane height
 // (4) + LRA flags (1).
 constexpr int kClusterBytesPerVertex = 37;
@@ -51,13 +49,13 @@ __device__ __forceinline__ void record_tail(const DevPtrs &d, const ClothDev &cd
 }
 
 template <int CS>
-__global__ void __launch_bounds__(kClusterBlock, 1) k_solve_cluster(DevPtrs d, ClusterArgs a) {
+__global__ void __launch_bounds__(kSolveSmallBlock, 1) k_solve_cluster(DevPtrs d, ClusterArgs a) {
     cg::cluster_group cluster = cg::this_cluster();
     const int r = (int)cluster.block_rank();
     const int c = a.cl_cloth[blockIdx.x / CS];
     const ClothDev &cd = d.cloth[c];
     const int V = cd.V, vo = cd.v_off;
-    const int chunk = (V + CS - 1) / CS;
+    const int chunk = cluster_chunk(V, CS);
     const int lo = r * chunk;
     const int n_own = max(0, min(V, lo + chunk) - lo);
     const int tid = threadIdx.x, bs = blockDim.x;
@@ -302,17 +300,55 @@ constexpr int kScatterBytesPerVertex = 37;
 constexpr float kFix = 33554432.f;           // 2^25
 constexpr float kFixInv = 1.f / 33554432.f;  // exact power of two
 
-template <int CS>
-__global__ void __launch_bounds__(kClusterBlock, 2) k_solve_cluster_scatter(DevPtrs d, ClusterArgs a) {
+// Distributed shared memory by 32-bit cluster addresses: `map_cluster` turns
+// an address of this CTA's shared memory into CTA o's.
+__device__ __forceinline__ uint32_t smem_addr(const void *p) { return (uint32_t)__cvta_generic_to_shared(p); }
+__device__ __forceinline__ uint32_t map_cluster(uint32_t addr, int o) {
+    uint32_t a;
+    asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"(addr), "r"(o));
+    return a;
+}
+__device__ __forceinline__ float4 ld_cluster(uint32_t addr) {
+    float4 v;
+    asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];"
+                 : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(addr) : "memory");
+    return v;
+}
+__device__ __forceinline__ void red_cluster(uint32_t addr, unsigned long long v) {
+    asm volatile("red.relaxed.cluster.shared::cluster.add.u64 [%0], %1;" : : "r"(addr), "l"(v) : "memory");
+}
+
+// What bounds it: the latency of an iteration's chain (remote positions, the
+// bend's arithmetic, the atomics' completion, two cluster barriers: 3 us an
+// iteration however small the cloth), then issue slots for the bends and, with
+// contacts, the remote atomics.  So positions and sums go by 32-bit cluster
+// addresses without a branch on the owner (a branch per vertex made a lane
+// wait for one remote load before the next was issued), what an iteration
+// reads from global memory through the same thread each time is kept in
+// registers, and a CTA has 1024 threads where it has an SM to itself.  One
+// flat 101x101 cloth, 16 CTAs: 119 us before, 104 with 512 threads, 78 with
+// 1024; 64 cloths of side 16..192, a third folded: 1.43 before, 1.32 ms.
+// 32-bit atomics on the CTA's own vertices were 10% faster without contacts
+// and 40% slower with them (four remote ones a correction instead of two);
+// contact corrections written to per-vertex lists in global memory and summed
+// by the owners were 15% faster on a full chip and 50% slower on one large
+// folded cloth; contacts before the other constraints were 7% slower.
+template <int CS, int BS>
+__global__ void __launch_bounds__(BS, kSolveLargeBlock / BS) k_solve_cluster_scatter(DevPtrs d, ClusterArgs a) {
     cg::cluster_group cluster = cg::this_cluster();
     const int r = (int)cluster.block_rank();
     const int c = a.cl_cloth[blockIdx.x / CS];
     const ClothDev &cd = d.cloth[c];
-    const int V = cd.V, vo = cd.v_off;
-    const int chunk = (V + CS - 1) / CS;
+    // the fields the iterations read, once: a cluster barrier makes every
+    // later global load go back to L2
+    const int V = cd.V, vo = cd.v_off, F = cd.F, iters = cd.iters, tri_bend = cd.tri_bend;
+    const float h = cd.h;
+    const int64_t lra_off = cd.lra_off;
+    const int chunk = cluster_chunk(V, CS);
     const int lo = r * chunk;
     const int n_own = max(0, min(V, lo + chunk) - lo);
-    const int tid = threadIdx.x, bs = blockDim.x;
+    const int tid = threadIdx.x;
+    constexpr int bs = BS;
     const int cap = a.chunk_cap;
     extern __shared__ float4 smem4[];
     float4 *xs = smem4;
@@ -320,23 +356,24 @@ __global__ void __launch_bounds__(kClusterBlock, 2) k_solve_cluster_scatter(DevP
     unsigned long long *ayz = axc + cap;
     float *gq = reinterpret_cast<float *>(ayz + cap);
     uint8_t *lra = reinterpret_cast<uint8_t *>(gq + cap);
+    __shared__ int s_fixed[8];
     const uint32_t magic = (uint32_t)((0x100000000ull + chunk - 1) / chunk);
+    const uint32_t xs_s = smem_addr(xs), axc_s = smem_addr(axc);
     auto owner = [&](int li) { return (int)__umulhi((uint32_t)li, magic); };
     auto X = [&](int li) -> float4 {
         const int o = owner(li);
-        if (o == r) return xs[li - lo];
-        return cluster.map_shared_rank(xs, o)[li - o * chunk];
+        return ld_cluster(map_cluster(xs_s, o) + 16u * (uint32_t)(li - o * chunk));
     };
-    auto add_corr = [&](int li, float3 v, bool count) {
+    auto add_fixed = [&](int li, int ix, int iy, int iz, uint32_t count) {
         const int o = owner(li);
-        const int k = li - o * chunk;
-        unsigned long long *pxc = o == r ? axc : cluster.map_shared_rank(axc, o);
-        unsigned long long *pyz = o == r ? ayz : cluster.map_shared_rank(ayz, o);
-        const int ix = __float2int_rn(v.x * kFix), iy = __float2int_rn(v.y * kFix), iz = __float2int_rn(v.z * kFix);
-        atomicAdd(pxc + k, ((unsigned long long)(uint32_t)ix << 32) + (count ? 1ull : 0ull));
-        atomicAdd(pyz + k, ((unsigned long long)(uint32_t)iy << 32) + (unsigned long long)(long long)iz);
+        const uint32_t p = map_cluster(axc_s, o) + 8u * (uint32_t)(li - o * chunk);
+        red_cluster(p, ((unsigned long long)(uint32_t)ix << 32) + count);
+        red_cluster(p + 8u * cap, ((unsigned long long)(uint32_t)iy << 32) + (unsigned long long)(long long)iz);
     };
+    auto fix = [](float v) { return __float2int_rn(v * kFix); };
+    auto add_corr = [&](int li, float3 v, bool count) { add_fixed(li, fix(v.x), fix(v.y), fix(v.z), count ? 1u : 0u); };
     const float qnan = __int_as_float(0x7fc00000);
+    if (tid < min(F, 8)) s_fixed[tid] = d.fixed[cd.f_off + tid] - vo;
     for (int i = tid; i < n_own; i += bs) {
         const int g = vo + lo + i;
         const float4 x4 = d.x[g];
@@ -345,10 +382,10 @@ __global__ void __launch_bounds__(kClusterBlock, 2) k_solve_cluster_scatter(DevP
         lra[i] = 0;
         float q = qnan;
         float4 qdbg = make_float4(0.f, 0.f, 0.f, 0.f);
-        if (cd.ground_on && x4.y <= cd.ground_y + cd.h) {
+        if (cd.ground_on && x4.y <= cd.ground_y + h) {
             const float3 pos = xyz(x4);
             const float3 nc = f3(0.f, 1.f, 0.f);
-            const float3 p0 = f3(1.f, cd.ground_y + cd.h, 1.f);
+            const float3 p0 = f3(1.f, cd.ground_y + h, 1.f);
             const float3 l = sub(pos, xyz(d.xp[g]));
             const float dd = dot(sub(p0, pos), nc) / dot(l, nc);
             const float3 qc = add(mul(l, dd), pos);
@@ -359,23 +396,23 @@ __global__ void __launch_bounds__(kClusterBlock, 2) k_solve_cluster_scatter(DevP
         if (d.dbg_ground_it || d.friction_any) d.ground_qc[g] = qdbg;
     }
     cluster.sync();
-    if (cd.F) {
+    if (F) {
         for (int i = tid; i < n_own; i += bs) {
             const float4 x4 = xs[i];
             uint8_t f = 0;
-            const int64_t base = cd.lra_off + (int64_t)(lo + i) * cd.F;
+            const int64_t base = lra_off + (int64_t)(lo + i) * F;
             if (x4.w != 0.f)
-                for (int j = 0; j < cd.F; ++j)
-                    if (dist(xyz(x4), xyz(X(d.fixed[cd.f_off + j] - vo))) > d.lra_l0[base + j]) f |= (uint8_t)(1u << j);
+                for (int j = 0; j < F; ++j)
+                    if (pin::len(pin::sub(xyz(x4), xyz(X(s_fixed[j])))) > d.lra_l0[base + j]) f |= (uint8_t)(1u << j);
             lra[i] = f;
             if (d.dbg_ground_it)
-                for (int j = 0; j < cd.F; ++j) d.lra_flag[base + j] = (f >> j) & 1u;
+                for (int j = 0; j < F; ++j) d.lra_flag[base + j] = (f >> j) & 1u;
         }
         cluster.sync();
     }
     if (cd.sphere_on) {
         const float3 sc = f3(cd.sphere_pos[0], cd.sphere_pos[1], cd.sphere_pos[2]);
-        const float rad = cd.sphere_r + cd.h;
+        const float rad = cd.sphere_r + h;
         for (int i = tid; i < n_own; i += bs) {
             const int g = vo + lo + i;
             const float4 x4 = xs[i], p4 = d.xp[g];
@@ -383,54 +420,94 @@ __global__ void __launch_bounds__(kClusterBlock, 2) k_solve_cluster_scatter(DevP
             int ret = 0;
             float3 q = f3(0.f, 0.f, 0.f);
             if (!is_zero(dir)) {
-                const float l = len(dir);
+                const float l = pin::len(dir);
                 dir = dvs(dir, l);
-                const float3 m = sub(xyz(p4), sc);
-                const float b = dot(m, dir);
-                const float cc = dot(m, m) - rad * rad;
+                const float3 m = pin::sub(xyz(p4), sc);
+                const float b = pin::dot(m, dir);
+                const float cc = pin::subr(pin::dot(m, m), pin::mulr(rad, rad));
                 if (!(cc > 0.f && b > 0.f)) {
-                    const float disc = b * b - cc;
+                    const float disc = __fmaf_rn(b, b, -cc);
                     if (!(disc < 0.f)) {
-                        const float t = -b - sqrtf(disc);
-                        if (t < 0.f) { q = add(xyz(p4), mul(dir, t)); ret = -1; }
-                        else if (!(t > l)) { q = add(xyz(p4), mul(dir, t)); ret = 1; }
+                        const float t = pin::subr(-b, sqrtf(disc));
+                        if (t < 0.f) { q = pin::fma(dir, t, xyz(p4)); ret = -1; }
+                        else if (!(t > l)) { q = pin::fma(dir, t, xyz(p4)); ret = 1; }
                     }
                 }
             }
             if (d.dbg_sphere) d.dbg_sphere[g] = (int8_t)ret;
             if (ret == -1) {
-                const float3 qs = add(sc, mul(normalize(sub(q, sc)), rad));
-                const float3 ns = normalize(sub(qs, sc));
-                d.xp[g] = f4(add(qs, mul(ns, 0.0001f)), p4.w);
+                const float3 cq = pin::sub(q, sc);
+                const float3 qs = pin::fma(dvs(cq, pin::len(cq)), rad, sc);
+                const float3 cs = pin::sub(qs, sc);
+                const float3 ns = dvs(cs, pin::len(cs));
+                d.xp[g] = f4(pin::fma(ns, 0.0001f, qs), p4.w);
                 xs[i] = f4(qs, x4.w);
             } else if (ret == 1) {
-                const float3 ns = normalize(sub(q, sc));
-                xs[i] = f4(add(q, mul(ns, 0.0001f)), x4.w);
+                const float3 cq = pin::sub(q, sc);
+                const float3 ns = dvs(cq, pin::len(cq));
+                xs[i] = f4(pin::fma(ns, 0.0001f, q), x4.w);
             }
         }
         cluster.sync();
     }
     const uint4 cr = d.crange[c];
     const uint32_t nvf_all = (uint32_t)min((uint64_t)*a.nvf, d.vf_cap);
-    const float h = cd.h;
+    const uint32_t nv = cr.y - cr.x, ncont = a.contact_gather ? 0u : nv + (cr.w - cr.z);
     // this CTA's share of the cloth's constraints (index order ~ vertex order)
     const int s_per = (cd.s_cnt + CS - 1) / CS, b_per = (cd.b_cnt + CS - 1) / CS;
     const int sb = cd.s_off + min(cd.s_cnt, r * s_per), se = cd.s_off + min(cd.s_cnt, (r + 1) * s_per);
     const int bb = cd.b_off + min(cd.b_cnt, r * b_per), be = cd.b_off + min(cd.b_cnt, (r + 1) * b_per);
     if (d.tape_x)  // a recorded step: x^0 = the prediction after the set-up
         for (int i = tid; i < n_own; i += bs) d.tape_x[vo + lo + i] = xs[i];
-    for (int it = 0; it < cd.iters; ++it) {
+    // What a thread's first constraints and first vertex read from global
+    // memory is the same in every iteration: kept in registers.
+    int2 sid0 = make_int2(0, 0);
+    float2 spar0 = make_float2(0.f, 0.f);
+    int4 bid0 = make_int4(0, 0, 0, 0);
+    float bkp0 = 0.f;
+    int cnt0 = 0;
+    if (sb + tid < se) { sid0 = __ldg(&d.s_ids[sb + tid]); spar0 = __ldg(&d.s_par[sb + tid]); }
+    if (bb + tid < be) { bid0 = __ldg(&d.b_ids[bb + tid]); bkp0 = __ldg(&d.b_kp[bb + tid]); }
+    if (tid < n_own) cnt0 = __ldg(&d.soff[vo + lo + tid + 1]) - __ldg(&d.soff[vo + lo + tid]);
+    for (int it = 0; it < iters; ++it) {
+        for (int i = tid; i < n_own; i += bs) {
+            const float4 x4 = xs[i];
+            const float cv = x4.y - gq[i];
+            const bool ground = cv < 0.f;
+            if (ground) add_fixed(lo + i, 0, fix(-cv), 0, 1u);
+            if (d.dbg_ground_it) {
+                const uint32_t bit = ground ? (1u << it) : 0u;
+                d.dbg_ground_it[vo + lo + i] = it == 0 ? bit : (d.dbg_ground_it[vo + lo + i] | bit);
+            }
+            const uint8_t f = lra[i];
+            if (f) {
+                const int64_t base = lra_off + (int64_t)(lo + i) * F;
+                for (int j = 0; j < F; ++j) {
+                    if (!((f >> j) & 1u)) continue;
+                    const float l0 = __ldg(&d.lra_l0[base + j]);
+                    const float3 diff = pin::sub(xyz(x4), xyz(X(s_fixed[j])));
+                    const float l = pin::len(diff);
+                    const float3 n = dvs(diff, l);
+                    add_corr(lo + i, pin::mul(n, -pin::subr(l, l0)), true);
+                }
+            }
+        }
         for (int k = sb + tid; k < se; k += bs) {
-            const int2 id = __ldg(&d.s_ids[k]);
-            const float2 par = __ldg(&d.s_par[k]);
+            const bool first = k == sb + tid;
+            const int2 id = first ? sid0 : __ldg(&d.s_ids[k]);
+            const float2 par = first ? spar0 : __ldg(&d.s_par[k]);
             const int i1 = id.x - vo, i2 = id.y - vo;
             const float4 p1 = X(i1), p2 = X(i2);
-            add_corr(i1, stretch_corr_pos(p1, p2, par.x, par.y, 0), false);
-            add_corr(i2, stretch_corr_pos(p1, p2, par.x, par.y, 1), false);
+            float3 q[2];
+            if (stretch_all_pos(p1, p2, par.x, par.y, q)) {
+                add_corr(i1, q[0], false);
+                add_corr(i2, q[1], false);
+            }
         }
-        for (int k = bb + tid; k < (cd.tri_bend ? bb : be); k += bs) {
-            const int4 id = __ldg(&d.b_ids[k]);
-            const float kp = __ldg(&d.b_kp[k]);
+        for (int k = bb + tid; k < (tri_bend ? bb : be); k += bs) {
+            const bool first = k == bb + tid;
+            const int4 id = first ? bid0 : __ldg(&d.b_ids[k]);
+            const float kp = first ? bkp0 : __ldg(&d.b_kp[k]);
             const int li[4] = {id.x - vo, id.y - vo, id.z - vo, id.w - vo};
             const float4 p[4] = {X(li[0]), X(li[1]), X(li[2]), X(li[3])};
             float3 q[4];
@@ -441,9 +518,10 @@ __global__ void __launch_bounds__(kClusterBlock, 2) k_solve_cluster_scatter(DevP
             }
         }
         // triangle bends (Physics/CudaPBD.cu:1149-1187), when the cloth uses them
-        for (int k = bb + tid; k < (cd.tri_bend ? be : bb); k += bs) {
-            const int4 id = __ldg(&d.b_ids[k]);
-            const float kp = __ldg(&d.b_kp[k]), h0 = __int_as_float(id.w);
+        for (int k = bb + tid; k < (tri_bend ? be : bb); k += bs) {
+            const bool first = k == bb + tid;
+            const int4 id = first ? bid0 : __ldg(&d.b_ids[k]);
+            const float kp = first ? bkp0 : __ldg(&d.b_kp[k]), h0 = __int_as_float(id.w);
             const int li[3] = {id.x - vo, id.y - vo, id.z - vo};
             const float4 p[3] = {X(li[0]), X(li[1]), X(li[2])};
 #pragma unroll
@@ -470,48 +548,22 @@ __global__ void __launch_bounds__(kClusterBlock, 2) k_solve_cluster_scatter(DevP
                 if (d.dbg_dyn_nz) d.dbg_dyn_nz[(size_t)it * d.dyn_cap + ent] = nz ? 1 : 0;
             }
         }
-        const uint32_t nv = cr.y - cr.x, ncont = a.contact_gather ? 0u : nv + (cr.w - cr.z);
         for (uint32_t k = r * bs + tid; k < ncont; k += CS * bs) {
             const bool isvf = k < nv;
             const uint32_t gi = isvf ? cr.x + k : cr.z + (k - nv);
+            const uint32_t ci = isvf ? gi : nvf_all + gi;
             const int4 v = isvf ? d.vf_v[gi] : d.ee_v[gi];
             const float4 w = isvf ? d.vf_w[gi] : d.ee_w[gi];
             const int li[4] = {v.x - vo, v.y - vo, v.z - vo, v.w - vo};
             const float4 P[4] = {X(li[0]), X(li[1]), X(li[2]), X(li[3])};
-            const uint32_t ent = 4u * (isvf ? gi : nvf_all + gi);
             float3 cs[4];
             contact_all_pos(P[0], P[1], P[2], P[3], w, isvf, h, cs);
 #pragma unroll
-            for (int j = 0; j < 4; ++j) {
-                const float3 corr = cs[j];
-                const bool nz = !is_zero(corr);
-                if (nz) add_corr(li[j], corr, true);
-                if (d.dbg_dyn_nz) d.dbg_dyn_nz[(size_t)it * d.dyn_cap + ent + j] = nz ? 1 : 0;
-            }
-        }
-        for (int i = tid; i < n_own; i += bs) {
-            const float4 x4 = xs[i];
-            const float cv = x4.y - gq[i];
-            const bool ground = cv < 0.f;
-            if (ground) {
-                atomicAdd(ayz + i, (unsigned long long)(uint32_t)__float2int_rn(-cv * kFix) << 32);
-                atomicAdd(axc + i, 1ull);
-            }
-            if (d.dbg_ground_it) {
-                const uint32_t bit = ground ? (1u << it) : 0u;
-                d.dbg_ground_it[vo + lo + i] = it == 0 ? bit : (d.dbg_ground_it[vo + lo + i] | bit);
-            }
-            const uint8_t f = lra[i];
-            if (f) {
-                const int64_t base = cd.lra_off + (int64_t)(lo + i) * cd.F;
-                for (int j = 0; j < cd.F; ++j) {
-                    if (!((f >> j) & 1u)) continue;
-                    const float3 diff = sub(xyz(x4), xyz(X(d.fixed[cd.f_off + j] - vo)));
-                    const float l = len(diff);
-                    const float3 n = dvs(diff, l);
-                    add_corr(lo + i, mul(n, -(l - d.lra_l0[base + j])), true);
-                }
-            }
+            for (int j = 0; j < 4; ++j)
+                if (!is_zero(cs[j])) add_corr(li[j], cs[j], true);
+            if (d.dbg_dyn_nz)
+#pragma unroll
+                for (int j = 0; j < 4; ++j) d.dbg_dyn_nz[(size_t)it * d.dyn_cap + 4u * ci + j] = is_zero(cs[j]) ? 0 : 1;
         }
         cluster.sync();
         for (int i = tid; i < n_own; i += bs) {
@@ -519,7 +571,8 @@ __global__ void __launch_bounds__(kClusterBlock, 2) k_solve_cluster_scatter(DevP
             const unsigned long long xc = axc[i], yz = ayz[i];
             const int sx = (int)(uint32_t)(xc >> 32), sz = (int)(uint32_t)yz;
             const int sy = (int)(uint32_t)((yz - (unsigned long long)(long long)sz) >> 32);
-            const float n = (float)(__ldg(&d.soff[g + 1]) - __ldg(&d.soff[g]) + (int)(uint32_t)xc);
+            const int stat = i == tid ? cnt0 : __ldg(&d.soff[g + 1]) - __ldg(&d.soff[g]);
+            const float n = (float)(stat + (int)(uint32_t)xc);
             float4 x4 = xs[i];
             x4.x += (__int2float_rn(sx) * kFixInv) / n;
             x4.y += (__int2float_rn(sy) * kFixInv) / n;
@@ -554,7 +607,7 @@ __global__ void __launch_bounds__(kClusterBlock, 2) k_solve_cluster_scatter(DevP
 }
 
 size_t cluster_smem_bytes(int chunk_cap, bool scatter) {
-    return (size_t)chunk_cap * (scatter ? kScatterBytesPerVertex : kClusterBytesPerVertex) + 128;
+    return (size_t)chunk_cap * (scatter ? kScatterBytesPerVertex : kClusterBytesPerVertex) + 64;
 }
 
 // Largest per-CTA vertex range the device's shared memory allows.
@@ -566,19 +619,31 @@ int cluster_chunk_cap(bool scatter) {
     return (optin - 256) / (scatter ? kScatterBytesPerVertex : kClusterBytesPerVertex);
 }
 
-template <int CS, bool SCATTER>
-static cudaError_t configure(size_t smem) {
-    auto k = SCATTER ? k_solve_cluster_scatter<CS> : k_solve_cluster<CS>;
+using SolveKernel = void (*)(DevPtrs, ClusterArgs);
+// The kernel of cs CTAs of bs threads per cloth (the gather form has one block size).
+static SolveKernel solve_kernel(int cs, int bs, bool scatter) {
+    if (!scatter) return cs == 16 ? k_solve_cluster<16> : cs == 4 ? k_solve_cluster<4> : k_solve_cluster<8>;
+    if (bs == kSolveLargeBlock)
+        return cs == 16  ? k_solve_cluster_scatter<16, kSolveLargeBlock>
+               : cs == 4 ? k_solve_cluster_scatter<4, kSolveLargeBlock>
+                         : k_solve_cluster_scatter<8, kSolveLargeBlock>;
+    return cs == 16  ? k_solve_cluster_scatter<16, kSolveSmallBlock>
+           : cs == 4 ? k_solve_cluster_scatter<4, kSolveSmallBlock>
+                     : k_solve_cluster_scatter<8, kSolveSmallBlock>;
+}
+
+static cudaError_t configure(SolveKernel k, int cs, size_t smem) {
     cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
-    if (CS > 8) e = cudaFuncSetAttribute(k, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+    if (cs > 8) e = cudaFuncSetAttribute(k, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
     return e;
 }
 
-static cudaLaunchConfig_t cluster_cfg(int cs, int nclusters, size_t smem, cudaStream_t st, cudaLaunchAttribute *attr) {
+static cudaLaunchConfig_t cluster_cfg(int cs, int bs, int nclusters, size_t smem, cudaStream_t st,
+                                      cudaLaunchAttribute *attr) {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(nclusters * cs);
-    cfg.blockDim = dim3(kClusterBlock);
+    cfg.blockDim = dim3(bs);
     cfg.dynamicSmemBytes = smem;
     cfg.stream = st;
     attr[0].id = cudaLaunchAttributeClusterDimension;
@@ -590,46 +655,33 @@ static cudaLaunchConfig_t cluster_cfg(int cs, int nclusters, size_t smem, cudaSt
     return cfg;
 }
 
-template <int CS, bool SCATTER>
-static cudaError_t launch_cs(const DevPtrs &d, const ClusterArgs &a, int nclusters, cudaStream_t st) {
-    const size_t smem = cluster_smem_bytes(a.chunk_cap, SCATTER);
-    cudaError_t e = configure<CS, SCATTER>(smem);
+cudaError_t launch_solve_cluster(const DevPtrs &d, const ClusterArgs &a, int cs, int bs, bool scatter, int nclusters,
+                                 cudaStream_t st) {
+    const SolveKernel k = solve_kernel(cs, bs, scatter);
+    const size_t smem = cluster_smem_bytes(a.chunk_cap, scatter);
+    const cudaError_t e = configure(k, cs, smem);
     if (e != cudaSuccess) return e;
     cudaLaunchAttribute attr[1];
-    cudaLaunchConfig_t cfg = cluster_cfg(CS, nclusters, smem, st, attr);
-    return cudaLaunchKernelEx(&cfg, SCATTER ? k_solve_cluster_scatter<CS> : k_solve_cluster<CS>, d, a);
+    cudaLaunchConfig_t cfg = cluster_cfg(cs, bs, nclusters, smem, st, attr);
+    return cudaLaunchKernelEx(&cfg, k, d, a);
 }
 
-cudaError_t launch_solve_cluster(const DevPtrs &d, const ClusterArgs &a, int cs, bool scatter, int nclusters,
-                                 cudaStream_t st) {
-    if (cs == 16) return scatter ? launch_cs<16, true>(d, a, nclusters, st) : launch_cs<16, false>(d, a, nclusters, st);
-    if (cs == 4) return scatter ? launch_cs<4, true>(d, a, nclusters, st) : launch_cs<4, false>(d, a, nclusters, st);
-    return scatter ? launch_cs<8, true>(d, a, nclusters, st) : launch_cs<8, false>(d, a, nclusters, st);
-}
-
-template <int CS, bool SCATTER>
-static int max_active(int chunk_cap) {
-    const size_t smem = cluster_smem_bytes(chunk_cap, SCATTER);
-    if (configure<CS, SCATTER>(smem) != cudaSuccess) {
+// How many clusters of cs CTAs of bs threads the device can hold at once (0: unsupported).
+int cluster_max_active(int cs, int bs, int chunk_cap, bool scatter) {
+    const SolveKernel k = solve_kernel(cs, bs, scatter);
+    const size_t smem = cluster_smem_bytes(chunk_cap, scatter);
+    if (configure(k, cs, smem) != cudaSuccess) {
         cudaGetLastError();
         return 0;
     }
     cudaLaunchAttribute attr[1];
-    cudaLaunchConfig_t cfg = cluster_cfg(CS, 64, smem, nullptr, attr);
+    cudaLaunchConfig_t cfg = cluster_cfg(cs, bs, 64, smem, nullptr, attr);
     int n = 0;
-    if (cudaOccupancyMaxActiveClusters(&n, SCATTER ? k_solve_cluster_scatter<CS> : k_solve_cluster<CS>, &cfg) !=
-        cudaSuccess) {
+    if (cudaOccupancyMaxActiveClusters(&n, k, &cfg) != cudaSuccess) {
         cudaGetLastError();
         return 0;
     }
     return n;
-}
-
-// How many clusters of cs CTAs the device can hold at once (0: unsupported).
-int cluster_max_active(int cs, int chunk_cap, bool scatter) {
-    if (cs == 16) return scatter ? max_active<16, true>(chunk_cap) : max_active<16, false>(chunk_cap);
-    if (cs == 4) return scatter ? max_active<4, true>(chunk_cap) : max_active<4, false>(chunk_cap);
-    return scatter ? max_active<8, true>(chunk_cap) : max_active<8, false>(chunk_cap);
 }
 
 }  // namespace lc

@@ -20,9 +20,19 @@ constexpr int kTraverseStack = 64;       // Collision/CudaBVH.cu:38
 constexpr int kTraverseBlockMax = 256;   // largest traversal block (the packet kernel is bounded for 6 of them per SM)
 constexpr int kScanBlocks = 1024;        // fixed grid of the device-count scans
 constexpr int kPairGroup = 32;           // consecutive pairs per narrowphase expansion warp (one per lane)
+constexpr int kSolveSmallBlock = 512;     // threads per CTA of the on-chip solvers: two CTAs per SM,
+constexpr int kSolveLargeBlock = 1024;    // or one (scatter form only)
 constexpr int kColliderSlots = LC_COLLIDER_SLOTS;  // static-collider contacts kept per cloth vertex and step
 constexpr int kColliderStack = 64;       // collider BVH traversal stack
 constexpr float kColliderMargin = 4.f;   // collider detection reach beyond the contact layer, in thicknesses
+
+// Vertices per CTA of a cloth of V vertices.  At least 2: the owner of a
+// vertex is found by a multiply-high by ceil(2^32 / chunk), which has to fit 32
+// bits.
+__host__ __device__ __forceinline__ int cluster_chunk(int V, int cs) {
+    const int c = (V + cs - 1) / cs;
+    return c < 2 ? 2 : c;
+}
 
 // Device error word bits (latched, reported by lc_batch_sync).
 enum : uint32_t {

@@ -8,6 +8,37 @@
 
 namespace lc {
 
+// The scatter solver's expressions: every product that feeds a sum is fused
+// explicitly and every other product and sum is rounded on its own (__fmul_rn
+// and __fadd_rn are never contracted), so its bits do not depend on how the
+// compiler schedules the code around them.
+namespace pin {
+__device__ __forceinline__ float mulr(float a, float b) { return __fmul_rn(a, b); }
+__device__ __forceinline__ float addr(float a, float b) { return __fadd_rn(a, b); }
+__device__ __forceinline__ float subr(float a, float b) { return __fsub_rn(a, b); }
+__device__ __forceinline__ float sum2(float a, float b, float c, float d) { return __fmaf_rn(a, b, mulr(c, d)); }  // a b + c d
+__device__ __forceinline__ float dot(float3 a, float3 b) {
+    return __fmaf_rn(a.z, b.z, __fmaf_rn(a.x, b.x, mulr(a.y, b.y)));
+}
+__device__ __forceinline__ float det2(float a, float b, float c, float d) { return __fmaf_rn(a, b, -mulr(c, d)); }  // a b - c d
+__device__ __forceinline__ float3 cross(float3 a, float3 b) {
+    return f3(det2(a.y, b.z, a.z, b.y), det2(a.z, b.x, a.x, b.z), det2(a.x, b.y, a.y, b.x));
+}
+__device__ __forceinline__ float3 cross_z2(float3 a, float3 b) {  // z with its other product fused
+    return f3(det2(a.y, b.z, a.z, b.y), det2(a.z, b.x, a.x, b.z), __fmaf_rn(-a.y, b.x, mulr(a.x, b.y)));
+}
+__device__ __forceinline__ float len(float3 a) { return sqrtf(dot(a, a)); }
+__device__ __forceinline__ float3 add(float3 a, float3 b) { return f3(addr(a.x, b.x), addr(a.y, b.y), addr(a.z, b.z)); }
+__device__ __forceinline__ float3 sub(float3 a, float3 b) { return f3(subr(a.x, b.x), subr(a.y, b.y), subr(a.z, b.z)); }
+__device__ __forceinline__ float3 mul(float3 a, float s) { return f3(mulr(a.x, s), mulr(a.y, s), mulr(a.z, s)); }
+__device__ __forceinline__ float3 fma(float3 a, float s, float3 c) {  // a s + c
+    return f3(__fmaf_rn(a.x, s, c.x), __fmaf_rn(a.y, s, c.y), __fmaf_rn(a.z, s, c.z));
+}
+__device__ __forceinline__ float3 mix(float3 a, float s, float3 b, float t) {  // a s + b t
+    return f3(sum2(a.x, s, b.x, t), sum2(a.y, s, b.y, t), sum2(a.z, s, b.z, t));
+}
+}  // namespace pin
+
 // Physics/CudaPBD.cu:986-1022 — stretch (distance) constraint.
 __device__ __forceinline__ float3 stretch_corr_pos(float4 a, float4 b, float l0, float kp, int role) {
     const float w1 = a.w, w2 = b.w;
@@ -19,6 +50,20 @@ __device__ __forceinline__ float3 stretch_corr_pos(float4 a, float4 b, float l0,
     const float3 n = dvs(diff, l);
     const float3 tt = dvs(mul(mul(n, l - l0), kp), ws);
     return role == 0 ? mul(tt, -w1) : mul(tt, w2);
+}
+
+// The same constraint evaluated once for both vertices; false: no correction.
+__device__ __forceinline__ bool stretch_all_pos(float4 a, float4 b, float l0, float kp, float3 out[2]) {
+    const float ws = pin::addr(a.w, b.w);
+    if (ws == 0.f) return false;
+    const float3 diff = pin::sub(xyz(a), xyz(b));
+    const float l = pin::len(diff);
+    if (l <= kEpsPbd) return false;
+    const float3 n = dvs(diff, l);
+    const float3 tt = dvs(pin::mul(pin::mul(n, pin::subr(l, l0)), kp), ws);
+    out[0] = pin::mul(tt, -a.w);
+    out[1] = pin::mul(tt, b.w);
+    return true;
 }
 
 // Physics/CudaPBD.cu:1024-1147 — bend constraint on the planes (0, p2, p3) and
@@ -77,22 +122,24 @@ __device__ __forceinline__ float3 tri_bend_corr_pos(float4 b0, float4 b1, float4
 __device__ __forceinline__ bool bend_all_pos(float4 a1, float4 a2, float4 a3, float4 a4, float kp, float kpi_gap,
                                              float3 q[4], float &s) {
     const float3 p2 = xyz(a2), p3 = xyz(a3), p4 = xyz(a4);
-    const float3 c23 = cross(p2, p3), c24 = cross(p2, p4);
-    const float l23 = len(c23), l24 = len(c24);
+    const float3 c23 = pin::cross(p2, p3), c24 = pin::cross_z2(p2, p4);
+    const float l23 = pin::len(c23), l24 = pin::len(c24);
     if (l23 <= kEpsPbd || l24 <= kEpsPbd) return false;
     const float3 n1 = dvs(c23, l23), n2 = dvs(c24, l24);
-    const float3 sv = add(n1, n2), tv = sub(n1, n2);
-    const float ss = dot(sv, sv), tt = dot(tv, tv);
+    const float3 sv = pin::add(n1, n2), tv = pin::sub(n1, n2);
+    const float ss = pin::dot(sv, sv), tt = pin::dot(tv, tv);
     if (ss == 0.f) return false;
     const float opd = 0.5f * ss, omd = 0.5f * tt;
     const float dphi = kpi_gap - 2.f * atan2f(sqrtf(ss), sqrtf(tt));
-    const float term = sqrtf(opd * omd) * dphi * kp;
-    const float3 u = sub(sv, mul(n1, opd)), w = sub(sv, mul(n2, opd));
-    q[2] = dvs(cross(p2, u), l23);
-    q[3] = dvs(cross(p2, w), l24);
-    q[1] = neg(add(dvs(cross(p3, u), l23), dvs(cross(p4, w), l24)));
-    q[0] = sub(sub(neg(q[1]), q[2]), q[3]);
-    const float sf = a1.w * dot(q[0], q[0]) + a2.w * dot(q[1], q[1]) + a3.w * dot(q[2], q[2]) + a4.w * dot(q[3], q[3]);
+    const float term = pin::mulr(pin::mulr(sqrtf(pin::mulr(opd, omd)), dphi), kp);
+    const float3 u = pin::fma(n1, -opd, sv), w = pin::fma(n2, -opd, sv);
+    q[2] = dvs(pin::cross(p2, u), l23);
+    q[3] = dvs(pin::cross(p2, w), l24);
+    q[1] = neg(add(dvs(pin::cross(p3, u), l23), dvs(pin::cross(p4, w), l24)));
+    q[0] = pin::sub(pin::sub(neg(q[1]), q[2]), q[3]);
+    float sf = pin::sum2(a1.w, pin::dot(q[0], q[0]), a2.w, pin::dot(q[1], q[1]));
+    sf = __fmaf_rn(a3.w, pin::dot(q[2], q[2]), sf);
+    sf = __fmaf_rn(a4.w, pin::dot(q[3], q[3]), sf);
     if (sf <= kEpsPbd) return false;
     s = term / sf;
     return true;
@@ -146,36 +193,40 @@ __device__ __forceinline__ void contact_all_pos(float4 A, float4 B, float4 C, fl
     if (isvf) {
         b[0] = 1.f;
         b[1] = clampf(-w.y, 0.f, 1.f), b[2] = clampf(-w.z, 0.f, 1.f), b[3] = clampf(-w.w, 0.f, 1.f);
-        const float3 q = add(add(mul(xyz(B), b[1]), mul(xyz(C), b[2])), mul(xyz(D), b[3]));
-        n = sub(xyz(A), q);
-        const float l = len(n);
+        const float3 q = pin::fma(xyz(D), b[3], pin::mix(xyz(B), b[1], xyz(C), b[2]));
+        n = pin::sub(xyz(A), q);
+        const float l = pin::len(n);
         n = dvs(n, l);
-        const float cc = l - h;
-        s = A.w + B.w * b[1] * b[1] + C.w * b[2] * b[2] + D.w * b[3] * b[3];
+        const float cc = pin::subr(l, h);
+        s = __fmaf_rn(pin::mulr(B.w, b[1]), b[1], A.w);
+        s = __fmaf_rn(pin::mulr(C.w, b[2]), b[2], s);
+        s = __fmaf_rn(pin::mulr(D.w, b[3]), b[3], s);
         if (s == 0.f) { out[0] = out[1] = out[2] = out[3] = f3(0.f, 0.f, 0.f); return; }
         s = cc / s;
         s = cc < 0.f ? s : 0.f;
-        out[0] = mul(n, -s * A.w);
-        out[1] = mul(mul(neg(n), b[1]), -s * B.w);
-        out[2] = mul(mul(neg(n), b[2]), -s * C.w);
-        out[3] = mul(mul(neg(n), b[3]), -s * D.w);
+        out[0] = pin::mul(n, pin::mulr(-s, A.w));
+        out[1] = pin::mul(pin::mul(neg(n), b[1]), pin::mulr(-s, B.w));
+        out[2] = pin::mul(pin::mul(neg(n), b[2]), pin::mulr(-s, C.w));
+        out[3] = pin::mul(pin::mul(neg(n), b[3]), pin::mulr(-s, D.w));
         return;
     }
     b[0] = w.x, b[1] = w.y, b[2] = -w.z, b[3] = -w.w;
-    const float3 q0 = add(mul(xyz(A), b[0]), mul(xyz(B), b[1]));
-    const float3 q1 = add(mul(xyz(C), b[2]), mul(xyz(D), b[3]));
-    n = sub(q0, q1);
-    const float l = len(n);
+    const float3 q0 = pin::mix(xyz(A), b[0], xyz(B), b[1]);
+    const float3 q1 = pin::mix(xyz(D), b[3], xyz(C), b[2]);
+    n = pin::sub(q0, q1);
+    const float l = pin::len(n);
     n = dvs(n, l);
-    const float cc = l - h;
-    s = A.w * b[0] * b[0] + B.w * b[1] * b[1] + C.w * b[2] * b[2] + D.w * b[3] * b[3];
+    const float cc = pin::subr(l, h);
+    s = pin::sum2(pin::mulr(A.w, b[0]), b[0], pin::mulr(B.w, b[1]), b[1]);
+    s = __fmaf_rn(pin::mulr(C.w, b[2]), b[2], s);
+    s = __fmaf_rn(pin::mulr(D.w, b[3]), b[3], s);
     if (s == 0.f) { out[0] = out[1] = out[2] = out[3] = f3(0.f, 0.f, 0.f); return; }
     s = cc / s;
     s = cc < 0.f ? s : 0.f;
-    out[0] = mul(mul(n, b[0]), -s * A.w);
-    out[1] = mul(mul(n, b[1]), -s * B.w);
-    out[2] = mul(mul(neg(n), b[2]), -s * C.w);
-    out[3] = mul(mul(neg(n), b[3]), -s * D.w);
+    out[0] = pin::mul(pin::mul(n, b[0]), pin::mulr(-s, A.w));
+    out[1] = pin::mul(pin::mul(n, b[1]), pin::mulr(-s, B.w));
+    out[2] = pin::mul(pin::mul(neg(n), b[2]), pin::mulr(-s, C.w));
+    out[3] = pin::mul(pin::mul(neg(n), b[3]), pin::mulr(-s, D.w));
 }
 
 // Static-collider contacts of vertex i (lc_batch_set_collider): each slot's
