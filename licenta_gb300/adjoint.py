@@ -57,6 +57,10 @@ class DiffCloth:
         counts = [self.batch.constraint_counts(c) for c in range(len(specs))]
         self.E = sum(e for e, _ in counts)
         self.B = sum(b for _, b in counts)
+        # the cloth of every vertex, stretch and bend constraint
+        self.vertex_cloth, self.stretch_cloth, self.bend_cloth = (
+            torch.from_numpy(np.repeat(np.arange(len(specs)), n)).to("cuda")
+            for n in (self.batch.num_vertices, [e for e, _ in counts], [b for _, b in counts]))
         self.initial = self.new_state()
         self.save(self.initial)
         torch.cuda.synchronize()
@@ -145,11 +149,6 @@ class ClothRollout(torch.autograd.Function):
         gks = torch.zeros(cloth.E, dtype=torch.float32, device="cuda")
         gkb = torch.zeros(cloth.B, dtype=torch.float32, device="cuda")
         ncl = len(cloth.batch.num_vertices)
-        vcl = torch.repeat_interleave(torch.arange(ncl, device="cuda"),
-                                      torch.tensor(cloth.batch.num_vertices, device="cuda"))
-        counts = [cloth.batch.constraint_counts(c) for c in range(ncl)]
-        ecl = torch.repeat_interleave(torch.arange(ncl, device="cuda"), torch.tensor([e for e, _ in counts], device="cuda"))
-        bcl = torch.repeat_interleave(torch.arange(ncl, device="cuda"), torch.tensor([b for _, b in counts], device="cuda"))
         exp60 = torch.zeros(ncl, dtype=torch.int32, device="cuda")
         for seg in range(len(ctx.ckpts) - 1, -1, -1):
             first = seg * cloth.every
@@ -180,7 +179,8 @@ class ClothRollout(torch.autograd.Function):
             if t.dim() == 2:
                 sc = sc.unsqueeze(1)
             return torch.where(t == 0, t, t * sc)
-        return (None, None, unscale(gks, ecl), unscale(gkb, bcl), unscale(gx + gxp, vcl), unscale(gv, vcl))
+        return (None, None, unscale(gks, cloth.stretch_cloth), unscale(gkb, cloth.bend_cloth),
+                unscale(gx + gxp, cloth.vertex_cloth), unscale(gv, cloth.vertex_cloth))
 
 
 def fit_cloth_stiffness(cloth: DiffCloth, steps: int, x0: torch.Tensor, v0: torch.Tensor, target: torch.Tensor,
@@ -197,11 +197,7 @@ def fit_cloth_stiffness(cloth: DiffCloth, steps: int, x0: torch.Tensor, v0: torc
     magnitude is beyond float range.  Returns (k, history) with history a
     list of (total loss, per-cloth losses) before each update."""
     C = len(cloth.batch.num_vertices)
-    counts = [cloth.batch.constraint_counts(c) for c in range(C)]
-    ecl = torch.repeat_interleave(torch.arange(C, device="cuda"), torch.tensor([e for e, _ in counts], device="cuda"))
-    bcl = torch.repeat_interleave(torch.arange(C, device="cuda"), torch.tensor([b for _, b in counts], device="cuda"))
-    vcl = torch.repeat_interleave(torch.arange(C, device="cuda"),
-                                  torch.tensor(cloth.batch.num_vertices, device="cuda"))
+    ecl, bcl, vcl = cloth.stretch_cloth, cloth.bend_cloth, cloth.vertex_cloth
     k = torch.full((C,), float(k0), device="cuda")
     step = torch.full((C,), float(step0), device="cuda")
     prev = torch.zeros(C, device="cuda")

@@ -10,6 +10,8 @@
 // integration reversed, the Jacobi iterations reversed (per constraint a
 // vector-Jacobian product written to its CSR slots, then a per-vertex gather
 // in a fixed order), prediction reversed, damping reversed (per-cloth sums).
+#include <algorithm>
+
 #include "lc_internal.cuh"
 
 namespace lc {
@@ -489,10 +491,15 @@ __global__ void k_adj_damp2(DevPtrs d, AdjPtrs A) {
 
 // float3-packed (3 floats per vertex) <-> float4 gradient buffers.
 // The caller's state gradients (3 packed floats per vertex) to and from the
-// float4 work copies, all three arrays in one launch.
+// float4 work copies, and its stiffness gradients (which may be null) to and
+// from the accumulators, in one launch each way: the kernels between them hold
+// no caller pointer, so one captured graph serves every set of buffers.
 __global__ void k_adj_unpack(AdjPtrs A, const float *__restrict__ gx, const float *__restrict__ gxp,
-                             const float *__restrict__ gv, int n) {
+                             const float *__restrict__ gv, const float *__restrict__ gks,
+                             const float *__restrict__ gkb, int n) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (gks && i < A.E) A.gks[i] = gks[i];
+    if (gkb && i < A.B) A.gkb[i] = gkb[i];
     if (i >= n) return;
     A.gx[i] = make_float4(gx[3 * i], gx[3 * i + 1], gx[3 * i + 2], 0.f);
     A.gxp[i] = make_float4(gxp[3 * i], gxp[3 * i + 1], gxp[3 * i + 2], 0.f);
@@ -507,8 +514,11 @@ __device__ __forceinline__ float put3(float *dst, int i, float4 v) {
 // flag (may be null): flag[c] = 1 when a state gradient of cloth c is above
 // kRescaleAbove in magnitude after the step.
 __global__ void k_adj_pack(DevPtrs d, AdjPtrs A, float *__restrict__ gx, float *__restrict__ gxp,
-                           float *__restrict__ gv, uint32_t *__restrict__ flag, int n) {
+                           float *__restrict__ gv, float *__restrict__ gks, float *__restrict__ gkb,
+                           uint32_t *__restrict__ flag, int n) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (gks && i < A.E) gks[i] = A.gks[i];
+    if (gkb && i < A.B) gkb[i] = A.gkb[i];
     if (i >= n) return;
     const float m = fmaxf(fmaxf(put3(gx, i, A.gx[i]), put3(gxp, i, A.gxp[i])), put3(gv, i, A.gv[i]));
     if (flag && m > kRescaleAbove) flag[d.vcloth[i]] = 1u;
@@ -543,12 +553,15 @@ __global__ void k_adj_rescale(DevPtrs d, float *__restrict__ gx, float *__restri
 // ---------------------------------------------------------------------------
 static inline int nb(int64_t n, int b = kThreads) { return (int)((n + b - 1) / b); }
 
-void launch_adj_unpack(const AdjPtrs &A, const float *gx, const float *gxp, const float *gv, int n, cudaStream_t st) {
-    if (n) k_adj_unpack<<<nb(n), kThreads, 0, st>>>(A, gx, gxp, gv, n);
+static int64_t pack_threads(const AdjPtrs &A, int n) { return std::max<int64_t>(n, std::max(A.E, A.B)); }
+
+void launch_adj_unpack(const AdjPtrs &A, const float *gx, const float *gxp, const float *gv, const float *gks,
+                       const float *gkb, int n, cudaStream_t st) {
+    if (n) k_adj_unpack<<<nb(pack_threads(A, n)), kThreads, 0, st>>>(A, gx, gxp, gv, gks, gkb, n);
 }
-void launch_adj_pack(const DevPtrs &d, const AdjPtrs &A, float *gx, float *gxp, float *gv, uint32_t *flag, int n,
-                     cudaStream_t st) {
-    if (n) k_adj_pack<<<nb(n), kThreads, 0, st>>>(d, A, gx, gxp, gv, flag, n);
+void launch_adj_pack(const DevPtrs &d, const AdjPtrs &A, float *gx, float *gxp, float *gv, float *gks, float *gkb,
+                     uint32_t *flag, int n, cudaStream_t st) {
+    if (n) k_adj_pack<<<nb(pack_threads(A, n)), kThreads, 0, st>>>(d, A, gx, gxp, gv, gks, gkb, flag, n);
 }
 void launch_adj_rescale(const DevPtrs &d, float *gx, float *gxp, float *gv, float *gks, float *gkb,
                         const uint32_t *flag, uint32_t *flag_next, int32_t *exponent, int E, int B, cudaStream_t st) {

@@ -36,9 +36,11 @@ void launch_narrow(const DevPtrs &d, const uint32_t *npairs, const uint32_t *ncv
                    int stage, cudaStream_t st);
 void launch_wind(const DevPtrs &d, cudaStream_t st);
 void launch_external(const DevPtrs &d, cudaStream_t st, float4 *save_x = nullptr, float4 *save_v = nullptr);
-void launch_adj_unpack(const AdjPtrs &A, const float *gx, const float *gxp, const float *gv, int n, cudaStream_t st);
-void launch_adj_pack(const DevPtrs &d, const AdjPtrs &A, float *gx, float *gxp, float *gv, uint32_t *flag, int n,
-                     cudaStream_t st);
+void launch_stiffness(const DevPtrs &d, const float *ks, const float *kb, int E, int B, cudaStream_t st);
+void launch_adj_unpack(const AdjPtrs &A, const float *gx, const float *gxp, const float *gv, const float *gks,
+                       const float *gkb, int n, cudaStream_t st);
+void launch_adj_pack(const DevPtrs &d, const AdjPtrs &A, float *gx, float *gxp, float *gv, float *gks, float *gkb,
+                     uint32_t *flag, int n, cudaStream_t st);
 void launch_adj_rescale(const DevPtrs &d, float *gx, float *gxp, float *gv, float *gks, float *gkb,
                         const uint32_t *flag, uint32_t *flag_next, int32_t *exponent, int E, int B, cudaStream_t st);
 void launch_adjoint(const DevPtrs &d, const AdjPtrs &A, float4 *a, float4 *g, const uint32_t *nvf, const uint32_t *nee,
@@ -396,23 +398,22 @@ struct lc_batch {
         free_collider_arrays();
     }
 
-    // graphs of the adjoint step (the recorded step and its reverse pass),
-    // one per set of gradient buffers and rescale parity, most recent first
+    // graphs of the adjoint step (the recorded step and its reverse pass), by
+    // which stiffness gradients it accumulates (1: stretch, 2: bend)
     struct AdjGraph {
-        uintptr_t key[7];
-        cudaGraph_t g;
-        cudaGraphExec_t e;
+        cudaGraph_t g = nullptr;
+        cudaGraphExec_t e = nullptr;
     };
-    std::vector<AdjGraph> adj_graphs;
+    AdjGraph adj_graphs[4];
 
     void invalidate_graph() {
         if (gexec) { cudaGraphExecDestroy(gexec); gexec = nullptr; }
         if (graph) { cudaGraphDestroy(graph); graph = nullptr; }
         for (AdjGraph &a : adj_graphs) {
-            cudaGraphExecDestroy(a.e);
-            cudaGraphDestroy(a.g);
+            if (a.e) cudaGraphExecDestroy(a.e);
+            if (a.g) cudaGraphDestroy(a.g);
+            a = AdjGraph{};
         }
-        adj_graphs.clear();
     }
 
     lc_status enqueue_step(cudaStream_t st);
@@ -945,6 +946,7 @@ static lc_status batch_build(lc_batch *b, const lc_cloth_desc *descs, int n, con
         LC_TRY(A.alloc(b->tape_xin, V, "tape_xin")); LC_TRY(A.alloc(b->tape_vb, V, "tape_vb"));
         LC_TRY(A.alloc(b->adj_a, V, "adj_a")); LC_TRY(A.alloc(b->adj_g, V, "adj_g"));
         LC_TRY(A.alloc(J.u, V, "adj_u"));
+        LC_TRY(A.alloc(J.gks, std::max<int64_t>(E, 1), "adj_gks")); LC_TRY(A.alloc(J.gkb, std::max<int64_t>(B, 1), "adj_gkb"));
         LC_TRY(A.alloc(J.gx, V, "adj_gx")); LC_TRY(A.alloc(J.gxp, V, "adj_gxp")); LC_TRY(A.alloc(J.gv, V, "adj_gv"));
         LC_TRY(A.alloc(J.slot, std::max<int64_t>(S, 1), "adj_slot"));
         LC_TRY(A.alloc(J.dyn, std::max<uint64_t>(d.dyn_cap, 1), "adj_dyn"));
@@ -1734,13 +1736,19 @@ lc_status lc_batch_set_constraint_stiffness(lc_batch *b, const float *ks, const 
     size_t E = 0, B = 0;
     for (int c = 0; c < b->C; ++c) { E += b->hosts[c].s_ids.size(); B += b->hosts[c].b_ids.size(); }
     LC_CUDA(cudaDeviceSynchronize());
+    if (!is_host) {  // steps in flight keep the old values; the new ones hold when the call returns
+        launch_stiffness(b->d, ks, kb, (int)E, (int)B, 0);
+        LC_CUDA(cudaGetLastError());
+        LC_CUDA(cudaStreamSynchronize(0));
+        return LC_OK;
+    }
     if (ks) {
         hs.resize(E);
-        if (E) LC_CUDA(cudaMemcpy(hs.data(), ks, sizeof(float) * E, is_host ? cudaMemcpyHostToHost : cudaMemcpyDeviceToHost));
+        if (E) std::memcpy(hs.data(), ks, sizeof(float) * E);
     }
     if (kb) {
         hb.resize(B);
-        if (B) LC_CUDA(cudaMemcpy(hb.data(), kb, sizeof(float) * B, is_host ? cudaMemcpyHostToHost : cudaMemcpyDeviceToHost));
+        if (B) std::memcpy(hb.data(), kb, sizeof(float) * B);
     }
     for (int c = 0; c < b->C; ++c)
         LC_TRY(lc_batch_set_stiffness(b, c, ks ? hs.data() + b->e_off[c] : nullptr, kb ? hb.data() + b->b_off[c] : nullptr));
@@ -1815,54 +1823,42 @@ static lc_status adjoint_step(lc_batch *b, float *gx, float *gxp, float *gv, flo
         const lc_status r = b->enqueue_step(s);
         b->recording = false;
         if (r != LC_OK) return r;
-        uint32_t *flag = exponent ? b->adj_flag + (size_t)b->adj_flip * b->C : nullptr;
-        launch_adj_unpack(b->adj, gx, gxp, gv, V, s);
-        launch_adjoint(b->d, b->adj, b->adj_a, b->adj_g, b->nvf, b->nee, b->narrow_grid, b->nfixed, gk_stretch,
-                       gk_bend, s);
-        launch_adj_pack(b->d, b->adj, gx, gxp, gv, flag, V, s);
-        if (exponent) {
-            uint32_t *next = b->adj_flag + (size_t)(1 - b->adj_flip) * b->C;
-            launch_adj_rescale(b->d, gx, gxp, gv, gk_stretch, gk_bend, flag, next, exponent, b->adj.E, b->adj.B, s);
-        }
+        launch_adjoint(b->d, b->adj, b->adj_a, b->adj_g, b->nvf, b->nee, b->narrow_grid, b->nfixed,
+                       gk_stretch ? b->adj.gks : nullptr, gk_bend ? b->adj.gkb : nullptr, s);
         LC_CUDA(cudaGetLastError());
         return LC_OK;
     };
+    launch_adj_unpack(b->adj, gx, gxp, gv, gk_stretch, gk_bend, V, st);
     if (!b->opt.use_graph || b->opt.debug_capture) {
         LC_TRY(enqueue(st));
     } else {
-        // about 130 short launches for a small cloth: replayed as one graph,
-        // captured once per set of gradient buffers and rescale parity
-        const uintptr_t key[7] = {(uintptr_t)gx, (uintptr_t)gxp, (uintptr_t)gv, (uintptr_t)gk_stretch,
-                                  (uintptr_t)gk_bend, (uintptr_t)exponent, (uintptr_t)b->adj_flip};
-        size_t k = 0;
-        while (k < b->adj_graphs.size() && std::memcmp(b->adj_graphs[k].key, key, sizeof(key)) != 0) ++k;
-        if (k == b->adj_graphs.size()) {
+        // about 120 short launches for a small cloth: replayed as one graph,
+        // which reads and writes the batch's own gradient copies only
+        lc_batch::AdjGraph &a = b->adj_graphs[(gk_stretch ? 1 : 0) | (gk_bend ? 2 : 0)];
+        if (!a.e) {
             LC_CUDA(cudaStreamBeginCapture(b->cap_stream, cudaStreamCaptureModeThreadLocal));
             const lc_status s = enqueue(b->cap_stream);
             cudaGraph_t g = nullptr;
             const cudaError_t e = cudaStreamEndCapture(b->cap_stream, &g);
             if (s != LC_OK) { if (g) cudaGraphDestroy(g); return s; }
             LC_CUDA(e);
-            lc_batch::AdjGraph a{};
-            std::memcpy(a.key, key, sizeof(key));
-            a.g = g;
             if (cudaGraphInstantiate(&a.e, g, 0) != cudaSuccess) {
+                cudaGetLastError();
                 cudaGraphDestroy(g);
+                a = lc_batch::AdjGraph{};
                 return fail(LC_ERR_CUDA, std::string(who) + ": graph instantiation failed");
             }
-            if (b->adj_graphs.size() == 4) {
-                cudaGraphExecDestroy(b->adj_graphs.back().e);
-                cudaGraphDestroy(b->adj_graphs.back().g);
-                b->adj_graphs.pop_back();
-            }
-            b->adj_graphs.insert(b->adj_graphs.begin(), a);
-            k = 0;
-        } else if (k) {
-            std::rotate(b->adj_graphs.begin(), b->adj_graphs.begin() + k, b->adj_graphs.begin() + k + 1);
-            k = 0;
+            a.g = g;
         }
-        LC_CUDA(cudaGraphLaunch(b->adj_graphs[k].e, st));
+        LC_CUDA(cudaGraphLaunch(a.e, st));
     }
+    uint32_t *flag = exponent ? b->adj_flag + (size_t)b->adj_flip * b->C : nullptr;
+    launch_adj_pack(b->d, b->adj, gx, gxp, gv, gk_stretch, gk_bend, flag, V, st);
+    if (exponent) {
+        uint32_t *next = b->adj_flag + (size_t)(1 - b->adj_flip) * b->C;
+        launch_adj_rescale(b->d, gx, gxp, gv, gk_stretch, gk_bend, flag, next, exponent, b->adj.E, b->adj.B, st);
+    }
+    LC_CUDA(cudaGetLastError());
     if (exponent) b->adj_flip = 1 - b->adj_flip;
     return LC_OK;
 }

@@ -214,6 +214,7 @@ struct AdjPtrs {
     float *fixed;            // 3 per pinned vertex: LRA contributions (block sums + atomics)
     float4 *u;               // dL/dx^{k+1} / count, per vertex
     float4 *gx, *gxp, *gv;   // state gradients: after the step on entry, before it on exit
+    float *gks, *gkb;        // dL/dk accumulators, copied in and out with the state gradients
     double *red;             // 8 per vertex block (partials), then 8 per cloth (totals)
     int nvblk_red;           // offset of the cloth totals in red
     int K;                   // solver iterations of the recorded step (max over cloths)
