@@ -55,8 +55,6 @@ void launch_friction(const DevPtrs &d, const uint32_t *nvf, cudaStream_t st);
 void launch_vertex_records(const DevPtrs &d, void *dst, int64_t stride, int pos_off, int nrm_off, cudaStream_t st);
 void launch_xyz_unpack(const float *src, float4 *dst, int n, cudaStream_t st);
 void launch_xyz_pack(const float4 *src, float *dst, int n, cudaStream_t st);
-void scan_u32(const uint32_t *in, uint32_t *out, const uint32_t *n_dev, uint32_t n_static, uint32_t n_cap,
-              uint32_t *partial, uint32_t *total_out, unsigned long long *total_out64, cudaStream_t st);
 unsigned long long morton3_host(float x, float y, float z, int mode);
 struct ClusterArgs {
     const int *cl_cloth;
@@ -470,8 +468,8 @@ lc_status lc_batch::enqueue_step(cudaStream_t st) {
     LC_KEV(2);
     launch_traverse(d, traverse_block, st);
     LC_KEV(3);
-    scan_u32(d.pair_cnt, d.pair_off, nullptr, (uint32_t)d.Ttot, (uint32_t)d.Ttot, d.scan_tmp, npairs,
-             &d.counters[0], st);
+    const uint32_t T = (uint32_t)d.Ttot, V = (uint32_t)d.Vtot;
+    scan_u32({d.pair_cnt, d.pair_off, nullptr, T, T, npairs, &d.counters[0]}, nullptr, d.scan_tmp, d.err, st);
     launch_pair_compact(d, st);
     LC_PHASE(4);
     // 5. Perform Triangle Tests
@@ -479,8 +477,8 @@ lc_status lc_batch::enqueue_step(cudaStream_t st) {
     launch_narrow(d, npairs, ncand, ncand_e, narrow_grid, 0, st);  // filter: masks + counts per group of pairs
     LC_KEV(5);
     const uint32_t gcap = (uint32_t)(d.pair_cap / kPairGroup + 1);
-    scan_u32(d.grp_vf_cnt, d.grp_vf_off, d.ngroups, 0, gcap, d.scan_tmp, ncand, nullptr, st);
-    scan_u32(d.grp_ee_cnt, d.grp_ee_off, d.ngroups, 0, gcap, d.scan_tmp, ncand_e, nullptr, st);
+    const ScanJob groups_ee{d.grp_ee_cnt, d.grp_ee_off, d.ngroups, 0, gcap, ncand_e, nullptr};
+    scan_u32({d.grp_vf_cnt, d.grp_vf_off, d.ngroups, 0, gcap, ncand, nullptr}, &groups_ee, d.scan_tmp, d.err, st);
     launch_narrow(d, npairs, ncand, ncand_e, narrow_grid, 1, st);  // expand
     LC_KEV(8);
     launch_narrow(d, npairs, ncand, ncand_e, narrow_grid, 2, st);  // VF CCD
@@ -488,8 +486,8 @@ lc_status lc_batch::enqueue_step(cudaStream_t st) {
     launch_narrow(d, npairs, ncand, ncand_e, narrow_grid, 5, st);  // EE CCD
     LC_KEV(10);
     const uint32_t hcap = (uint32_t)(d.cand_cap / 32 + 1);
-    scan_u32(d.hitg_cnt[0], d.hitg_off[0], d.hitg_n, 0, hcap, d.scan_tmp, nvf, &d.counters[1], st);
-    scan_u32(d.hitg_cnt[1], d.hitg_off[1], d.hitg_n + 1, 0, hcap, d.scan_tmp, nee, &d.counters[2], st);
+    const ScanJob hits_ee{d.hitg_cnt[1], d.hitg_off[1], d.hitg_n + 1, 0, hcap, nee, &d.counters[2]};
+    scan_u32({d.hitg_cnt[0], d.hitg_off[0], d.hitg_n, 0, hcap, nvf, &d.counters[1]}, &hits_ee, d.scan_tmp, d.err, st);
     launch_narrow(d, npairs, ncand, ncand_e, narrow_grid, 3, st);  // write contacts
     launch_narrow(d, npairs, ncand, ncand_e, narrow_grid, 4, st);  // per-cloth ranges
     launch_collider(d, narrow_grid, st);                            // static colliders (lc_batch_set_collider)
@@ -506,7 +504,7 @@ lc_status lc_batch::enqueue_step(cudaStream_t st) {
         LC_CUDA(cudaMemsetAsync(d.dyn_cnt, 0, sizeof(uint32_t) * (size_t)d.Vtot, st));
         LC_CUDA(cudaMemsetAsync(d.dyn_cur, 0, sizeof(uint32_t) * (size_t)d.Vtot, st));
         launch_dyn(d, nvf, nee, narrow_grid, 0, st);
-        scan_u32(d.dyn_cnt, d.dyn_off, nullptr, (uint32_t)d.Vtot, (uint32_t)d.Vtot, d.scan_tmp, nullptr, nullptr, st);
+        scan_u32({d.dyn_cnt, d.dyn_off, nullptr, V, V, nullptr, nullptr}, nullptr, d.scan_tmp, d.err, st);
         launch_dyn(d, nvf, nee, narrow_grid, 1, st);
         if (ordered || recording) launch_dyn(d, nvf, nee, narrow_grid, 2, st);
     }
@@ -832,7 +830,8 @@ static lc_status batch_build(lc_batch *b, const lc_cloth_desc *descs, int n, con
     LC_TRY(A.alloc(d.damp, 16 * (size_t)n, "damp"));
     LC_TRY(A.alloc(d.counters, 4, "counters"));
     LC_TRY(A.alloc(d.err, 1, "err"));
-    LC_TRY(A.alloc(d.scan_tmp, kScanBlocks + 1, "scan_tmp"));
+    LC_TRY(A.alloc(d.scan_tmp, kScanScratch, "scan_tmp"));
+    LC_CUDA(cudaMemset(d.scan_tmp, 0, sizeof(uint32_t) * kScanScratch));
     int *stc, *sts, *tf; LC_TRY(A.alloc(stc, stile_cloth.size(), "stile_cloth"));
     LC_TRY(A.alloc(sts, stile_start.size(), "stile_start")); LC_TRY(A.alloc(tf, n + 1, "tile_first"));
     d.stile_cloth = stc; d.stile_start = sts; b->tile_first = tf;
@@ -2210,7 +2209,8 @@ lc_status lc_lbvh_create(int32_t max_triangles, int32_t chunk_size, int32_t mort
     LC_TRY(A.alloc(d.pair_cnt, T, "pair_cnt")); LC_TRY(A.alloc(d.pair_off, T + 1, "pair_off"));
     LC_TRY(A.alloc(d.pair_chunk, PC, "pair_chunk")); LC_TRY(A.alloc(d.pairs, PC, "pairs"));
     LC_TRY(A.alloc(d.counters, 4, "counters")); LC_TRY(A.alloc(d.err, 1, "err"));
-    LC_TRY(A.alloc(d.scan_tmp, kScanBlocks + 1, "scan_tmp"));
+    LC_TRY(A.alloc(d.scan_tmp, kScanScratch, "scan_tmp"));
+    LC_CUDA(cudaMemset(d.scan_tmp, 0, sizeof(uint32_t) * kScanScratch));
     int *stc, *sts, *tf;
     LC_TRY(A.alloc(stc, tiles, "stile_cloth")); LC_TRY(A.alloc(sts, tiles, "stile_start")); LC_TRY(A.alloc(tf, 2, "tile_first"));
     d.stile_cloth = stc; d.stile_start = sts; b.tile_first = tf;
@@ -2268,8 +2268,8 @@ lc_status lc_lbvh_pairs(lc_lbvh *h, uint32_t *out_pairs, uint64_t cap, uint64_t 
     lc_batch &b = h->b;
     DevPtrs &d = b.d;
     launch_traverse(d, b.traverse_block, st);
-    scan_u32(d.pair_cnt, d.pair_off, nullptr, (uint32_t)d.Ttot, (uint32_t)d.Ttot, d.scan_tmp, b.npairs,
-             &d.counters[0], st);
+    scan_u32({d.pair_cnt, d.pair_off, nullptr, (uint32_t)d.Ttot, (uint32_t)d.Ttot, b.npairs, &d.counters[0]}, nullptr,
+             d.scan_tmp, d.err, st);
     launch_pair_compact(d, st);
     LC_CUDA(cudaGetLastError());
     uint32_t n = 0;

@@ -46,8 +46,6 @@
 
 namespace lc {
 void launch_sort(const DevPtrs &d, const int *tile_first, int passes, cudaStream_t st);
-void scan_u32(const uint32_t *in, uint32_t *out, const uint32_t *n_dev, uint32_t n_static, uint32_t n_cap,
-              uint32_t *partial, uint32_t *total_out, unsigned long long *total_out64, cudaStream_t st);
 void set_last_error(const std::string &msg);
 
 namespace {
@@ -482,7 +480,8 @@ lc_status lc_broadphase_create(const lc_broadphase_desc *desc, lc_broadphase **o
     const uint64_t counts = std::max<uint64_t>(N, E);
     LC_TRY_BP(b.alloc(b.cnt, counts, "counts"));
     LC_TRY_BP(b.alloc(b.off, counts + 1, "offsets"));
-    LC_TRY_BP(b.alloc(b.scan_tmp, kScanBlocks + 1, "scan partials"));
+    LC_TRY_BP(b.alloc(b.scan_tmp, kScanScratch, "scan partials"));
+    LC_BP_CUDA(cudaMemset(b.scan_tmp, 0, sizeof(uint32_t) * kScanScratch));
     LC_TRY_BP(b.alloc(b.total, 1, "total"));
     LC_TRY_BP(b.alloc(b.tests, 1, "tests"));
     LC_TRY_BP(b.alloc(b.err, 1, "error word"));
@@ -547,13 +546,14 @@ lc_status lc_broadphase_update(lc_broadphase *b, const float *box_min, const flo
     } else if (n > 0 && (m == LC_BP_GRID || m == LC_BP_HASH)) {
         k_bp_grid_entries<<<nblocks(n), kThreads, 0, st>>>(b->grid, box_min, box_max, n, b->cnt, nullptr, 0, nullptr,
                                                             nullptr, nullptr, b->err);
-        scan_u32(b->cnt, b->off, nullptr, (uint32_t)n, (uint32_t)n, b->scan_tmp, b->total, nullptr, st);
+        scan_u32({b->cnt, b->off, nullptr, (uint32_t)n, (uint32_t)n, b->total, nullptr}, nullptr, b->scan_tmp, b->err, st);
         uint32_t tot = 0, err = 0;
         LC_BP_CUDA(cudaMemcpyAsync(&tot, b->total, sizeof(tot), cudaMemcpyDeviceToHost, st));
         LC_BP_CUDA(cudaMemcpyAsync(&err, b->err, sizeof(err), cudaMemcpyDeviceToHost, st));
         LC_BP_CUDA(cudaStreamSynchronize(st));
         if (err || tot > b->max_keys) {
             LC_BP_CUDA(cudaMemset(b->err, 0, sizeof(uint32_t)));
+            if (err & ERR_SORT) return bp_fail(LC_ERR_TIMEOUT, "lc_broadphase_update: scan wait exceeded its bound");
             return bp_fail(LC_ERR_CAPACITY_OVERFLOW, "lc_broadphase_update: the boxes cover more grid cells than "
                                                      "lc_broadphase_desc.max_entries (" + std::to_string(tot) + ")");
         }
@@ -614,7 +614,8 @@ lc_status lc_broadphase_test(lc_broadphase *b, uint32_t *pairs, uint64_t cap, ui
     run(b->cnt, nullptr, nullptr);
     uint32_t tot = 0;
     if (units) {
-        scan_u32(b->cnt, b->off, nullptr, (uint32_t)units, (uint32_t)units, b->scan_tmp, b->total, nullptr, st);
+        scan_u32({b->cnt, b->off, nullptr, (uint32_t)units, (uint32_t)units, b->total, nullptr}, nullptr, b->scan_tmp,
+                 b->err, st);
         if (pairs && cap) run(nullptr, b->off, pairs);
         LC_BP_CUDA(cudaMemcpyAsync(&tot, b->total, sizeof(tot), cudaMemcpyDeviceToHost, st));
     }

@@ -18,7 +18,8 @@ constexpr int kSortTile = 2048;          // keys per sort tile (256 threads x 8)
 constexpr int kSortPassesMax = 8;        // 8-bit digits of a 63-bit key
 constexpr int kTraverseStack = 64;       // Collision/CudaBVH.cu:38
 constexpr int kTraverseBlockMax = 256;   // largest traversal block (the packet kernel is bounded for 6 of them per SM)
-constexpr int kScanBlocks = 1024;        // fixed grid of the device-count scans
+constexpr uint32_t kScanBlocks = 304;    // largest grid of the device-count scans
+constexpr uint32_t kScanScratch = 2 * (2 * kScanBlocks + 2);  // u32 words of scratch of two scans in one launch
 constexpr int kPairGroup = 32;           // consecutive pairs per narrowphase expansion warp (one per lane)
 constexpr int kSolveSmallBlock = 512;     // threads per CTA of the on-chip solvers: two CTAs per SM,
 constexpr int kSolveLargeBlock = 1024;    // or one (scatter form only)
@@ -45,6 +46,20 @@ enum : uint32_t {
     ERR_COLL_OVERFLOW = 1u << 6,   // more static-collider contacts at a vertex than kColliderSlots
     ERR_SORT = 1u << 7,            // a sort look-back wait ran past its bound
 };
+
+// One exclusive scan of u32 counts (lc_scan.cu): in has min(*n_dev, n_cap)
+// entries (n_static when n_dev is null), out one more, its total.
+struct ScanJob {
+    const uint32_t *in;
+    uint32_t *out;
+    const uint32_t *n_dev;
+    uint32_t n_static, n_cap;
+    uint32_t *total;               // may be null
+    unsigned long long *total64;   // may be null
+};
+// One or two scans in one launch (b may be null); scratch: kScanScratch words,
+// zero before the first scan that uses it.
+void scan_u32(const ScanJob &a, const ScanJob *b, uint32_t *scratch, uint32_t *err, cudaStream_t st);
 
 // Per-cloth descriptor in device memory.
 struct ClothDev {
@@ -163,7 +178,7 @@ struct DevPtrs {
     double *damp;          // 16 per cloth
     unsigned long long *counters;  // [0] pairs [1] vf [2] ee [3] dropped
     uint32_t *err;
-    uint32_t *scan_tmp;    // kScanBlocks + 1 partials
+    uint32_t *scan_tmp;    // kScanScratch words, zero between scans
     // sort bookkeeping
     const int *stile_cloth;   // sort tile -> cloth
     const int *stile_start;   // sort tile -> first slot (global)

@@ -26,8 +26,6 @@
 namespace lc {
 void launch_narrow(const DevPtrs &d, const uint32_t *npairs, const uint32_t *ncv, const uint32_t *nce, int grid,
                    int stage, cudaStream_t st);
-void scan_u32(const uint32_t *in, uint32_t *out, const uint32_t *n_dev, uint32_t n_static, uint32_t n_cap,
-              uint32_t *partial, uint32_t *total_out, unsigned long long *total_out64, cudaStream_t st);
 void set_last_error(const std::string &msg);  // lc_api.cu: text for lc_last_error_string()
 
 constexpr uint32_t ERR_NP_INPUT = 1u << 8;  // a caller index was out of range
@@ -162,7 +160,7 @@ lc_status lc_narrowphase_create(int32_t max_vertices, int32_t max_triangles, uin
               h->alloc(d.grp_vf_off, GC + 1) && h->alloc(d.grp_ee_off, GC + 1) && h->alloc(d.ngroups, 1) &&
               h->alloc(d.cand, d.cand_cap) && h->alloc(d.cand_e, d.cand_cap) && h->alloc(d.hitg_n, 2) &&
               h->alloc(d.vf_v, d.vf_cap) && h->alloc(d.vf_w, d.vf_cap) && h->alloc(d.ee_v, d.ee_cap) &&
-              h->alloc(d.ee_w, d.ee_cap) && h->alloc(d.hit_n, 2) && h->alloc(d.scan_tmp, kScanBlocks + 1) &&
+              h->alloc(d.ee_w, d.ee_cap) && h->alloc(d.hit_n, 2) && h->alloc(d.scan_tmp, kScanScratch) &&
               h->alloc(d.err, 1) && h->alloc(d.counters, 4) && h->alloc(h->npairs, 1) && h->alloc(h->ncand, 1) &&
               h->alloc(h->ncand_e, 1) && h->alloc(h->nvf, 1) && h->alloc(h->nee, 1) &&
               h->alloc(d.vf_tn, d.vf_cap) && h->alloc(d.ee_tn, d.ee_cap);
@@ -182,6 +180,7 @@ lc_status lc_narrowphase_create(int32_t max_vertices, int32_t max_triangles, uin
     if (e == cudaSuccess) e = cudaMemset(d.err, 0, sizeof(uint32_t));
     if (e == cudaSuccess) e = cudaMemset(d.hitg_n, 0, 2 * sizeof(uint32_t));
     if (e == cudaSuccess) e = cudaMemset(d.ngroups, 0, sizeof(uint32_t));
+    if (e == cudaSuccess) e = cudaMemset(d.scan_tmp, 0, sizeof(uint32_t) * kScanScratch);
     int dev = 0, sms = 0;
     if (e == cudaSuccess) e = cudaGetDevice(&dev);
     if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
@@ -230,16 +229,16 @@ lc_status lc_narrowphase_run(lc_narrowphase *h, int32_t mode, const float *x, co
     // the ordered expansion
     launch_narrow(d, h->npairs, h->ncand, h->ncand_e, h->grid, ccd ? 0 : 6, st);
     const uint32_t gcap = (uint32_t)(d.pair_cap / kPairGroup + 1);
-    scan_u32(d.grp_vf_cnt, d.grp_vf_off, d.ngroups, 0, gcap, d.scan_tmp, h->ncand, nullptr, st);
-    scan_u32(d.grp_ee_cnt, d.grp_ee_off, d.ngroups, 0, gcap, d.scan_tmp, h->ncand_e, nullptr, st);
+    const ScanJob groups_ee{d.grp_ee_cnt, d.grp_ee_off, d.ngroups, 0, gcap, h->ncand_e, nullptr};
+    scan_u32({d.grp_vf_cnt, d.grp_vf_off, d.ngroups, 0, gcap, h->ncand, nullptr}, &groups_ee, d.scan_tmp, d.err, st);
     launch_narrow(d, h->npairs, h->ncand, h->ncand_e, h->grid, 1, st);
     // Collision/CudaPrimitiveTests.cu:96-238: CCD on x_prev and v; or :21-94,
     // the discrete tests at x_prev
     launch_narrow(d, h->npairs, h->ncand, h->ncand_e, h->grid, ccd ? 2 : 7, st);
     launch_narrow(d, h->npairs, h->ncand, h->ncand_e, h->grid, ccd ? 5 : 8, st);
     const uint32_t hcap = (uint32_t)(d.cand_cap / 32 + 1);
-    scan_u32(d.hitg_cnt[0], d.hitg_off[0], d.hitg_n, 0, hcap, d.scan_tmp, h->nvf, nullptr, st);
-    scan_u32(d.hitg_cnt[1], d.hitg_off[1], d.hitg_n + 1, 0, hcap, d.scan_tmp, h->nee, nullptr, st);
+    const ScanJob hits_ee{d.hitg_cnt[1], d.hitg_off[1], d.hitg_n + 1, 0, hcap, h->nee, nullptr};
+    scan_u32({d.hitg_cnt[0], d.hitg_off[0], d.hitg_n, 0, hcap, h->nvf, nullptr}, &hits_ee, d.scan_tmp, d.err, st);
     launch_narrow(d, h->npairs, h->ncand, h->ncand_e, h->grid, 3, st);
     if (vf_cap)
         k_np_out<<<(unsigned)std::max<uint64_t>((std::min(vf_cap, d.vf_cap) + nb - 1) / nb, 1), nb, 0, st>>>(
@@ -257,6 +256,7 @@ lc_status lc_narrowphase_run(lc_narrowphase *h, int32_t mode, const float *x, co
     *ee_count = counts[1];
     if (err & ERR_NP_INPUT)
         return np_fail(LC_ERR_INVALID_ARG, "lc_narrowphase_run: a triangle or pair index is out of range");
+    if (err & ERR_SORT) return np_fail(LC_ERR_TIMEOUT, "lc_narrowphase_run: scan wait exceeded its bound");
     if (err & ERR_CAND_OVERFLOW)
         return np_fail(LC_ERR_CAPACITY_OVERFLOW, "lc_narrowphase_run: candidate capacity exceeded");
     if ((err & (ERR_VF_OVERFLOW | ERR_EE_OVERFLOW)) || counts[0] > vf_cap || counts[1] > ee_cap)

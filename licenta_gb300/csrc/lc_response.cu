@@ -20,8 +20,6 @@
 #include "lc_internal.cuh"
 
 namespace lc {
-void scan_u32(const uint32_t *in, uint32_t *out, const uint32_t *n_dev, uint32_t n_static, uint32_t n_cap,
-              uint32_t *partial, uint32_t *total_out, unsigned long long *total_out64, cudaStream_t st);
 void set_last_error(const std::string &msg);
 
 namespace {
@@ -174,13 +172,14 @@ extern "C" lc_status lc_solve_collisions(float *x, const float *x_prev, float *v
     LC_R_CUDA(cudaMallocAsync((void **)&cur, sizeof(uint32_t) * V, st));
     LC_R_CUDA(cudaMallocAsync((void **)&flag, sizeof(uint32_t) * V, st));
     LC_R_CUDA(cudaMallocAsync((void **)&rank, sizeof(uint32_t) * (V + 1), st));
-    LC_R_CUDA(cudaMallocAsync((void **)&part, sizeof(uint32_t) * (kScanBlocks + 1), st));
+    LC_R_CUDA(cudaMallocAsync((void **)&part, sizeof(uint32_t) * kScanScratch, st));
     LC_R_CUDA(cudaMallocAsync((void **)&bad, sizeof(uint32_t), st));
     LC_R_CUDA(cudaMallocAsync((void **)&slots, sizeof(uint32_t) * std::max<uint64_t>(S, 1), st));
     LC_R_CUDA(cudaMallocAsync((void **)&vals, sizeof(float4) * std::max<uint64_t>(S, 1), st));
     LC_R_CUDA(cudaMemsetAsync(cnt, 0, sizeof(uint32_t) * V, st));
     LC_R_CUDA(cudaMemsetAsync(cur, 0, sizeof(uint32_t) * V, st));
     LC_R_CUDA(cudaMemsetAsync(bad, 0, sizeof(uint32_t), st));
+    LC_R_CUDA(cudaMemsetAsync(part, 0, sizeof(uint32_t) * kScanScratch, st));
     if (C) {
         k_imp_check<<<cblk, nb, 0, st>>>(vf, num_vf, ee, num_ee, V, bad);
         LC_R_CUDA(cudaMemcpyAsync(&hbad, bad, sizeof(uint32_t), cudaMemcpyDeviceToHost, st));
@@ -193,13 +192,13 @@ extern "C" lc_status lc_solve_collisions(float *x, const float *x_prev, float *v
         k_imp_create<<<cblk, nb, 0, st>>>(x_prev, v, vf, num_vf, ee, num_ee, stiffness, vertex_mass, timestep,
                                           thickness, vals, cnt);
     }
-    scan_u32(cnt, off, nullptr, (uint32_t)V, (uint32_t)V, part, nullptr, nullptr, st);
+    scan_u32({cnt, off, nullptr, (uint32_t)V, (uint32_t)V, nullptr, nullptr}, nullptr, part, nullptr, st);
     if (C) {
         k_imp_fill<<<cblk, nb, 0, st>>>(vf, num_vf, ee, num_ee, off, cur, slots);
         k_imp_sort<<<vblk, nb, 0, st>>>(off, slots, V);
     }
     k_imp_flag<<<vblk, nb, 0, st>>>(cnt, flag, V);
-    scan_u32(flag, rank, nullptr, (uint32_t)V, (uint32_t)V, part, nullptr, nullptr, st);
+    scan_u32({flag, rank, nullptr, (uint32_t)V, (uint32_t)V, nullptr, nullptr}, nullptr, part, nullptr, st);
     k_imp_apply<<<vblk, nb, 0, st>>>(x, x_prev, v, fixed, V, off, slots, rank, vals, (C + 255) / 256 * 256,
                                      vertex_mass, timestep);
     LC_R_CUDA(cudaGetLastError());

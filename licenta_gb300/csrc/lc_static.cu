@@ -34,8 +34,6 @@ void launch_post_sort(const DevPtrs &d, cudaStream_t st);
 void launch_karras(const DevPtrs &d, cudaStream_t st);
 void launch_refit(const DevPtrs &d, cudaStream_t st);
 void launch_traverse(const DevPtrs &d, int block, cudaStream_t st);
-void scan_u32(const uint32_t *in, uint32_t *out, const uint32_t *n_dev, uint32_t n_static, uint32_t n_cap,
-              uint32_t *partial, uint32_t *total_out, unsigned long long *total_out64, cudaStream_t st);
 
 namespace {
 
@@ -79,7 +77,7 @@ constexpr Layout make_layout() {
     l.stile_cloth = o; o += al(4 * (size_t)kStaticTiles);
     l.stile_start = o; o += al(4 * (size_t)kStaticTiles);
     l.tile_first = o; o += al(8);
-    l.scan_tmp = o; o += al(4 * (kScanBlocks + 1));
+    l.scan_tmp = o; o += al(4 * kScanScratch);
     l.counters = o; o += al(8 * 4);
     l.err = o; o += al(4);
     l.npairs = o; o += al(4);
@@ -97,8 +95,9 @@ static __device__ __align__(256) unsigned char g_lbvh_scratch[kLayout.total];
 // Per-call set-up of the small tables that the LBVH kernels read, and the
 // counters that must start at zero (the array keeps the previous call's data).
 __global__ void k_static_init(ClothDev *cd, int *tcloth, int *stile_cloth, int *stile_start, int *tile_first,
-                              unsigned long long *counters, uint32_t *err, int T, int chunk, int mode) {
+                              unsigned long long *counters, uint32_t *err, uint32_t *scan, int T, int chunk, int mode) {
     const int t = blockIdx.x * blockDim.x + threadIdx.x;
+    for (uint32_t k = t; k < kScanScratch; k += gridDim.x * blockDim.x) scan[k] = 0;
     if (t == 0) {
         ClothDev c;
         memset(&c, 0, sizeof(c));
@@ -236,7 +235,8 @@ extern "C" lc_status lc_lbvh_pairs_static(const float *tri_min, const float *tri
     const int nb = (T + kThreads - 1) / kThreads;
     k_static_init<<<nb, kThreads, 0, st>>>(const_cast<ClothDev *>(d.cloth), const_cast<int *>(d.tcloth),
                                            const_cast<int *>(d.stile_cloth), const_cast<int *>(d.stile_start),
-                                           const_cast<int *>(tile_first), d.counters, d.err, T, chunk, morton_mode);
+                                           const_cast<int *>(tile_first), d.counters, d.err, d.scan_tmp, T, chunk,
+                                           morton_mode);
     launch_leaves_from_boxes(d, tri_min, tri_max, T, morton_mode, st);
     launch_sort(d, tile_first, morton_mode == LC_MORTON_K30 ? 4 : 8, st);
     launch_post_sort(d, st);
@@ -245,7 +245,8 @@ extern "C" lc_status lc_lbvh_pairs_static(const float *tri_min, const float *tri
     launch_karras(d, st);
     launch_refit(d, st);
     launch_traverse(d, 128, st);
-    scan_u32(d.pair_cnt, d.pair_off, nullptr, (uint32_t)T, (uint32_t)T, d.scan_tmp, npairs, &d.counters[0], st);
+    scan_u32({d.pair_cnt, d.pair_off, nullptr, (uint32_t)T, (uint32_t)T, npairs, &d.counters[0]}, nullptr, d.scan_tmp,
+             d.err, st);
     const int nwb = (T * 32 + kThreads - 1) / kThreads;  // one warp per leaf
     if (cap) k_static_compact<<<nwb, kThreads, 0, st>>>(d.pair_cnt, d.pair_off, d.pair_chunk, T, chunk,
                                                          reinterpret_cast<uint2 *>(out_pairs), cap);
