@@ -26,10 +26,8 @@ void launch_collider(const DevPtrs &d, int grid, cudaStream_t st);
 void launch_collider_faces(const DevPtrs &d, int ntri, cudaStream_t st);
 void launch_leaves_from_boxes(const DevPtrs &d, const float *bmin, const float *bmax, int T, int mode,
                               cudaStream_t st);
-void launch_sort(const DevPtrs &d, const int *tile_first, int passes, cudaStream_t st);
-void launch_post_sort(const DevPtrs &d, cudaStream_t st);
-void launch_karras(const DevPtrs &d, cudaStream_t st);
-void launch_refit(const DevPtrs &d, cudaStream_t st);
+void launch_morton_sort(const DevPtrs &d, const int *tile_first, int mode, int max_T, cudaStream_t st);
+void launch_hierarchy(const DevPtrs &d, int max_T, cudaStream_t st);
 void launch_traverse(const DevPtrs &d, int block, cudaStream_t st);
 void launch_pair_compact(const DevPtrs &d, cudaStream_t st);
 void launch_narrow(const DevPtrs &d, const uint32_t *npairs, const uint32_t *ncv, const uint32_t *nce, int grid,
@@ -338,7 +336,8 @@ struct lc_batch {
     uint32_t *npairs = nullptr, *nvf = nullptr, *nee = nullptr, *ncand = nullptr, *ncand_e = nullptr;
     int max_iters = 1;
     bool any_wind = false, any_sphere = false;
-    int sort_passes = 8;
+    int morton_mode = LC_MORTON_REF63;
+    int max_T = 0;  // triangles of the largest cloth
     int narrow_grid = 0;
     int jacobi_block = 256, traverse_block = 128;
     cudaGraph_t graph = nullptr;
@@ -456,13 +455,9 @@ lc_status lc_batch::enqueue_step(cudaStream_t st) {
     LC_PHASE(2);
     // 3. Build BVH
     LC_KEV(6);
-    launch_sort(d, tile_first, sort_passes, st);
+    launch_morton_sort(d, tile_first, morton_mode, max_T, st);
     LC_KEV(7);
-    launch_post_sort(d, st);
-    LC_CUDA(cudaMemcpyAsync(d.perm, d.perm_alt, sizeof(uint32_t) * d.Ttot, cudaMemcpyDeviceToDevice, st));
-    LC_CUDA(cudaMemsetAsync(d.parent, 0xFF, sizeof(int) * (size_t)d.Ntot, st));
-    launch_karras(d, st);
-    launch_refit(d, st);
+    launch_hierarchy(d, max_T, st);
     LC_PHASE(3);
     // 4. Create Triangle Tests
     LC_KEV(2);
@@ -687,6 +682,18 @@ static void fill_cloth_dev(const HostCloth &hc, ClothDev &cd) {
     cd.wind_var_max = p.windMaxVariation;
 }
 
+// The range tree over the leaves of C cloths of T triangles in all.
+static lc_status alloc_range_tree(lc_batch *b, int64_t T, int C) {
+    DevPtrs &d = b->d;
+    DeviceArena &A = b->arena;
+    LC_TRY(A.alloc(d.rmin, T + (int64_t)kRangePad * C, "range boxes")); LC_TRY(A.alloc(d.rmax, T + (int64_t)kRangePad * C, "range boxes"));
+    LC_TRY(A.alloc(d.far, T, "far nodes")); LC_TRY(A.alloc(d.nfar, 1, "far node count"));
+    LC_TRY(A.alloc(d.eq3, C, "equal-code flags")); LC_TRY(A.alloc(d.tree_done, C, "range tree counters"));
+    LC_CUDA(cudaMemset(d.eq3, 0, sizeof(int) * (size_t)C));
+    LC_CUDA(cudaMemset(d.tree_done, 0, sizeof(int) * (size_t)C));
+    return LC_OK;
+}
+
 static lc_status batch_build(lc_batch *b, const lc_cloth_desc *descs, int n, const lc_batch_options &opt_in) {
     lc_batch_options opt = opt_in;
     // adjoint batches: the reverse pass replays the global-memory Jacobi
@@ -745,7 +752,8 @@ static lc_status batch_build(lc_batch *b, const lc_cloth_desc *descs, int n, con
     // pair slots below 2^31: the narrowphase loops stride 32-bit pair indices
     if (V > (1ll << 31) - 2 || T > (1ll << 31) - 2 || E + B >= (1ll << 29) || PC > 0x7FFFFFFFll)
         return fail(LC_ERR_INVALID_ARG, "batch too large for 32-bit indices");
-    b->sort_passes = b->hosts[0].p.mortonMode == LC_MORTON_K30 ? 4 : 8;
+    b->morton_mode = b->hosts[0].p.mortonMode;
+    for (const HostCloth &hc : b->hosts) b->max_T = std::max(b->max_T, hc.T);
     for (int c = 0; c < n && opt.adjoint; ++c)
         if (b->cds[c].tri_bend)
             return fail(LC_ERR_NOT_SUPPORTED, "adjoint: triangle bending is not differentiated");
@@ -771,7 +779,7 @@ static lc_status batch_build(lc_batch *b, const lc_cloth_desc *descs, int n, con
     LC_TRY(A.alloc(d.x, V, "x")); LC_TRY(A.alloc(d.x2, V, "x2")); LC_TRY(A.alloc(d.xp, V, "xp"));
     LC_TRY(A.alloc(d.v, V, "v")); LC_TRY(A.alloc(d.vn, V, "vn"));
     int4 *tri; LC_TRY(A.alloc(tri, T, "tri")); d.tri = tri;
-    LC_TRY(A.alloc(d.perm, T, "perm")); LC_TRY(A.alloc(d.perm_alt, T, "perm_alt"));
+    LC_TRY(A.alloc(d.perm, T, "perm"));
     LC_TRY(A.alloc(d.tri_slot, T, "tri_slot"));
     LC_TRY(A.alloc(d.keys, T, "keys")); LC_TRY(A.alloc(d.keys_alt, T, "keys_alt"));
     LC_TRY(A.alloc(d.payload, T, "payload")); LC_TRY(A.alloc(d.payload_alt, T, "payload_alt"));
@@ -783,6 +791,7 @@ static lc_status batch_build(lc_batch *b, const lc_cloth_desc *descs, int n, con
     LC_TRY(A.alloc(d.parent, N, "parent")); LC_TRY(A.alloc(d.child, I, "child"));
     LC_TRY(A.alloc(d.rml, I, "rml"));
     LC_TRY(A.alloc(d.wnode, 4 * std::max<int64_t>(I, 1), "wnode")); LC_TRY(A.alloc(d.visit, I, "visit"));
+    LC_TRY(alloc_range_tree(b, T, n));
     LC_TRY(A.alloc(d.nend, I, "node range ends"));
     LC_TRY(A.alloc(d.rexit, 2 * std::max<int64_t>(I, 1), "refit exits")); LC_TRY(A.alloc(d.nrexit, 1, "refit exit count"));
     LC_TRY(A.alloc(d.pair_cnt, T, "pair_cnt")); LC_TRY(A.alloc(d.pair_off, T + 1, "pair_off"));
@@ -2192,19 +2201,21 @@ lc_status lc_lbvh_create(int32_t max_triangles, int32_t chunk_size, int32_t mort
     b.cds[0].morton_mode = morton_mode;
     b.cds[0].leaf_quirk = 0;
     b.cds[0].morton_scale = 1.f;
-    b.sort_passes = morton_mode == LC_MORTON_K30 ? 4 : 8;
+    b.morton_mode = morton_mode;
     d.C = 1;
     ClothDev *cdev;
     LC_TRY(A.alloc(cdev, 1, "cloth table")); d.cloth = cdev; b.cloth_dev = cdev;
     int *tcl; LC_TRY(A.alloc(tcl, T, "tcloth")); d.tcloth = tcl;
     LC_CUDA(cudaMemset(tcl, 0, sizeof(int) * T));
-    LC_TRY(A.alloc(d.perm, T, "perm")); LC_TRY(A.alloc(d.perm_alt, T, "perm_alt"));
+    LC_TRY(A.alloc(d.perm, T, "perm"));
     LC_TRY(A.alloc(d.keys, T, "keys")); LC_TRY(A.alloc(d.keys_alt, T, "keys_alt"));
     LC_TRY(A.alloc(d.payload, T, "payload")); LC_TRY(A.alloc(d.payload_alt, T, "payload_alt"));
     LC_TRY(A.alloc(d.nmin, N, "nmin")); LC_TRY(A.alloc(d.nmax, N, "nmax"));
     LC_TRY(A.alloc(d.leaf_tmp_min, T, "leaf_tmp_min")); LC_TRY(A.alloc(d.leaf_tmp_max, T, "leaf_tmp_max"));
     LC_TRY(A.alloc(d.parent, N, "parent")); LC_TRY(A.alloc(d.child, I, "child"));
     LC_TRY(A.alloc(d.rml, I, "rml")); LC_TRY(A.alloc(d.visit, I, "visit")); LC_TRY(A.alloc(d.nend, I, "node range ends"));
+    LC_TRY(alloc_range_tree(&b, T, 1));
+    LC_TRY(A.alloc(d.wnode, 4 * std::max<int64_t>(I, 1), "wnode"));
     LC_TRY(A.alloc(d.rexit, 2 * std::max<int64_t>(I, 1), "refit exits")); LC_TRY(A.alloc(d.nrexit, 1, "refit exit count"));
     LC_TRY(A.alloc(d.pair_cnt, T, "pair_cnt")); LC_TRY(A.alloc(d.pair_off, T + 1, "pair_off"));
     LC_TRY(A.alloc(d.pair_chunk, PC, "pair_chunk")); LC_TRY(A.alloc(d.pairs, PC, "pairs"));
@@ -2252,12 +2263,8 @@ lc_status lc_lbvh_build(lc_lbvh *h, const float *tri_min, const float *tri_max, 
     d.Itot = T - 1;
     LC_CUDA(cudaMemsetAsync(d.counters, 0, sizeof(unsigned long long) * 4, st));
     launch_leaves_from_boxes(d, tri_min, tri_max, T, b.cds[0].morton_mode, st);
-    launch_sort(d, b.tile_first, b.sort_passes, st);
-    launch_post_sort(d, st);
-    LC_CUDA(cudaMemcpyAsync(d.perm, d.perm_alt, sizeof(uint32_t) * T, cudaMemcpyDeviceToDevice, st));
-    LC_CUDA(cudaMemsetAsync(d.parent, 0xFF, sizeof(int) * (size_t)d.Ntot, st));
-    launch_karras(d, st);
-    launch_refit(d, st);
+    launch_morton_sort(d, b.tile_first, b.morton_mode, T, st);
+    launch_hierarchy(d, T, st);
     LC_CUDA(cudaGetLastError());
     return LC_OK;
 }

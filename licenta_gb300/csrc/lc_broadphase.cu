@@ -45,7 +45,7 @@
 #include "lc_internal.cuh"
 
 namespace lc {
-void launch_sort(const DevPtrs &d, const int *tile_first, int passes, cudaStream_t st);
+void launch_sort(const DevPtrs &d, const int *tile_first, int shift0, int passes, bool alt, cudaStream_t st);
 void set_last_error(const std::string &msg);
 
 namespace {
@@ -383,7 +383,7 @@ struct lc_broadphase {
     // sort of up to max_keys u64 keys with u32 payload (one segment)
     DevPtrs sd{};
     int *tile_first = nullptr;
-    int sort_passes = 4;
+    int sort_shift = 0;  // first bit of the 32 the sort looks at
     uint64_t max_keys = 0;
     // counts, offsets and the scan's scratch
     uint32_t *cnt = nullptr, *off = nullptr, *scan_tmp = nullptr, *total = nullptr;
@@ -433,7 +433,7 @@ struct lc_broadphase {
         LC_BP_CUDA(cudaStreamSynchronize(st));
         sd.nstiles = (int)starts.size();
         sd.Ttot = (int)std::min<uint64_t>(count, 0x7FFFFFFFull);  // the one-sweep's 30-bit count check
-        launch_sort(sd, tile_first, sort_passes, st);
+        launch_sort(sd, tile_first, sort_shift, 4, false, st);
         return LC_OK;
     }
 };
@@ -509,7 +509,9 @@ lc_status lc_broadphase_create(const lc_broadphase_desc *desc, lc_broadphase **o
         LC_TRY_BP(b.alloc(d.payload, keys, "payload"));
         LC_TRY_BP(b.alloc(d.payload_alt, keys, "payload"));
         LC_TRY_BP(b.alloc(b.tile_first, 2, "tile table"));
-        b.sort_passes = q.method == LC_BP_BVH ? 8 : 4;
+        // a BVH key's low half is the object's index, the order the stable
+        // sort starts from: 4 passes over the top half instead of 8
+        b.sort_shift = q.method == LC_BP_BVH ? 32 : 0;
     }
     if (E) LC_TRY_BP(b.alloc(b.ecell, E, "cell entries"));
     if (q.method == LC_BP_BVH) {

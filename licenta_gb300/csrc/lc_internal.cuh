@@ -16,6 +16,7 @@ constexpr int kSortBits = 8;
 constexpr int kSortBuckets = 1 << kSortBits;
 constexpr int kSortTile = 2048;          // keys per sort tile (256 threads x 8)
 constexpr int kSortPassesMax = 8;        // 8-bit digits of a 63-bit key
+constexpr int kRangePad = 32;            // range-tree entries of a cloth of T leaves: at most T + kRangePad
 constexpr int kTraverseStack = 64;       // Collision/CudaBVH.cu:38
 constexpr int kTraverseBlockMax = 256;   // largest traversal block (the packet kernel is bounded for 6 of them per SM)
 constexpr uint32_t kScanBlocks = 304;    // largest grid of the device-count scans
@@ -114,15 +115,14 @@ struct DevPtrs {
     float4 *vn;            // running vertex normals
     const int4 *tri;       // original triangle -> (v1, v2, v3 global ids, features)
     uint32_t *perm;        // slot -> original triangle (global)
-    uint32_t *perm_alt;
     int4 *tri_slot;        // slot -> its triangle record (tri[perm[slot]]), written after each sort
     unsigned long long *keys, *keys_alt;
-    uint32_t *payload, *payload_alt;  // pre-sort slot carried through the sort
+    uint32_t *payload, *payload_alt;  // original triangle carried through the sort
     float4 *fn;            // face normal per original triangle
     const int *vt_off;     // vertex -> incident original triangles (CSR)
     const int *vt_idx;
     float4 *nmin, *nmax;   // node AABBs
-    float4 *leaf_tmp_min, *leaf_tmp_max;  // pre-sort leaf boxes (fixed mode)
+    float4 *leaf_tmp_min, *leaf_tmp_max;  // leaf boxes by original triangle (fixed mode)
     int *parent;
     int2 *child;
     int2 *rml;
@@ -130,6 +130,11 @@ struct DevPtrs {
     int *nend;             // per internal node: the other end j of its leaf range (may be null)
     int2 *rexit;           // refit: (cloth, node) arrivals left for the upper pass (2 x internal nodes)
     uint32_t *nrexit;      // their count (cleared by k_karras)
+    int *far;              // slots of the nodes k_karras leaves to k_karras_far, and their count
+    uint32_t *nfar;
+    float4 *rmin, *rmax;   // aligned ranges of leaves, level by level from two leaves up: a cloth's at t_off + kRangePad c
+    int *eq3;              // per cloth: three equal codes meet in the step's order (null: no range tree, the climb for all)
+    int *tree_done;        // per cloth: blocks of k_range_tree that finished (zero between launches)
     float4 *wnode;         // 4 per internal node: {lmin, left} {lmax, rmll} {rmin, right} {rmax, rmlr} (may be null)
     uint32_t *pair_cnt;    // per slot
     uint32_t *pair_off;    // per slot (exclusive scan), + total at [Ttot]

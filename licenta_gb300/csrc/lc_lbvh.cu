@@ -6,9 +6,13 @@
 // roundings of the reference kernels, so Morton codes, tree topology, pair
 // lists and contact lists are bit-exact against the FP32 oracle for the
 // same input positions.
+#include <algorithm>
+#include <cooperative_groups.h>
 #include <cuda/atomic>
 
 #include "lc_internal.cuh"
+
+namespace cg = cooperative_groups;
 
 namespace lc {
 
@@ -52,7 +56,10 @@ unsigned long long morton3_host(float x, float y, float z, int mode) { return mo
 // Triangle update: Physics/CudaDeformableUtils.cu:120-151.  One thread per
 // slot; the swept, thickness-inflated box goes to leaf (T-1+slot) — the
 // pre-sort slot, which is the reference's leaf-AABB quirk — or to a
-// temporary that the post-sort gather places under the sorted leaf.
+// temporary, by original triangle, that the post-sort gather places under the
+// sorted leaf.  The keys, with the original triangle as payload, start in the
+// alternate buffers: after an even number of passes they are there again, and
+// the post-sort writes the final order to keys and perm.
 // ---------------------------------------------------------------------------
 __global__ void k_triangles(DevPtrs d) {
     const int s = blockIdx.x * blockDim.x + threadIdx.x;
@@ -74,15 +81,17 @@ __global__ void k_triangles(DevPtrs d) {
         d.nmin[node] = f4(smn, 0.f);
         d.nmax[node] = f4(smx, 0.f);
     } else {
-        d.leaf_tmp_min[s] = f4(smn, 0.f);
-        d.leaf_tmp_max[s] = f4(smx, 0.f);
+        d.leaf_tmp_min[orig] = f4(smn, 0.f);
+        d.leaf_tmp_max[orig] = f4(smx, 0.f);
     }
+    if (local == 0 && d.eq3) d.eq3[c] = 0;
+    if (s == 0) *d.nfar = 0;
     const float3 mid = add(smn, dvs(sub(smx, smn), 2.f));
     const float qx = (mid.x - cd.morton_origin[0]) * cd.morton_scale;
     const float qy = (mid.y - cd.morton_origin[1]) * cd.morton_scale;
     const float qz = (mid.z - cd.morton_origin[2]) * cd.morton_scale;
-    d.keys[s] = morton3(qx, qy, qz, cd.morton_mode);
-    d.payload[s] = (uint32_t)local;
+    d.keys_alt[s] = morton3(qx, qy, qz, cd.morton_mode);
+    d.payload_alt[s] = orig;
 }
 
 // Standalone LBVH: leaf boxes supplied by the caller (one cloth, T slots).
@@ -95,9 +104,10 @@ __global__ void k_leaves_from_boxes(DevPtrs d, const float *__restrict__ bmin, c
     d.leaf_tmp_min[s] = f4(mn, 0.f);
     d.leaf_tmp_max[s] = f4(mx, 0.f);
     const float3 mid = add(mn, dvs(sub(mx, mn), 2.f));
-    d.keys[s] = morton3(mid.x, mid.y, mid.z, mode);
-    d.payload[s] = (uint32_t)s;
-    d.perm[s] = (uint32_t)s;
+    d.keys_alt[s] = morton3(mid.x, mid.y, mid.z, mode);
+    d.payload_alt[s] = (uint32_t)s;
+    if (s == 0 && d.eq3) d.eq3[0] = 0;
+    if (s == 0) *d.nfar = 0;
 }
 
 // ---------------------------------------------------------------------------
@@ -184,7 +194,7 @@ constexpr uint32_t kStatAgg = 1u << 30, kStatPre = 2u << 30, kStatCount = kStatA
 constexpr uint32_t kLookbackSpins = 1u << 22;  // bound on the status waits of one look-back (then ERR_SORT)
 constexpr int kLookbackWindow = 8;               // earlier tiles' statuses read per look-back step
 __global__ void __launch_bounds__(kThreads) k_sort_hist_all(DevPtrs d, const unsigned long long *__restrict__ keys,
-                                                            int passes) {
+                                                            int shift0, int passes) {
     static_assert(kThreads == kSortBuckets, "one thread per digit");
     constexpr int R = kSortTile / kThreads;
     __shared__ uint32_t h[kSortPassesMax][kSortBuckets];
@@ -206,7 +216,7 @@ __global__ void __launch_bounds__(kThreads) k_sort_hist_all(DevPtrs d, const uns
         for (int p = 0; p < passes; ++p) {
             // a digit common to the whole warp (the high digits of nearby
             // Morton codes) is one atomic; otherwise one per lane
-            const uint32_t dig = valid ? (uint32_t)(key >> (p * kSortBits)) & (kSortBuckets - 1) : kSortBuckets;
+            const uint32_t dig = valid ? (uint32_t)(key >> (shift0 + p * kSortBits)) & (kSortBuckets - 1) : kSortBuckets;
             const uint32_t d0 = __shfl_sync(0xffffffffu, dig, 0);
             if (__all_sync(0xffffffffu, dig == d0)) {
                 if (lane == 0 && d0 < kSortBuckets) atomicAdd(&h[p][d0], 32u);
@@ -219,6 +229,21 @@ __global__ void __launch_bounds__(kThreads) k_sort_hist_all(DevPtrs d, const uns
     uint32_t *seg = d.sseg + kSortPassesMax + (size_t)c * kSortPassesMax * kSortBuckets;
     for (int p = 0; p < passes; ++p)
         if (h[p][t]) atomicAdd(&seg[p * kSortBuckets + t], h[p][t]);
+}
+
+// Lanes of the warp whose digit equals this one's: eight votes, one per bit of
+// the digit.  __match_any_sync gives the same mask in one instruction, but a
+// sort pass is bound by its rate: a sort in one launch of 1922, 7938 or 20 k
+// keys took 19, 46 and 44 us with it, 17, 42 and 40 us so.
+__device__ __forceinline__ uint32_t digit_peers(uint32_t dig) {
+    uint32_t peers = 0xffffffffu;
+#pragma unroll
+    for (int b = 0; b < kSortBits; ++b) {
+        const bool bit = (dig >> b) & 1u;
+        const uint32_t v = __ballot_sync(0xffffffffu, bit);
+        peers &= bit ? v : ~v;
+    }
+    return peers;
 }
 
 // One tile per block, ranked without block-wide rounds: warp w takes the
@@ -272,8 +297,8 @@ __global__ void __launch_bounds__(kThreads, 4) k_sort_scatter(DevPtrs d, const u
         const bool valid = li < n;
         kr[r] = valid ? kin[start + li] : 0ull;
         pr[r] = valid ? pin[start + li] : 0u;
-        const uint32_t dig = valid ? (uint32_t)(kr[r] >> shift) & (kSortBuckets - 1) : kSortBuckets;
-        const uint32_t peers = __match_any_sync(0xffffffffu, dig);
+        const uint32_t dig = (uint32_t)(kr[r] >> shift) & (kSortBuckets - 1);
+        const uint32_t peers = digit_peers(dig) & __ballot_sync(0xffffffffu, valid);
         const uint32_t before = valid ? wcnt[wid][dig] : 0u;
         rk[r] = before + __popc(peers & lt_mask);
         __syncwarp();
@@ -396,45 +421,542 @@ __global__ void __launch_bounds__(kThreads, 4) k_sort_scatter(DevPtrs d, const u
     }
 }
 
-// After the sort: new triangle order and (fixed mode) leaf boxes gathered by
-// the permutation.
-__global__ void k_post_sort(DevPtrs d) {
+// ---------------------------------------------------------------------------
+// The low half of 63-bit keys.  The passes above sort such keys by their top
+// half only (bits 32..62, about a millimetre of a metre per axis): half the
+// passes.  Keys that share it stay in their order before the sort, in runs
+// that are almost always of one or two keys; the post-sort ranks the keys of
+// a run of at most kTieRun by (low half, position), which completes the stable
+// sort, and longer runs are radix-sorted in place by one block each before it.
+// A sort of a million keys: 8 passes and the histogram 178 us, 4 passes, the
+// long-run search and the ranks 100 us.
+// ---------------------------------------------------------------------------
+constexpr int kTieRun = 64;
+__device__ __forceinline__ uint32_t top_half(unsigned long long k) { return (uint32_t)(k >> 32); }
+
+// Stable sort of the keys [a, e) (with payload) by their low half, one block,
+// 8-bit digits, through the other buffer; the result is where it started.
+__device__ void sort_run(unsigned long long *k0, uint32_t *p0, unsigned long long *k1, uint32_t *p1, int a, int e) {
+    __shared__ uint32_t hist[kSortBuckets], base[kSortBuckets], wcnt[kThreads / 32][kSortBuckets], wsum[kThreads / 32];
+    static_assert(kThreads == kSortBuckets, "one thread per digit");
+    const int t = threadIdx.x, lane = t & 31, wid = t >> 5;
+    for (int p = 0; p < 4; ++p) {
+        const int shift = p * kSortBits;
+        __syncthreads();
+        hist[t] = 0;
+        __syncthreads();
+        for (int i = a + t; i < e; i += kThreads) atomicAdd(&hist[(uint32_t)(k0[i] >> shift) & (kSortBuckets - 1)], 1u);
+        __syncthreads();
+        uint32_t incl = hist[t];
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const uint32_t v = __shfl_up_sync(0xffffffffu, incl, o);
+            if (lane >= o) incl += v;
+        }
+        if (lane == 31) wsum[wid] = incl;
+        __syncthreads();
+        uint32_t run = (uint32_t)a + incl - hist[t];
+        for (int w = 0; w < wid; ++w) run += wsum[w];
+        base[t] = run;
+        for (int i0 = a; i0 < e; i0 += kThreads) {  // tiles in order: index order is (warp, lane)
+#pragma unroll
+            for (int w = 0; w < kThreads / 32; ++w) wcnt[w][t] = 0;
+            __syncthreads();
+            const int i = i0 + t;
+            const bool valid = i < e;
+            const unsigned long long key = valid ? k0[i] : 0ull;
+            const uint32_t dig = valid ? (uint32_t)(key >> shift) & (kSortBuckets - 1) : kSortBuckets;
+            const uint32_t peers = __match_any_sync(0xffffffffu, dig);
+            const uint32_t rank = __popc(peers & ((1u << lane) - 1u));
+            if (valid && rank == 0) wcnt[wid][dig] = __popc(peers);
+            __syncthreads();
+            uint32_t b = base[t];
+#pragma unroll
+            for (int w = 0; w < kThreads / 32; ++w) {
+                const uint32_t c = wcnt[w][t];
+                wcnt[w][t] = b;
+                b += c;
+            }
+            base[t] = b;
+            __syncthreads();
+            if (valid) {
+                const uint32_t o = wcnt[wid][dig] + rank;
+                k1[o] = key;
+                p1[o] = p0[i];
+            }
+            __syncthreads();
+        }
+        unsigned long long *tk = k0; k0 = k1; k1 = tk;
+        uint32_t *tp = p0; p0 = p1; p1 = tp;
+    }
+    __syncthreads();
+}
+
+// Runs longer than kTieRun: the thread of a run's first slot finds it, its
+// block sorts it unless it is in order already (equal codes are).
+__global__ void __launch_bounds__(kThreads) k_sort_long_runs(DevPtrs d) {
+    __shared__ int q_first[kThreads], q_end[kThreads], s_n;
+    const int s = blockIdx.x * kThreads + threadIdx.x;
+    if (threadIdx.x == 0) s_n = 0;
+    __syncthreads();
+    if (s < d.Ttot) {
+        const ClothDev &cd = d.cloth[d.tcloth[s]];
+        const int end = cd.t_off + cd.T;
+        if (s + kTieRun < end) {
+            const uint32_t top = top_half(d.keys_alt[s]);
+            if (top_half(d.keys_alt[s + kTieRun]) == top && (s == cd.t_off || top_half(d.keys_alt[s - 1]) != top)) {
+                int lo = s + kTieRun, hi = end;  // keys [s, lo] have this top half, hi has not (or is the end)
+                while (hi - lo > 1) {
+                    const int m = lo + (hi - lo) / 2;
+                    if (top_half(d.keys_alt[m]) == top) lo = m;
+                    else hi = m;
+                }
+                const int k = atomicAdd(&s_n, 1);
+                q_first[k] = s;
+                q_end[k] = hi;
+            }
+        }
+    }
+    __syncthreads();
+    for (int k = 0; k < s_n; ++k) {
+        const int a = q_first[k], e = q_end[k];
+        bool wrong = false;
+        for (int i = a + threadIdx.x; i + 1 < e; i += kThreads) wrong = wrong || d.keys_alt[i] > d.keys_alt[i + 1];
+        if (__syncthreads_or(wrong)) sort_run(d.keys_alt, d.payload_alt, d.keys, d.payload, a, e);
+    }
+}
+
+// A sorted slot's outputs: key, triangle order and record, (fixed mode) the
+// leaf box, and no parents yet.
+__device__ __forceinline__ void put_slot(const DevPtrs &d, const ClothDev &cd, int s, unsigned long long key,
+                                         uint32_t orig) {
+    d.keys[s] = key;
+    d.perm[s] = orig;
+    if (d.tri_slot) d.tri_slot[s] = d.tri[orig];  // one gather per slot instead of two per pair
+    const int local = s - cd.t_off, leaf = cd.n_off + (cd.T - 1) + local;
+    if (!cd.leaf_quirk) {
+        d.nmin[leaf] = d.leaf_tmp_min[orig];
+        d.nmax[leaf] = d.leaf_tmp_max[orig];
+    }
+    d.parent[leaf] = -1;
+    if (local < cd.T - 1) d.parent[cd.n_off + local] = -1;
+}
+
+// The final place of slot s's key in its run of equal top halves (keys in
+// [first, end), sorted by top half), and whether three equal keys meet in it.
+template <class Keys>
+__device__ __forceinline__ int tie_place(const Keys &keys, int s, int first, int end, unsigned long long key,
+                                         bool &three) {
+    const uint32_t top = top_half(key);
+    int a = s, e = s + 1;
+    while (a > first && s - a < kTieRun && top_half(keys[a - 1]) == top) --a;
+    while (e < end && e - s <= kTieRun && top_half(keys[e]) == top) ++e;
+    if (e - a > kTieRun) {  // sorted in place already
+        three = s > first && s + 1 < end && keys[s - 1] == key && keys[s + 1] == key;
+        return s;
+    }
+    int r = a, same = 0;
+    for (int j = a; j < e; ++j) {
+        const unsigned long long q = keys[j];
+        r += q < key || (q == key && j < s);
+        same += q == key;
+    }
+    three = same >= 3;
+    return r;
+}
+
+// After the sort: the low halves (halves != 0), the new triangle order and the
+// cloths in which three equal codes meet (their hierarchy may be malformed).
+__global__ void k_post_sort(DevPtrs d, int halves) {
     const int s = blockIdx.x * blockDim.x + threadIdx.x;
     if (s >= d.Ttot) return;
     const int c = d.tcloth[s];
     const ClothDev &cd = d.cloth[c];
-    const int src = cd.t_off + (int)d.payload[s];
-    const uint32_t orig = d.perm[src];
-    d.perm_alt[s] = orig;
-    if (d.tri_slot) d.tri_slot[s] = d.tri[orig];  // one gather per slot instead of two per pair
-    if (!cd.leaf_quirk) {
-        const int node = cd.n_off + (cd.T - 1) + (s - cd.t_off);
-        d.nmin[node] = d.leaf_tmp_min[src];
-        d.nmax[node] = d.leaf_tmp_max[src];
+    const int first = cd.t_off, end = cd.t_off + cd.T;
+    const unsigned long long key = d.keys_alt[s];
+    const unsigned long long prev = s > first ? d.keys_alt[s - 1] : ~key, next = s + 1 < end ? d.keys_alt[s + 1] : ~key;
+    int place = s;
+    bool three = prev == key && next == key;
+    if (halves && (top_half(prev) == top_half(key) || top_half(next) == top_half(key)))
+        place = tie_place(d.keys_alt, s, first, end, key, three);
+    if (three && d.eq3) d.eq3[c] = 1;
+    put_slot(d, cd, place, key, d.payload_alt[s]);
+}
+
+// Segments of at most CS R 1024 keys: sort and post-sort in one launch, one
+// cluster of CS CTAs per segment, every key in a register or in shared memory
+// throughout.  A key moves as one word, the 32 bits sorted by over its position
+// before the sort; a pass ranks the CTA's keys per warp, exchanges the CTAs'
+// digit counts and stores each key straight into the shared memory of the CTA
+// that holds its place.  The full keys and payloads are fetched by position at
+// the end.  Bound by barriers and by one SM's rate of ranking (5 us per 1024
+// keys and four passes in one CTA), hence CTAs rather than keys per thread
+// where few segments leave SMs idle.
+constexpr int kSmallThreads = 1024;
+constexpr int kSmallCtas = 8;
+template <int CS, int R>
+struct SegmentSort {
+    static constexpr int W = kSmallThreads / 32, N = R * kSmallThreads;  // warps and keys per CTA
+    static constexpr size_t kSmem = (size_t)N * 8 + (size_t)W * kSortBuckets * 4;
+};
+__device__ __forceinline__ uint32_t shared_of(const void *p, int rank) {
+    uint32_t a;
+    asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"((uint32_t)__cvta_generic_to_shared(p)), "r"(rank));
+    return a;
+}
+template <int CS, int R>
+__global__ void __launch_bounds__(kSmallThreads) k_sort_segment(DevPtrs d, int halves) {
+    using S = SegmentSort<CS, R>;
+    constexpr int W = S::W, N = S::N;
+    extern __shared__ unsigned long long s_key[];                                               // N
+    uint32_t(*wcnt)[kSortBuckets] = reinterpret_cast<uint32_t(*)[kSortBuckets]>(s_key + N);    // per warp and digit
+    __shared__ uint32_t qsum[4][kSortBuckets], ctot[kSortBuckets], s_base[kSortBuckets], wsum[kSortBuckets / 32];
+    __shared__ int s_long;
+    cg::cluster_group cluster = cg::this_cluster();
+    const int rank = CS > 1 ? (int)cluster.block_rank() : 0;
+    const int t = threadIdx.x, lane = t & 31, wid = t >> 5;
+    const int dig0 = t & (kSortBuckets - 1), q0 = t / kSortBuckets;  // digit and quarter of the warps
+    const int c = blockIdx.x / CS;
+    const ClothDev &cd = d.cloth[c];
+    const int n = cd.T, off = cd.t_off, first = rank * N;            // this CTA's first place
+    auto barrier = [&]() {
+        if (CS > 1) cluster.sync();
+        else __syncthreads();
+    };
+    auto place_of = [&](int r) { return wid * 32 * R + r * 32 + lane; };  // index order is (warp, step, lane)
+    unsigned long long w[R];
+    uint32_t rk[R];
+    // bits sorted by (the top or the low half) over the position
+    auto word = [&](int pos, bool top) {
+        const unsigned long long k = d.keys_alt[off + pos];
+        return (top ? k & 0xffffffff00000000ull : k << 32) | (unsigned)pos;
+    };
+    auto pass = [&](int shift) {
+        for (int k = t; k < W * kSortBuckets; k += kSmallThreads) (&wcnt[0][0])[k] = 0;
+        __syncthreads();
+        const uint32_t below = (1u << lane) - 1u;
+#pragma unroll
+        for (int r = 0; r < R; ++r) {  // ranks among the warp's earlier keys of the digit
+            const uint32_t dig = (uint32_t)(w[r] >> shift) & (kSortBuckets - 1);
+            const uint32_t peers = digit_peers(dig);
+            const uint32_t before = wcnt[wid][dig];
+            rk[r] = before + __popc(peers & below);
+            __syncwarp();
+            if ((peers & below) == 0) wcnt[wid][dig] = before + __popc(peers);
+            __syncwarp();
+        }
+        __syncthreads();
+        uint32_t part = 0;
+#pragma unroll
+        for (int k = 0; k < W / 4; ++k) part += wcnt[q0 * (W / 4) + k][dig0];
+        qsum[q0][dig0] = part;
+        __syncthreads();
+        uint32_t mine = 0, all = 0, before = 0;
+        if (q0 == 0) ctot[dig0] = mine = qsum[0][dig0] + qsum[1][dig0] + qsum[2][dig0] + qsum[3][dig0];
+        barrier();  // counts published, and every CTA's keys are in registers
+        if (q0 == 0) {
+            all = mine;
+            if (CS > 1) {
+                all = 0;
+#pragma unroll
+                for (int k = 0; k < CS; ++k) {
+                    uint32_t v;
+                    asm volatile("ld.shared::cluster.u32 %0, [%1];" : "=r"(v) : "r"(shared_of(&ctot[dig0], k)) : "memory");
+                    before += k < rank ? v : 0u;
+                    all += v;
+                }
+            }
+            uint32_t incl = all;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const uint32_t v = __shfl_up_sync(0xffffffffu, incl, o);
+                if (lane >= o) incl += v;
+            }
+            if (lane == 31) wsum[dig0 / 32] = incl;
+            s_base[dig0] = incl - all + before;
+        }
+        __syncthreads();
+        uint32_t run = s_base[dig0];
+#pragma unroll
+        for (int k = 0; k < kSortBuckets / 32; ++k) run += k < dig0 / 32 ? wsum[k] : 0u;
+#pragma unroll
+        for (int k = 0; k < 3; ++k) run += k < q0 ? qsum[k][dig0] : 0u;
+#pragma unroll
+        for (int k = 0; k < W / 4; ++k) {
+            uint32_t &slot = wcnt[q0 * (W / 4) + k][dig0];
+            const uint32_t v = slot;
+            slot = run;
+            run += v;
+        }
+        __syncthreads();
+#pragma unroll
+        for (int r = 0; r < R; ++r) {
+            const uint32_t pos = wcnt[wid][(uint32_t)(w[r] >> shift) & (kSortBuckets - 1)] + rk[r];
+            if (CS > 1)
+                asm volatile("st.shared::cluster.u64 [%0], %1;"
+                             : : "r"(shared_of(s_key, (int)(pos / N)) + 8u * (pos % N)), "l"(w[r]) : "memory");
+            else
+                s_key[pos] = w[r];
+        }
+        barrier();
+#pragma unroll
+        for (int r = 0; r < R; ++r) w[r] = s_key[place_of(r)];
+    };
+    // places past the segment hold words above every key of it: they stay last
+#pragma unroll
+    for (int r = 0; r < R; ++r) w[r] = first + place_of(r) < n ? word(first + place_of(r), halves != 0) : ~0ull;
+    for (int p = 0; p < 4; ++p) pass(32 + p * kSortBits);
+    if (halves) {  // a long run of equal top halves: by low half first, then by top half again
+        if (t == 0) s_long = 0;
+        __syncthreads();
+#pragma unroll
+        for (int r = 0; r < R; ++r) {
+            const int i = place_of(r);  // a run longer than kTieRun has over half of that in one CTA
+            if (i + kTieRun / 2 < N && first + i + kTieRun / 2 < n && top_half(s_key[i]) == top_half(s_key[i + kTieRun / 2])) s_long = 1;
+        }
+        barrier();
+        bool any = s_long != 0;
+        if (CS > 1) {
+#pragma unroll
+            for (int k = 0; k < CS; ++k) {
+                int v;
+                asm volatile("ld.shared::cluster.s32 %0, [%1];" : "=r"(v) : "r"(shared_of(&s_long, k)) : "memory");
+                any = any || v != 0;
+            }
+        }
+        if (any)
+            for (int half = 0; half < 2; ++half) {
+#pragma unroll
+                for (int r = 0; r < R; ++r) {
+                    const int i = first + place_of(r);
+                    const int pos = half ? (int)(uint32_t)w[r] : i;
+                    w[r] = i < n ? word(pos, half != 0) : ~0ull;
+                }
+                for (int p = 0; p < 4; ++p) pass(32 + p * kSortBits);
+            }
     }
+    barrier();
+    // full keys by place, for the runs of equal top halves
+    unsigned long long key[R];
+    uint32_t pay[R];
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+        const bool have = first + place_of(r) < n;
+        const int pos = (int)(uint32_t)w[r];
+        key[r] = have ? d.keys_alt[off + pos] : ~0ull;
+        pay[r] = have ? d.payload_alt[off + pos] : 0u;
+        s_key[place_of(r)] = key[r];
+    }
+    barrier();
+    struct Keys {  // by place in the segment
+        const unsigned long long *own;
+        int rank;
+        __device__ __forceinline__ unsigned long long operator[](int i) const {
+            if (CS == 1 || i / N == rank) return own[i % N];
+            unsigned long long v;
+            asm volatile("ld.shared::cluster.u64 %0, [%1];" : "=l"(v) : "r"(shared_of(own, i / N) + 8u * (i % N)) : "memory");
+            return v;
+        }
+    };
+    const Keys keys{s_key, rank};
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+        const int i = first + place_of(r);
+        if (i >= n) continue;
+        const unsigned long long prev = i > 0 ? keys[i - 1] : ~key[r], next = i + 1 < n ? keys[i + 1] : ~key[r];
+        int place = i;
+        bool three = prev == key[r] && next == key[r];
+        if (halves && (top_half(prev) == top_half(key[r]) || top_half(next) == top_half(key[r])))
+            place = tie_place(keys, i, 0, n, key[r], three);
+        if (three && d.eq3) d.eq3[c] = 1;
+        put_slot(d, cd, off + place, key[r], pay[r]);
+    }
+    barrier();  // no CTA leaves while another reads its keys
 }
 
 // ---------------------------------------------------------------------------
 // Karras hierarchy: Collision/CudaBVH.cu:163-242, Core/CudaUtils.cu:338-362.
 // ---------------------------------------------------------------------------
-__device__ __forceinline__ int delta(const unsigned long long *__restrict__ m, int i, int j, int maxi) {
+// A cloth's sorted keys by local index, as far as the block's own slots and one
+// on each side go; an access beyond them only sets `out`.
+struct BlockKeys {
+    const unsigned long long *own;  // shared: slots [b0 - 1, b0 + n]
+    int b0, n;                      // local index of the block's first slot (negative: it begins in an earlier cloth), slots
+    mutable bool out;
+    __device__ __forceinline__ unsigned long long operator[](int i) const {
+        const unsigned k = (unsigned)(i - b0 + 1);
+        if (k < (unsigned)n + 2u) return own[k];
+        out = true;
+        return 0ull;
+    }
+};
+template <class Keys>
+__device__ __forceinline__ int delta(const Keys &m, int i, int j, int maxi) {
     if (j < 0 || j > maxi) return -1;
     const unsigned long long x = m[i] ^ m[j];
     return x ? __clzll((long long)x) : __clzll((long long)((unsigned long long)i ^ (unsigned long long)j)) + 64;
 }
 __device__ __forceinline__ int sgn_ref(int a) { return signbit((float)a) ? -1 : 1; }
 
-__global__ void k_karras(DevPtrs d) {
-    const int s = blockIdx.x * blockDim.x + threadIdx.x;
-    if (s == 0 && d.nrexit) *d.nrexit = 0;  // k_refit_local appends to it
-    if (s >= d.Ttot) return;
-    const int c = d.tcloth[s];
+// ---------------------------------------------------------------------------
+// Node boxes without a climb.  A node's box is the union of the leaf boxes in
+// its range, and min / max are exact, so any grouping gives the bits of the
+// bottom-up refit: a binary tree over aligned runs of leaves (level k's entry j
+// holds the union of the leaves [j 2^k, (j + 1) 2^k)) answers every range with
+// at most two entries per level, and half of the nodes need two or three leaf
+// boxes.  k_range_tree builds it with one block per 2048 leaves (levels 1..11)
+// and the last block of a cloth the levels above; k_karras then writes every
+// node complete, the traversal's record included.  The climb was bound by its
+// chain of arrivals to the root, 31 us for 1922 triangles as for a million.
+// From codes to records (us; cloths of 1922, 20 k and 522 k triangles, 30 cloths
+// of 620 k, 64 of 1.92 M, a million random boxes): 60, 74, 124, 143, 272, 179
+// with the climb, 28, 54, 93, 102, 219, 173 so.
+// Cloths in which three equal codes meet keep the climb (below): there the
+// reference's hierarchy may not be a tree, and which nodes it reaches counts.
+// ---------------------------------------------------------------------------
+constexpr int kTreeTop = 512;  // nodes of a level that one block combines in shared memory
+__device__ __forceinline__ int half_up(int n) { return (n + 1) >> 1; }
+constexpr int kTreeThreads = 512;
+__global__ void __launch_bounds__(kTreeThreads) k_range_tree(DevPtrs d) {
+    static_assert(kSortTile == 4 * kTreeThreads, "levels 1..5 per warp, 6..11 over 64 warp results");
+    __shared__ float4 s_min[kTreeTop], s_max[kTreeTop];
+    __shared__ int s_last;
+    const int c = d.stile_cloth[blockIdx.x];
     const ClothDev &cd = d.cloth[c];
-    const int id = s - cd.t_off;
-    const int In = cd.T - 1;
-    if (id >= In) return;
-    const unsigned long long *m = d.keys + cd.t_off;
-    // FindRange
+    if (d.eq3[c]) return;
+    const int T = cd.T, first = d.stile_start[blockIdx.x] - cd.t_off;  // local first leaf of the tile
+    const int t = threadIdx.x, lane = t & 31;
+    const float4 *lmin = d.nmin + cd.n_off + (T - 1), *lmax = d.nmax + cd.n_off + (T - 1);
+    float4 *rmin = d.rmin + cd.t_off + kRangePad * c, *rmax = d.rmax + cd.t_off + kRangePad * c;
+    for (int q = 0; q < 4; ++q) {
+        const int li = first + q * kTreeThreads + t;
+        if (first + q * kTreeThreads >= T) break;
+        float3 mn = f3(0.f, 0.f, 0.f), mx = mn;
+        if (li < T) { mn = xyz(lmin[li]); mx = xyz(lmax[li]); }
+        int off = 0, n = T;
+#pragma unroll
+        for (int k = 1; k <= 5; ++k) {
+            const int o = 1 << (k - 1);
+            const float3 a = f3(__shfl_down_sync(0xffffffffu, mn.x, o), __shfl_down_sync(0xffffffffu, mn.y, o),
+                                __shfl_down_sync(0xffffffffu, mn.z, o));
+            const float3 b = f3(__shfl_down_sync(0xffffffffu, mx.x, o), __shfl_down_sync(0xffffffffu, mx.y, o),
+                                __shfl_down_sync(0xffffffffu, mx.z, o));
+            if ((lane & (2 * o - 1)) == 0 && li < T) {
+                if (li + o < T) { mn = vmin(mn, a); mx = vmax(mx, b); }
+                rmin[off + (li >> k)] = f4(mn, 0.f);
+                rmax[off + (li >> k)] = f4(mx, 0.f);
+            }
+            n = half_up(n);
+            off += n;
+        }
+        if (lane == 0 && li < T) { s_min[q * 16 + (t >> 5)] = f4(mn, 0.f); s_max[q * 16 + (t >> 5)] = f4(mx, 0.f); }
+    }
+    int off = 0, n = T;  // after level k: off = where level k + 1 starts, n = level k's entries
+    for (int k = 1; k <= 5; ++k) { n = half_up(n); off += n; }
+    __syncthreads();
+    if (t < 32) {
+        for (int k = 6; k <= 11; ++k) {
+            const int j = t, per = 1 << k;
+            const bool mine = j < (kSortTile >> k) && first + j * per < T;
+            float3 mn = f3(0.f, 0.f, 0.f), mx = mn;
+            if (mine) {
+                mn = xyz(s_min[2 * j]); mx = xyz(s_max[2 * j]);
+                if (first + j * per + per / 2 < T) { mn = vmin(mn, xyz(s_min[2 * j + 1])); mx = vmax(mx, xyz(s_max[2 * j + 1])); }
+                rmin[off + (first >> k) + j] = f4(mn, 0.f);
+                rmax[off + (first >> k) + j] = f4(mx, 0.f);
+            }
+            __syncwarp();
+            if (mine) { s_min[j] = f4(mn, 0.f); s_max[j] = f4(mx, 0.f); }
+            __syncwarp();
+            n = half_up(n);
+            off += n;
+        }
+    }
+    if (T <= kSortTile) return;
+    // the last of the cloth's blocks to finish builds the levels above
+    if (t == 0) {
+        __threadfence();
+        s_last = atomicAdd(&d.tree_done[c], 1) == (T + kSortTile - 1) / kSortTile - 1;
+        if (s_last) d.tree_done[c] = 0;
+    }
+    __syncthreads();
+    if (!s_last) return;
+    __threadfence();
+    off = 0;
+    n = T;
+    int prev = 0;
+    for (int k = 1; k <= 11; ++k) { prev = off; n = half_up(n); off += n; }  // prev: where level 11 starts
+    while (n > kTreeTop) {  // more than a million leaves: level by level through memory
+        const int m = half_up(n);
+        for (int j = t; j < m; j += kTreeThreads) {
+            float3 mn = xyz(__ldcg(&rmin[prev + 2 * j])), mx = xyz(__ldcg(&rmax[prev + 2 * j]));
+            if (2 * j + 1 < n) {
+                mn = vmin(mn, xyz(__ldcg(&rmin[prev + 2 * j + 1])));
+                mx = vmax(mx, xyz(__ldcg(&rmax[prev + 2 * j + 1])));
+            }
+            rmin[off + j] = f4(mn, 0.f);
+            rmax[off + j] = f4(mx, 0.f);
+        }
+        __threadfence();
+        __syncthreads();
+        prev = off;
+        off += m;
+        n = m;
+    }
+    for (int j = t; j < n; j += kTreeThreads) { s_min[j] = __ldcg(&rmin[prev + j]); s_max[j] = __ldcg(&rmax[prev + j]); }
+    __syncthreads();
+    while (n > 1) {
+        const int m = half_up(n);
+        float3 mn = f3(0.f, 0.f, 0.f), mx = mn;
+        const int j = t;  // m <= kTreeTop / 2 = one entry per thread
+        if (j < m) {
+            mn = xyz(s_min[2 * j]); mx = xyz(s_max[2 * j]);
+            if (2 * j + 1 < n) { mn = vmin(mn, xyz(s_min[2 * j + 1])); mx = vmax(mx, xyz(s_max[2 * j + 1])); }
+            rmin[off + j] = f4(mn, 0.f);
+            rmax[off + j] = f4(mx, 0.f);
+        }
+        __syncthreads();
+        if (j < m) { s_min[j] = f4(mn, 0.f); s_max[j] = f4(mx, 0.f); }
+        __syncthreads();
+        off += m;
+        n = m;
+    }
+}
+
+// Union of the leaf boxes [a, b]: each level takes the range's first and last
+// entry, whether or not the level above covers them (taking a box twice
+// changes nothing), so there is no branch on them.  n leaves at lmin / lmax,
+// the levels above at rmin / rmax.
+__device__ __forceinline__ void range_box(const float4 *lmin, const float4 *lmax, const float4 *rmin, const float4 *rmax,
+                                          int n, int a, int b, float3 &mn, float3 &mx) {
+    mn = vmin(xyz(lmin[a]), xyz(lmin[b]));
+    mx = vmax(xyz(lmax[a]), xyz(lmax[b]));
+    int l = a, r = b;  // this level's entries l .. r
+    while (r - l > 1) {
+        l = (l + 1) >> 1;
+        r = (r - 1) >> 1;
+        if (l > r) break;
+        mn = vmin(mn, vmin(xyz(rmin[l]), xyz(rmin[r])));
+        mx = vmax(mx, vmax(xyz(rmax[l]), xyz(rmax[r])));
+        n = half_up(n);
+        rmin += n;
+        rmax += n;
+    }
+}
+
+__device__ __forceinline__ void put_wnode(const DevPtrs &d, size_t node, float3 lmn, float3 lmx, float3 rmn, float3 rmx,
+                                          int2 ch, int2 rm) {
+    float4 *w = d.wnode + 4 * node;
+    w[0] = f4(lmn, __int_as_float(ch.x));
+    w[1] = f4(lmx, __int_as_float(rm.x));
+    w[2] = f4(rmn, __int_as_float(ch.y));
+    w[3] = f4(rmx, __int_as_float(rm.y));
+}
+
+// Range and split of internal node id (FindRange, FindSplit): the range's far
+// end j and the last leaf of the left child.
+template <class Keys>
+__device__ __forceinline__ void karras_range(const Keys &m, int id, int In, int &j, int &split) {
     const int dd = sgn_ref(delta(m, id, id + 1, In) - delta(m, id, id - 1, In));
     const int delmin = delta(m, id, id - dd, In);
     int lmax = 2;
@@ -442,10 +964,9 @@ __global__ void k_karras(DevPtrs d) {
     int l = 0;
     for (int t = lmax / 2; t >= 1; t /= 2)
         if (delta(m, id, id + (l + t) * dd, In) > delmin) l += t;
-    const int j = id + l * dd;
+    j = id + l * dd;
     const int first = min(id, j), last = max(id, j);
     // FindSplit (code-only prefix)
-    int split;
     const unsigned long long fc = m[first], lc = m[last];
     if (fc == lc) {
         split = (first + last) >> 1;
@@ -461,9 +982,27 @@ __global__ void k_karras(DevPtrs d) {
             }
         } while (step > 1);
     }
+}
+
+// Writes node `id` of a cloth; where the hierarchy is a tree (boxes), with
+// everything the refit and the record pass would write, from its children's
+// boxes.
+__device__ __forceinline__ void put_node(const DevPtrs &d, const ClothDev &cd, int id, int j, int split, bool boxes,
+                                         float3 amn, float3 amx, float3 bmn, float3 bmx) {
+    const int In = cd.T - 1, first = min(id, j), last = max(id, j);
     const int left = split == first ? In + split : split;
     const int right = split + 1 == last ? In + split + 1 : split + 1;
     d.child[cd.i_off + id] = make_int2(left, right);
+    if (boxes) {
+        const int2 rm = make_int2(In + split, In + last);
+        d.nmin[cd.n_off + id] = f4(vmin(amn, bmn), 0.f);
+        d.nmax[cd.n_off + id] = f4(vmax(amx, bmx), 0.f);
+        d.rml[cd.i_off + id] = rm;
+        d.parent[cd.n_off + left] = id;
+        d.parent[cd.n_off + right] = id;
+        put_wnode(d, (size_t)(cd.i_off + id), amn, amx, bmn, bmx, make_int2(left, right), rm);
+        return;
+    }
     if (d.nend) d.nend[cd.i_off + id] = j;
     // An internal node that the refit never reaches (possible only when a run
     // of >= 3 equal codes makes two nodes claim one child) keeps stale data in
@@ -475,6 +1014,128 @@ __global__ void k_karras(DevPtrs d) {
     atomicMax(&d.parent[cd.n_off + left], id);
     atomicMax(&d.parent[cd.n_off + right], id);
     d.visit[cd.i_off + id] = 0;
+}
+
+// One thread per internal node.  A block takes SPAN slots; nodes whose search
+// stays in them take their keys, and the boxes of their children (from a small
+// range tree over the block's leaves), from shared memory.  The few others,
+// whose searches go through memory for a dozen dependent loads or more, are
+// queued for k_karras_far: a lane in such a search holds up its warp, and
+// nearly every warp would have one.  SPAN = kSortTile: blocks are the sort's
+// tiles, for cloths of one tile, which have no such nodes (and need no range
+// tree in memory); SPAN = 256: any.
+template <int BS, int SPAN>
+struct KarrasBlock {
+    static constexpr bool kWhole = SPAN == kSortTile;  // a block holds a whole cloth
+    static constexpr size_t kSmem = (size_t)4 * SPAN * sizeof(float4) + (size_t)(SPAN + 2) * 8 + (size_t)SPAN * 4;
+};
+template <int BS, int SPAN>
+__global__ void __launch_bounds__(BS) k_karras(DevPtrs d) {
+    constexpr bool kWhole = KarrasBlock<BS, SPAN>::kWhole;
+    extern __shared__ float4 s_min[];                                     // leaves, then the levels above
+    float4 *s_max = s_min + 2 * SPAN;
+    unsigned long long *s_key = reinterpret_cast<unsigned long long *>(s_max + 2 * SPAN);
+    int *s_far = reinterpret_cast<int *>(s_key + SPAN + 2);
+    __shared__ int s_nfar;
+    __shared__ uint32_t s_base;
+    const int t = threadIdx.x;
+    const int B0 = kWhole ? d.stile_start[blockIdx.x] : blockIdx.x * SPAN;
+    const int B1 = kWhole ? B0 + d.cloth[d.stile_cloth[blockIdx.x]].T : min(B0 + SPAN, d.Ttot);
+    if (blockIdx.x == 0 && t == 0 && d.nrexit) *d.nrexit = 0;  // k_refit_local appends to it
+    if (t == 0) {
+        s_nfar = 0;
+        s_key[0] = B0 > 0 ? d.keys[B0 - 1] : 0ull;
+        s_key[B1 - B0 + 1] = B1 < d.Ttot ? d.keys[B1] : 0ull;
+    }
+    // (block-uniform: flagged cloths take their boxes from the climb)
+    const bool tree = d.eq3 && !(d.eq3[d.tcloth[B0]] && d.eq3[d.tcloth[B1 - 1]]);
+#pragma unroll
+    for (int q = 0; q < SPAN / BS; ++q) {
+        const int k = q * BS + t;
+        if (k >= B1 - B0) break;
+        s_key[k + 1] = d.keys[B0 + k];
+        if (tree) {
+            const ClothDev &cd = d.cloth[d.tcloth[B0 + k]];
+            const int leaf = cd.n_off + (cd.T - 1) + B0 + k - cd.t_off;
+            s_min[k] = d.nmin[leaf];
+            s_max[k] = d.nmax[leaf];
+        }
+    }
+    __syncthreads();
+    if (tree) {  // levels over the block's slots: level k's entry e covers slots [e 2^k, (e + 1) 2^k)
+        int from = 0;
+        for (int n = SPAN / 2; n >= 1; n >>= 1) {
+            const int to = from + 2 * n;
+            if (t < n && (t + 1) * (SPAN / n) <= B1 - B0) {
+                s_min[to + t] = f4(vmin(xyz(s_min[from + 2 * t]), xyz(s_min[from + 2 * t + 1])), 0.f);
+                s_max[to + t] = f4(vmax(xyz(s_max[from + 2 * t]), xyz(s_max[from + 2 * t + 1])), 0.f);
+            }
+            __syncthreads();
+            from = to;
+        }
+    }
+#pragma unroll 1
+    for (int q = 0; q < SPAN / BS; ++q) {
+        const int s = B0 + q * BS + t;
+        if (s >= B1) break;
+        const int c = d.tcloth[s];
+        const ClothDev &cd = d.cloth[c];
+        const int id = s - cd.t_off, In = cd.T - 1;
+        if (id >= In) continue;
+        const BlockKeys m{s_key, B0 - cd.t_off, B1 - B0, false};
+        int j, split;
+        karras_range(m, id, In, j, split);
+        const int first = min(id, j) + cd.t_off - B0, last = max(id, j) + cd.t_off - B0, mid = split + cd.t_off - B0;
+        // (a range may end on the neighbouring slot without a search past it, at the cloth's end)
+        if (!kWhole && (m.out || first < 0 || last >= B1 - B0)) {
+            s_far[atomicAdd(&s_nfar, 1)] = s;
+            continue;
+        }
+        const bool boxes = tree && !d.eq3[c];
+        float3 amn, amx, bmn, bmx;
+        if (boxes) {
+            range_box(s_min, s_max, s_min + SPAN, s_max + SPAN, SPAN, first, mid, amn, amx);
+            range_box(s_min, s_max, s_min + SPAN, s_max + SPAN, SPAN, mid + 1, last, bmn, bmx);
+        }
+        put_node(d, cd, id, j, split, boxes, amn, amx, bmn, bmx);
+    }
+    if (kWhole) return;
+    __syncthreads();
+    if (t == 0) s_base = s_nfar ? atomicAdd(d.nfar, (uint32_t)s_nfar) : 0u;
+    __syncthreads();
+    for (int k = t; k < s_nfar; k += BS) d.far[s_base + k] = s_far[k];
+}
+
+// The queued nodes, searched through memory, with the cloth's range tree for
+// the boxes: two lanes per node, one for each child's box.
+__global__ void __launch_bounds__(kThreads) k_karras_far(DevPtrs d) {
+    const uint32_t n = *d.nfar;
+    const bool tree = d.eq3 != nullptr;
+    const uint32_t lane2 = threadIdx.x & 1u;
+    const uint32_t stride = gridDim.x * (kThreads / 2);
+    for (uint32_t e0 = (blockIdx.x * kThreads + (threadIdx.x & ~31u)) / 2; e0 < n; e0 += stride) {  // warp-uniform
+        const uint32_t e = e0 + (threadIdx.x & 31u) / 2;
+        const bool valid = e < n;
+        const int s = d.far[valid ? e : e0], c = d.tcloth[s];
+        const ClothDev &cd = d.cloth[c];
+        const int id = s - cd.t_off, In = cd.T - 1;
+        const unsigned long long *m = d.keys + cd.t_off;
+        int j, split;
+        karras_range(m, id, In, j, split);
+        const bool boxes = tree && !d.eq3[c];
+        float3 mn = f3(0.f, 0.f, 0.f), mx = mn;
+        if (boxes) {
+            const float4 *lmin = d.nmin + cd.n_off + In, *lmax = d.nmax + cd.n_off + In;
+            const float4 *rmin = d.rmin + cd.t_off + kRangePad * c, *rmax = d.rmax + cd.t_off + kRangePad * c;
+            range_box(lmin, lmax, rmin, rmax, cd.T, lane2 ? split + 1 : min(id, j), lane2 ? max(id, j) : split, mn, mx);
+        }
+        __syncwarp();
+        const float3 omn = f3(__shfl_xor_sync(0xffffffffu, mn.x, 1), __shfl_xor_sync(0xffffffffu, mn.y, 1),
+                              __shfl_xor_sync(0xffffffffu, mn.z, 1));
+        const float3 omx = f3(__shfl_xor_sync(0xffffffffu, mx.x, 1), __shfl_xor_sync(0xffffffffu, mx.y, 1),
+                              __shfl_xor_sync(0xffffffffu, mx.z, 1));
+        if (valid && lane2 == 0) put_node(d, cd, id, j, split, boxes, mn, mx, omn, omx);
+    }
 }
 
 // Bottom-up refit: Collision/CudaBVH.cu:128-149.  The second arrival at a
@@ -514,6 +1175,7 @@ __device__ __forceinline__ void refit_climb(const DevPtrs &d, const ClothDev &cd
     atomicOr(d.err, ERR_TREE);
 }
 
+constexpr int kRefitBlock = 1024;
 // One thread per leaf, the whole climb in L2 (the allocation-free entry).
 __global__ void k_refit(DevPtrs d) {
     const int s = blockIdx.x * blockDim.x + threadIdx.x;
@@ -552,7 +1214,8 @@ __global__ void __launch_bounds__(kThreads) k_refit_local(DevPtrs d) {
     const int tid = threadIdx.x;
     const int B0 = blockIdx.x * kThreads, B1 = min(B0 + kThreads, d.Ttot);
     const int s = B0 + tid;
-    const bool valid = s < d.Ttot;
+    const bool valid = s < d.Ttot && d.eq3[d.tcloth[s]];  // the other cloths' nodes are complete
+    if (!__syncthreads_or(valid)) return;
     int c = 0, id = 0, In = 0;
     const ClothDev *cdp = nullptr;
     s_visit[tid] = 0;
@@ -632,23 +1295,39 @@ __global__ void k_refit_upper(DevPtrs d) {
 // Wide node records for the traversal: per internal node both children's
 // boxes, with the child ids and rightmost leaves in the w lanes, so that one
 // node visit is one contiguous 64-byte read instead of six dependent ones.
-// A separate pass after the refit, not part of it: a node the refit never
-// reaches (a run of >= 3 equal codes, see k_karras) still gets its record
-// from its children's boxes, as the per-node reads of the traversal see them.
+// For the cloths that took the climb, and after it, not part of it: a node
+// the refit never reaches (a run of >= 3 equal codes, see k_karras) still gets
+// its record from its children's boxes, as the per-node reads of the traversal
+// see them.
 __global__ void k_pack_nodes(DevPtrs d) {
     const int s = blockIdx.x * blockDim.x + threadIdx.x;
-    if (s >= d.Ttot) return;
+    if (s >= d.Ttot || !d.eq3[d.tcloth[s]]) return;
     const ClothDev &cd = d.cloth[d.tcloth[s]];
     const int k = s - cd.t_off;
     if (k >= cd.T - 1) return;
-    const int2 ch = d.child[cd.i_off + k], rm = d.rml[cd.i_off + k];
+    const int2 ch = d.child[cd.i_off + k];
     const float4 *nmin = d.nmin + cd.n_off, *nmax = d.nmax + cd.n_off;
-    const float4 a = nmin[ch.x], b = nmax[ch.x], c = nmin[ch.y], e = nmax[ch.y];
-    float4 *w = d.wnode + 4 * (size_t)(cd.i_off + k);
-    w[0] = make_float4(a.x, a.y, a.z, __int_as_float(ch.x));
-    w[1] = make_float4(b.x, b.y, b.z, __int_as_float(rm.x));
-    w[2] = make_float4(c.x, c.y, c.z, __int_as_float(ch.y));
-    w[3] = make_float4(e.x, e.y, e.z, __int_as_float(rm.y));
+    put_wnode(d, (size_t)(cd.i_off + k), xyz(nmin[ch.x]), xyz(nmax[ch.x]), xyz(nmin[ch.y]), xyz(nmax[ch.y]), ch,
+              d.rml[cd.i_off + k]);
+}
+
+// Climb and records of flagged cloths, a block per cloth in one launch: for
+// batches of small cloths, where the three launches above cost more than they
+// do.
+__global__ void __launch_bounds__(kRefitBlock) k_refit_block(DevPtrs d) {
+    const int c = blockIdx.x;
+    if (!d.eq3[c]) return;
+    const ClothDev &cd = d.cloth[c];
+    const int In = cd.T - 1;
+    for (int id = threadIdx.x; id <= In && In > 0; id += kRefitBlock) refit_climb(d, cd, d.parent[cd.n_off + In + id]);
+    __threadfence();
+    __syncthreads();
+    const float4 *nmin = d.nmin + cd.n_off, *nmax = d.nmax + cd.n_off;
+    for (int k = threadIdx.x; k < In; k += kRefitBlock) {
+        const int2 ch = d.child[cd.i_off + k];
+        put_wnode(d, (size_t)(cd.i_off + k), xyz(__ldcg(&nmin[ch.x])), xyz(__ldcg(&nmax[ch.x])), xyz(__ldcg(&nmin[ch.y])),
+                  xyz(__ldcg(&nmax[ch.y])), ch, __ldcg(&d.rml[cd.i_off + k]));
+    }
 }
 
 // Leaf-vs-tree traversal: Collision/CudaBVH.cu:23-113.  Pairs (i, j>i) in
@@ -701,8 +1380,6 @@ __global__ void k_traverse(DevPtrs d) {
     d.pair_cnt[s] = (uint32_t)got;
     if (dropped) atomicAdd(&d.counters[3], (unsigned long long)dropped);
 }
-
-
 
 // The traversal as a packet: a left-first depth-first walk of a Karras tree
 // meets the leaves in increasing index order, so leaf i's result is the
@@ -1632,53 +2309,115 @@ void launch_leaves_from_boxes(const DevPtrs &d, const float *bmin, const float *
                               cudaStream_t st) {
     if (T) k_leaves_from_boxes<<<nblk(T), kThreads, 0, st>>>(d, bmin, bmax, T, mode);
 }
-void launch_sort(const DevPtrs &d, const int *tile_first, int passes, cudaStream_t st) {
+// Sorts by `passes` 8-bit digits from bit shift0 up (an even number: the result
+// is where the keys were).  alt: the keys start in keys_alt / payload_alt.
+void launch_sort(const DevPtrs &d, const int *tile_first, int shift0, int passes, bool alt, cudaStream_t st) {
     if (!d.nstiles) return;
-    // One-sweep wherever the scratch exists (not in the allocation-free
-    // entry, whose one tile needs no look-back) and the digit counts fit the
-    // status word's 30 bits; the per-pass histogram and per-segment offsets
-    // block remain for the rest.
+    unsigned long long *k0 = alt ? d.keys_alt : d.keys, *k1 = alt ? d.keys : d.keys_alt;
+    uint32_t *p0 = alt ? d.payload_alt : d.payload, *p1 = alt ? d.payload : d.payload_alt;
+    // One-sweep wherever the digit counts fit the status word's 30 bits; the
+    // per-pass histogram and per-segment offsets block remain for the rest.
     const bool sweep = d.sstat && d.sseg && d.Ttot <= (int64_t)kStatCount && passes <= kSortPassesMax;
     if (sweep) {
         cudaMemsetAsync(d.sseg, 0, sizeof(uint32_t) * (kSortPassesMax + (size_t)d.C * kSortPassesMax * kSortBuckets), st);
-        k_sort_hist_all<<<d.nstiles, kThreads, 0, st>>>(d, d.keys, passes);
+        k_sort_hist_all<<<d.nstiles, kThreads, 0, st>>>(d, k0, shift0, passes);
     }
     for (int p = 0; p < passes; ++p) {
-        const bool even = (p & 1) == 0;
-        const unsigned long long *kin = even ? d.keys : d.keys_alt;
-        unsigned long long *kout = even ? d.keys_alt : d.keys;
-        const uint32_t *pin = even ? d.payload : d.payload_alt;
-        uint32_t *pout = even ? d.payload_alt : d.payload;
+        const int shift = shift0 + p * kSortBits;
         if (sweep) {
-            k_sort_scatter<true><<<d.nstiles, kThreads, 0, st>>>(d, kin, pin, kout, pout, p * kSortBits, p, tile_first);
+            k_sort_scatter<true><<<d.nstiles, kThreads, 0, st>>>(d, k0, p0, k1, p1, shift, p, tile_first);
         } else {
-            k_sort_hist<<<d.nstiles, kThreads, 0, st>>>(d, kin, p * kSortBits);
+            k_sort_hist<<<d.nstiles, kThreads, 0, st>>>(d, k0, shift);
             k_sort_offsets<<<d.C, kSortBuckets * kOffsetsSplit, 0, st>>>(d, tile_first);
-            k_sort_scatter<false><<<d.nstiles, kThreads, 0, st>>>(d, kin, pin, kout, pout, p * kSortBits, p, tile_first);
+            k_sort_scatter<false><<<d.nstiles, kThreads, 0, st>>>(d, k0, p0, k1, p1, shift, p, tile_first);
         }
+        std::swap(k0, k1);
+        std::swap(p0, p1);
     }
 }
-void launch_post_sort(const DevPtrs &d, cudaStream_t st) {
-    if (d.Ttot) k_post_sort<<<nblk(d.Ttot), kThreads, 0, st>>>(d);
+
+template <int CS, int R>
+static cudaError_t sort_segments(const DevPtrs &d, int halves, cudaStream_t st) {
+    const size_t smem = SegmentSort<CS, R>::kSmem;
+    const cudaError_t e =
+        cudaFuncSetAttribute(k_sort_segment<CS, R>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e != cudaSuccess) return e;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(d.C * CS);
+    cfg.blockDim = dim3(kSmallThreads);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = CS;
+    attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = CS > 1 ? 1 : 0;
+    return cudaLaunchKernelEx(&cfg, k_sort_segment<CS, R>, d, halves);
 }
-void launch_karras(const DevPtrs &d, cudaStream_t st) {
-    if (d.Ttot) k_karras<<<nblk(d.Ttot), kThreads, 0, st>>>(d);
-}
-void launch_refit(const DevPtrs &d, cudaStream_t st) {
+
+// Sort by Morton code and its outputs (keys, perm, tri_slot, fixed-mode leaf
+// boxes) from the codes in keys_alt.  max_T: the largest segment.  Measured (us,
+// the launches of one step timed together) one CTA per segment / eight / the
+// general passes: one segment of 1922 17 / 21 / 54, of 7938 42 / 23 / 54, of
+// 15842 - / 30 / 56, of 31752 - / 42 / 59, of 64082 - / 67 / 64; 8 segments up
+// to 32258 - / 41 / 58; 16 up to 6498 39 / 36 / 54; 64 up to 7938 41 / 82 / 58;
+// 64 up to 31752 - / 178 / 110.  So one CTA up to 2048 keys, eight for at most
+// eight segments of up to 32768, one up to 8192, and the passes beyond.
+void launch_morton_sort(const DevPtrs &d, const int *tile_first, int mode, int max_T, cudaStream_t st) {
     if (!d.Ttot) return;
-    if (d.nend) {
-        // the upper pass: a grid-stride loop over the arrivals left, sized to
-        // be resident at once
-        k_refit_local<<<nblk(d.Ttot), kThreads, 0, st>>>(d);
-        k_refit_upper<<<std::min(nblk(2 * (int64_t)std::max(d.Itot, 1)), 1024), kThreads, 0, st>>>(d);
-    } else {
-        k_refit<<<nblk(d.Ttot), kThreads, 0, st>>>(d);
+    const int halves = mode == LC_MORTON_K30 ? 0 : 1, shift0 = halves ? 32 : 0;
+    cudaError_t e = cudaErrorNotSupported;
+    if (max_T <= kSmallThreads) e = sort_segments<1, 1>(d, halves, st);
+    else if (max_T <= 2 * kSmallThreads) e = sort_segments<1, 2>(d, halves, st);
+    else if (d.C <= kSmallCtas) {
+        if (max_T <= kSmallCtas * kSmallThreads) e = sort_segments<kSmallCtas, 1>(d, halves, st);
+        else if (max_T <= 2 * kSmallCtas * kSmallThreads) e = sort_segments<kSmallCtas, 2>(d, halves, st);
+        else if (max_T <= 4 * kSmallCtas * kSmallThreads) e = sort_segments<kSmallCtas, 4>(d, halves, st);
     }
+    else if (max_T <= 4 * kSmallThreads) e = sort_segments<1, 4>(d, halves, st);
+    else if (max_T <= 8 * kSmallThreads) e = sort_segments<1, 8>(d, halves, st);
+    if (e == cudaSuccess) return;
+    cudaGetLastError();
+    launch_sort(d, tile_first, shift0, 4, true, st);
+    if (halves) k_sort_long_runs<<<nblk(d.Ttot), kThreads, 0, st>>>(d);
+    k_post_sort<<<nblk(d.Ttot), kThreads, 0, st>>>(d, halves);
+}
+// The hierarchy with its boxes and records.
+void launch_hierarchy(const DevPtrs &d, int max_T, cudaStream_t st) {
+    if (!d.Ttot) return;
+    using Any = KarrasBlock<kThreads, kThreads>;
+    using Whole = KarrasBlock<1024, kSortTile>;
+    const int far_blocks = std::min(nblk(d.Ttot, 2 * kThreads), 1024);
+    if (!d.eq3) {  // the allocation-free entry: no range tree, the climb for all
+        k_karras<kThreads, kThreads><<<nblk(d.Ttot), kThreads, Any::kSmem, st>>>(d);
+        k_karras_far<<<far_blocks, kThreads, 0, st>>>(d);
+        k_refit<<<nblk(d.Ttot), kThreads, 0, st>>>(d);
+        return;
+    }
+    if (max_T <= kSortTile && cudaFuncSetAttribute(k_karras<1024, kSortTile>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                                   (int)Whole::kSmem) == cudaSuccess) {
+        k_karras<1024, kSortTile><<<d.nstiles, 1024, Whole::kSmem, st>>>(d);
+    } else {
+        cudaGetLastError();
+        k_range_tree<<<d.nstiles, kTreeThreads, 0, st>>>(d);
+        k_karras<kThreads, kThreads><<<nblk(d.Ttot), kThreads, Any::kSmem, st>>>(d);
+        k_karras_far<<<far_blocks, kThreads, 0, st>>>(d);
+    }
+    // cloths in which three equal codes meet
+    if (max_T <= 4 * kSortTile) {
+        k_refit_block<<<d.C, kRefitBlock, 0, st>>>(d);
+        return;
+    }
+    // the upper pass: a grid-stride loop over the arrivals left, sized to be
+    // resident at once
+    k_refit_local<<<nblk(d.Ttot), kThreads, 0, st>>>(d);
+    k_refit_upper<<<std::min(nblk(2 * (int64_t)std::max(d.Itot, 1)), 1024), kThreads, 0, st>>>(d);
+    k_pack_nodes<<<nblk(d.Ttot), kThreads, 0, st>>>(d);
 }
 void launch_traverse(const DevPtrs &d, int block, cudaStream_t st) {
     if (!d.Ttot) return;
     if (d.wnode) {
-        k_pack_nodes<<<nblk(d.Ttot), kThreads, 0, st>>>(d);
         k_traverse_packet<<<nblk(d.Ttot, block), block, 0, st>>>(d);
     } else {
         k_traverse<<<nblk(d.Ttot, block), block, 0, st>>>(d);

@@ -29,10 +29,8 @@
 namespace lc {
 void launch_leaves_from_boxes(const DevPtrs &d, const float *bmin, const float *bmax, int T, int mode,
                               cudaStream_t st);
-void launch_sort(const DevPtrs &d, const int *tile_first, int passes, cudaStream_t st);
-void launch_post_sort(const DevPtrs &d, cudaStream_t st);
-void launch_karras(const DevPtrs &d, cudaStream_t st);
-void launch_refit(const DevPtrs &d, cudaStream_t st);
+void launch_morton_sort(const DevPtrs &d, const int *tile_first, int mode, int max_T, cudaStream_t st);
+void launch_hierarchy(const DevPtrs &d, int max_T, cudaStream_t st);
 void launch_traverse(const DevPtrs &d, int block, cudaStream_t st);
 
 namespace {
@@ -45,7 +43,7 @@ constexpr size_t al(size_t n) { return (n + 255) & ~size_t(255); }
 
 // Layout of the scratch array (bytes, each piece 256-byte aligned).
 struct Layout {
-    size_t cloth, tcloth, keys, keys_alt, payload, payload_alt, perm, perm_alt, leaf_min, leaf_max, nmin, nmax,
+    size_t cloth, tcloth, keys, keys_alt, payload, payload_alt, perm, far, leaf_min, leaf_max, nmin, nmax,
         parent, child, rml, visit, pair_cnt, pair_off, pair_chunk, shist, stile_cloth, stile_start, tile_first,
         scan_tmp, counters, err, npairs, total;
 };
@@ -61,7 +59,7 @@ constexpr Layout make_layout() {
     l.payload = o; o += al(4 * T);
     l.payload_alt = o; o += al(4 * T);
     l.perm = o; o += al(4 * T);
-    l.perm_alt = o; o += al(4 * T);
+    l.far = o; o += al(4 * (T + 1));
     l.leaf_min = o; o += al(16 * T);
     l.leaf_max = o; o += al(16 * T);
     l.nmin = o; o += al(16 * N);
@@ -209,7 +207,8 @@ extern "C" lc_status lc_lbvh_pairs_static(const float *tri_min, const float *tri
     d.payload = reinterpret_cast<uint32_t *>(base + L.payload);
     d.payload_alt = reinterpret_cast<uint32_t *>(base + L.payload_alt);
     d.perm = reinterpret_cast<uint32_t *>(base + L.perm);
-    d.perm_alt = reinterpret_cast<uint32_t *>(base + L.perm_alt);
+    d.far = reinterpret_cast<int *>(base + L.far);
+    d.nfar = reinterpret_cast<uint32_t *>(base + L.far) + kStaticMaxT;
     d.leaf_tmp_min = reinterpret_cast<float4 *>(base + L.leaf_min);
     d.leaf_tmp_max = reinterpret_cast<float4 *>(base + L.leaf_max);
     d.nmin = reinterpret_cast<float4 *>(base + L.nmin);
@@ -238,12 +237,8 @@ extern "C" lc_status lc_lbvh_pairs_static(const float *tri_min, const float *tri
                                            const_cast<int *>(tile_first), d.counters, d.err, d.scan_tmp, T, chunk,
                                            morton_mode);
     launch_leaves_from_boxes(d, tri_min, tri_max, T, morton_mode, st);
-    launch_sort(d, tile_first, morton_mode == LC_MORTON_K30 ? 4 : 8, st);
-    launch_post_sort(d, st);
-    LC_STATIC_CUDA(cudaMemcpyAsync(d.perm, d.perm_alt, sizeof(uint32_t) * T, cudaMemcpyDeviceToDevice, st));
-    LC_STATIC_CUDA(cudaMemsetAsync(d.parent, 0xFF, sizeof(int) * (size_t)d.Ntot, st));
-    launch_karras(d, st);
-    launch_refit(d, st);
+    launch_morton_sort(d, tile_first, morton_mode, T, st);
+    launch_hierarchy(d, T, st);
     launch_traverse(d, 128, st);
     scan_u32({d.pair_cnt, d.pair_off, nullptr, (uint32_t)T, (uint32_t)T, npairs, &d.counters[0]}, nullptr, d.scan_tmp,
              d.err, st);
