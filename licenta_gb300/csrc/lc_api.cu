@@ -415,6 +415,7 @@ struct lc_batch {
 
     lc_status enqueue_step(cudaStream_t st);
     lc_status setup_cluster();
+    lc_status setup_global_solver();
 
     // profiling: when non-null, events are recorded at phase boundaries
     cudaEvent_t *prof_ev = nullptr;    // 8 events per step
@@ -592,12 +593,21 @@ static double estimate_solve(const lc_batch &b, const std::vector<int> &largest_
     return end + 1.5 * own * per_cta(0);
 }
 
+// Global-memory solver: the corrections of one iteration.
+lc_status lc_batch::setup_global_solver() {
+    if (d.corr) return LC_OK;
+    float4 *corr;
+    LC_TRY(arena.alloc(corr, std::max<size_t>((size_t)d.Etot + 4 * (size_t)d.Btot, 1), "corrections"));
+    d.corr = corr;
+    return LC_OK;
+}
+
 // Cluster-resident solver: picks the cluster size for the largest cloth and
 // the cluster -> cloth schedule (largest cloths first).  Leaves use_cluster
 // false when some cloth does not fit on chip.
 lc_status lc_batch::setup_cluster() {
     use_cluster = false;
-    if (opt.solver_variant == 1) return LC_OK;
+    if (opt.solver_variant == 1) return setup_global_solver();
     // the scatter form is the default on-chip solver (each constraint
     // evaluated once per iteration); variant 2 selects the gather form
     const bool scatter = opt.solver_variant != 2;
@@ -634,7 +644,7 @@ lc_status lc_batch::setup_cluster() {
     }
     if (!cs) {
         if (opt.solver_variant >= 2) return fail(LC_ERR_NOT_SUPPORTED, "cluster solver: a cloth does not fit on chip");
-        return LC_OK;
+        return setup_global_solver();
     }
     cluster_cs = cs;
     cluster_bs = bs;
@@ -981,6 +991,8 @@ static lc_status batch_build(lc_batch *b, const lc_cloth_desc *descs, int n, con
         J.E = (int)E; J.B = (int)B;
         b->nfixed = (int)F;
     }
+    d.Etot = (int)E;
+    d.Btot = (int)B;
     b->narrow_grid = sm_count() * 8;
     b->jacobi_block = opt.block_size > 0 ? opt.block_size : 256;
     LC_TRY(b->setup_cluster());

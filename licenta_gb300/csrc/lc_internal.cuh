@@ -175,6 +175,10 @@ struct DevPtrs {
     const float2 *s_par;   // (l0, kp)
     const int4 *b_ids;     // bend (p1, p2, p3, p4)
     const float *b_kp;
+    // global-memory solver, one iteration: a row of Etot for the stretch
+    // constraints and four of Btot for the bends (see k_constraints)
+    float4 *corr;
+    int Etot, Btot;
     // LRA / ground
     const int *fixed;      // global ids of pinned vertices, per cloth at f_off
     const float *lra_l0;

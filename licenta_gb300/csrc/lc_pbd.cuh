@@ -52,17 +52,23 @@ __device__ __forceinline__ float3 stretch_corr_pos(float4 a, float4 b, float l0,
     return role == 0 ? mul(tt, -w1) : mul(tt, w2);
 }
 
-// The same constraint evaluated once for both vertices; false: no correction.
-__device__ __forceinline__ bool stretch_all_pos(float4 a, float4 b, float l0, float kp, float3 out[2]) {
+// The same constraint evaluated once for both vertices, whose corrections are
+// -w1 t and w2 t; false: no correction.
+__device__ __forceinline__ bool stretch_vec_pos(float4 a, float4 b, float l0, float kp, float3 &t) {
     const float ws = pin::addr(a.w, b.w);
     if (ws == 0.f) return false;
     const float3 diff = pin::sub(xyz(a), xyz(b));
     const float l = pin::len(diff);
     if (l <= kEpsPbd) return false;
     const float3 n = dvs(diff, l);
-    const float3 tt = dvs(pin::mul(pin::mul(n, pin::subr(l, l0)), kp), ws);
-    out[0] = pin::mul(tt, -a.w);
-    out[1] = pin::mul(tt, b.w);
+    t = dvs(pin::mul(pin::mul(n, pin::subr(l, l0)), kp), ws);
+    return true;
+}
+__device__ __forceinline__ bool stretch_all_pos(float4 a, float4 b, float l0, float kp, float3 out[2]) {
+    float3 t;
+    if (!stretch_vec_pos(a, b, l0, kp, t)) return false;
+    out[0] = pin::mul(t, -a.w);
+    out[1] = pin::mul(t, b.w);
     return true;
 }
 
@@ -106,13 +112,17 @@ __device__ __forceinline__ float3 bend_corr_pos(float4 a1, float4 a2, float4 a3,
 // Physics/CudaPBD.cu:1149-1187 — triangle bending (useTriangleBending): the
 // middle vertex v of three collinear grid vertices (b0, v, b1) is kept at the
 // rest distance h0 from their centroid.  Slot roles: 0 = b0, 1 = b1, 2 = v.
-__device__ __forceinline__ float3 tri_bend_corr_pos(float4 b0, float4 b1, float4 v, float kp, float h0, int role) {
+// Their corrections are 2 w0 t, 2 w1 t and -4 wv t.
+__device__ __forceinline__ float3 tri_bend_vec_pos(float4 b0, float4 b1, float4 v, float kp, float h0) {
     const float W = b0.w + b1.w + 2.f * v.w;
     const float3 c = dvs(add(add(xyz(b0), xyz(b1)), xyz(v)), 3.f);
     const float3 hv = sub(xyz(v), c);
     const float l = len(hv);
     if (l <= kEpsPbd) return f3(0.f, 0.f, 0.f);
-    const float3 term = mul(mul(dvs(hv, W), kp), 1.f - h0 / l);
+    return mul(mul(dvs(hv, W), kp), 1.f - h0 / l);
+}
+__device__ __forceinline__ float3 tri_bend_corr_pos(float4 b0, float4 b1, float4 v, float kp, float h0, int role) {
+    const float3 term = tri_bend_vec_pos(b0, b1, v, kp, h0);
     return role == 0 ? mul(term, 2.f * b0.w) : role == 1 ? mul(term, 2.f * b1.w) : mul(term, -4.f * v.w);
 }
 

@@ -321,30 +321,20 @@ __global__ void k_sphere(DevPtrs d) {
 }
 
 // ---------------------------------------------------------------------------
-// Jacobi iteration (Physics/CudaPBD.cu:648-659) as a per-vertex gather:
-// every vertex evaluates the constraints it belongs to on the positions of
-// the previous iteration (xa) and writes its own update to xb.  The sum is
+// Jacobi iteration (Physics/CudaPBD.cu:648-659) in two launches.
+// k_constraints evaluates every stretch and bend constraint once on the
+// positions of the previous iteration (xa) and stores what the corrections of
+// its vertices share, constraint by constraint; k_jacobi scales and sums a
+// vertex's corrections in order, adds the terms that are its own and the
+// contacts, and writes its update to xb.  Bound by the L2: 64 bytes written
+// and 128 read per edge with its bend, which stay there for 512 x 512 vertices
+// (105 MB with the constraints' own data).  An iteration of that cloth takes
+// JACOBI_US; 72 us when each vertex evaluated its 18 constraints itself (a chain of
+// three loads per evaluation), 67 us when every correction was stored at its
+// vertex's place (scattered half-sector writes).  The sum is
 // associated like the reference's accumulator: ((ground + LRA) + static) +
 // dynamic, then x += acc / count.
 // ---------------------------------------------------------------------------
-__device__ __forceinline__ float3 stretch_corr(const DevPtrs &d, const float4 *__restrict__ xa, uint32_t k,
-                                               int role) {
-    const int2 id = __ldg(&d.s_ids[k]);
-    const float2 par = __ldg(&d.s_par[k]);
-    return stretch_corr_pos(xa[id.x], xa[id.y], par.x, par.y, role);
-}
-
-__device__ __forceinline__ float3 tri_bend_corr(const DevPtrs &d, const float4 *__restrict__ xa, uint32_t k,
-                                                int role) {
-    const int4 id = __ldg(&d.b_ids[k]);
-    return tri_bend_corr_pos(xa[id.x], xa[id.y], xa[id.z], __ldg(&d.b_kp[k]), __int_as_float(id.w), role);
-}
-
-__device__ __forceinline__ float3 bend_corr(const DevPtrs &d, const float4 *__restrict__ xa, uint32_t k, int role) {
-    const int4 id = __ldg(&d.b_ids[k]);
-    return bend_corr_pos(xa[id.x], xa[id.y], xa[id.z], xa[id.w], __ldg(&d.b_kp[k]), d.kpi_gap, role);
-}
-
 __device__ __forceinline__ float3 contact_corr(const DevPtrs &d, const float4 *__restrict__ xa, uint32_t e,
                                                uint32_t nvf, float h) {
     const uint32_t c = e >> 2;
@@ -355,6 +345,43 @@ __device__ __forceinline__ float3 contact_corr(const DevPtrs &d, const float4 *_
     return contact_corr_pos(xa[v.x], xa[v.y], xa[v.z], xa[v.w], w, isvf, h, slot);
 }
 
+// Blocks [0, nbs) take the stretch constraints, the others the bends.  Entry
+// (q, s) of a constraint's vertex of inverse mass w: the correction -(w s) q, for
+// the second vertex of a stretch (which shares the entry of the first) +(w s) q.
+__global__ void __launch_bounds__(kThreads) k_constraints(DevPtrs d, const float4 *__restrict__ xa, int nbs) {
+    const bool bend = (int)blockIdx.x >= nbs;
+    const int k = (blockIdx.x - (bend ? nbs : 0)) * kThreads + threadIdx.x;
+    if (k >= (bend ? d.Btot : d.Etot)) return;
+    if (!bend) {
+        const int2 id = __ldg(&d.s_ids[k]);
+        const float2 par = __ldg(&d.s_par[k]);
+        float3 t;
+        if (!stretch_vec_pos(xa[id.x], xa[id.y], par.x, par.y, t)) t = f3(0.f, 0.f, 0.f);
+        d.corr[k] = f4(t, 1.f);
+        return;
+    }
+    const int4 id = __ldg(&d.b_ids[k]);
+    const float kp = __ldg(&d.b_kp[k]);
+    const float4 a = xa[id.x], b = xa[id.y], c = xa[id.z];
+    float4 *out = d.corr + d.Etot + k;
+    const size_t B = d.Btot;
+    if (d.cloth[d.vcloth[id.x]].tri_bend) {
+        const float3 t = tri_bend_vec_pos(a, b, c, kp, __int_as_float(id.w));
+        out[0] = out[B] = f4(t, -2.f);
+        out[2 * B] = f4(t, 4.f);
+        return;
+    }
+    float3 q[4];
+    float s;
+    if (!bend_all_pos(a, b, c, xa[id.w], kp, d.kpi_gap, q, s)) {
+        q[0] = q[1] = q[2] = q[3] = f3(0.f, 0.f, 0.f);
+        s = 0.f;
+    }
+#pragma unroll
+    for (int j = 0; j < 4; ++j) out[j * B] = f4(q[j], s);
+}
+
+constexpr int kEntryBatch = 6;
 __global__ void k_jacobi(DevPtrs d, const float4 *__restrict__ xa, float4 *__restrict__ xb, int it,
                          const uint32_t *__restrict__ nvf_dev) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
@@ -403,12 +430,22 @@ __global__ void k_jacobi(DevPtrs d, const float4 *__restrict__ xa, float4 *__res
     {
         float3 sa = f3(0.f, 0.f, 0.f);
         const int s0 = d.soff[i], s1 = d.soff[i + 1];
-        for (int e = s0; e < s1; ++e) {
-            const uint32_t ent = __ldg(&d.sent[e]);
-            const uint32_t k = ent & 0x1FFFFFFFu;
-            const int role = (int)((ent >> 29) & 3u);
-            sa = add(sa, (ent >> 31) ? (cd.tri_bend ? tri_bend_corr(d, xa, k, role) : bend_corr(d, xa, k, role))
-                                     : stretch_corr(d, xa, k, role));
+        for (int e = s0; e < s1; e += kEntryBatch) {  // the loads of a batch in flight together
+            uint32_t ent[kEntryBatch];
+            float4 r[kEntryBatch];
+#pragma unroll
+            for (int j = 0; j < kEntryBatch; ++j) ent[j] = __ldg(&d.sent[min(e + j, s1 - 1)]);
+#pragma unroll
+            for (int j = 0; j < kEntryBatch; ++j) {
+                const uint32_t k = ent[j] & 0x1FFFFFFFu, role = (ent[j] >> 29) & 3u;
+                r[j] = d.corr[(ent[j] >> 31) ? (size_t)d.Etot + role * (size_t)d.Btot + k : (size_t)k];
+            }
+#pragma unroll
+            for (int j = 0; j < kEntryBatch; ++j) {
+                if (e + j >= s1) break;
+                const float f = xi4.w * r[j].w;
+                sa = add(sa, mul(xyz(r[j]), (ent[j] >> 29) == 1u ? f : -f));
+            }
         }
         acc = add(acc, sa);
         cnt += s1 - s0;
@@ -493,6 +530,8 @@ void launch_solver_setup(const DevPtrs &d, bool sphere, cudaStream_t st) {
 }
 void launch_jacobi(const DevPtrs &d, const float4 *xa, float4 *xb, int it, const uint32_t *nvf, int block,
                    cudaStream_t st) {
+    const int nbs = nblk(d.Etot), nbb = nblk(d.Btot);
+    if (nbs + nbb) k_constraints<<<nbs + nbb, kThreads, 0, st>>>(d, xa, nbs);
     if (d.Vtot) k_jacobi<<<nblk(d.Vtot, block), block, 0, st>>>(d, xa, xb, it, nvf);
 }
 void launch_integrate(const DevPtrs &d, const float4 *xs, cudaStream_t st) {
