@@ -15,6 +15,8 @@
 #include <unordered_map>
 #include <unordered_set>
 #include <queue>
+#include <limits>
+#include <utility>
 #include <vector>
 
 #include "lc_internal.cuh"
@@ -46,8 +48,9 @@ void launch_adjoint(const DevPtrs &d, const AdjPtrs &A, float4 *a, float4 *g, co
 void launch_vertex_normals(const DevPtrs &d, cudaStream_t st);
 void launch_dyn(const DevPtrs &d, const uint32_t *nvf, const uint32_t *nee, int grid, int phase, cudaStream_t st);
 void launch_solver_setup(const DevPtrs &d, bool sphere, cudaStream_t st);
+bool tiles_supported();
 void launch_jacobi(const DevPtrs &d, const float4 *xa, float4 *xb, int it, const uint32_t *nvf, int block,
-                   cudaStream_t st);
+                   size_t tile_smem, cudaStream_t st);
 void launch_integrate(const DevPtrs &d, const float4 *xs, cudaStream_t st);
 void launch_friction(const DevPtrs &d, const uint32_t *nvf, cudaStream_t st);
 void launch_vertex_records(const DevPtrs &d, void *dst, int64_t stride, int pos_off, int nrm_off, cudaStream_t st);
@@ -416,6 +419,9 @@ struct lc_batch {
     lc_status enqueue_step(cudaStream_t st);
     lc_status setup_cluster();
     lc_status setup_global_solver();
+    lc_status setup_tiles();
+    lc_status build_tiles(int target, bool &fit);
+    size_t tile_smem = 0;          // of the global-memory solver's tiles
 
     // profiling: when non-null, events are recorded at phase boundaries
     cudaEvent_t *prof_ev = nullptr;    // 8 events per step
@@ -523,7 +529,7 @@ lc_status lc_batch::enqueue_step(cudaStream_t st) {
     for (int it = 0; it < max_iters; ++it) {
         if (recording) b = tape_x + (size_t)(it + 1) * d.Vtot;
         if (it == 0) LC_KEV(0);
-        launch_jacobi(d, a, b, it, nvf, jacobi_block, st);
+        launch_jacobi(d, a, b, it, nvf, jacobi_block, tile_smem, st);
         if (it == 0) LC_KEV(1);
         if (recording) a = b;
         else std::swap(a, b);
@@ -593,12 +599,176 @@ static double estimate_solve(const lc_batch &b, const std::vector<int> &largest_
     return end + 1.5 * own * per_cta(0);
 }
 
-// Global-memory solver: the corrections of one iteration.
+// Global-memory solver: its tiles or, without, the corrections of one iteration.
 lc_status lc_batch::setup_global_solver() {
-    if (d.corr) return LC_OK;
+    if (d.corr || d.ntiles || !d.Vtot) return LC_OK;
+    LC_TRY(setup_tiles());
+    if (d.ntiles) return LC_OK;
     float4 *corr;
     LC_TRY(arena.alloc(corr, std::max<size_t>((size_t)d.Etot + 4 * (size_t)d.Btot, 1), "corrections"));
     d.corr = corr;
+    return LC_OK;
+}
+
+// The cloths cut into tiles for the global-memory solver.  Vertices per tile:
+// two tiles on an SM, as many turns of the chip as the largest tile that fits
+// asks for, evenly filled, and 64 at least (us per iteration with 64 / 128 / 216
+// / 300 / 431 vertices: 64 squared 10 / 12 / 12 / 13 / 14, 256 squared 24 / 18 /
+// 15 / 16 / 17, 512 squared 68 / 45 / 38 / 36 / 35: constraints across tiles are
+// evaluated in each).  Leaves ntiles 0 where tiles of 32 vertices do not fit.
+lc_status lc_batch::setup_tiles() {
+    for (int most = 448; most >= 32; most -= most / 8) {
+        const int slots = 2 * sm_count(), turns = (int)((d.Vtot + (int64_t)slots * most - 1) / ((int64_t)slots * most));
+        const int per = (int)((d.Vtot + (int64_t)slots * turns - 1) / ((int64_t)slots * turns));
+        bool fit = false;
+        LC_TRY(build_tiles(std::min(most, std::max(per, 64)), fit));
+        if (fit) break;
+    }
+    return LC_OK;
+}
+
+// Tiles of at most `target` vertices, in Morton order of the rest positions.
+// fit: whether each tile's positions and entries fit half of an SM.
+lc_status lc_batch::build_tiles(int target, bool &fit) {
+    fit = false;
+    std::vector<SolveTile> tiles;
+    std::vector<int> vert, rows, sk, bk;
+    std::vector<uint2> ts;
+    std::vector<uint4> tb;
+    vert.reserve(2 * (size_t)d.Vtot);
+    ts.reserve((size_t)d.Etot + d.Etot / 4);
+    sk.reserve(ts.capacity());
+    tb.reserve((size_t)d.Btot + d.Btot / 3);
+    bk.reserve(tb.capacity());
+    size_t smem = 0;
+    for (int c = 0; c < C; ++c) {
+        const HostCloth &hc = hosts[c];
+        const ClothDev &cd = cds[c];
+        const int V = hc.V;
+        constexpr float kMax = std::numeric_limits<float>::max();
+        float lo[3] = {kMax, kMax, kMax}, hi[3] = {-kMax, -kMax, -kMax};
+        for (int i = 0; i < V; ++i)
+            for (int a = 0; a < 3; ++a) {
+                lo[a] = std::min(lo[a], hc.pos[3 * i + a]);
+                hi[a] = std::max(hi[a], hc.pos[3 * i + a]);
+            }
+        float ext = 0.f;
+        for (int a = 0; a < 3; ++a) ext = std::max(ext, hi[a] - lo[a]);
+        std::vector<std::pair<uint32_t, int>> order(V), buf(V);
+        std::vector<int> digit_count(3 * 1024, 0);
+        for (int i = 0; i < V; ++i) {
+            uint32_t code = 0;
+            for (int a = 0; a < 3; ++a) {
+                const float u = ext > 0.f ? (hc.pos[3 * i + a] - lo[a]) / ext * 1023.f : 0.f;
+                uint32_t q = u > 0.f ? (uint32_t)std::min(u, 1023.f) : 0u;
+                q = (q | (q << 16)) & 0x030000ffu;  // two zeros between its bits
+                q = (q | (q << 8)) & 0x0300f00fu;
+                q = (q | (q << 4)) & 0x030c30c3u;
+                q = (q | (q << 2)) & 0x09249249u;
+                code |= q << a;
+            }
+            order[i] = {code, i};
+            for (int p = 0; p < 3; ++p) ++digit_count[1024 * p + ((code >> (10 * p)) & 1023u)];
+        }
+        for (int p = 0; p < 3; ++p) {  // by code, three passes of ten bits
+            int *at = digit_count.data() + 1024 * p, sum = 0;
+            for (int k = 0; k < 1024; ++k) sum += std::exchange(at[k], sum);
+            for (const auto &o : order) buf[at[(o.first >> (10 * p)) & 1023u]++] = o;
+            order.swap(buf);
+        }
+        std::vector<int> rec_s(hc.s_ids.size(), -1), rec_b(hc.b_ids.size(), -1);  // a constraint's latest record
+        std::vector<int> vpos(V, -1);      // local index in the current tile
+        const int ntile = (V + target - 1) / target, per = (V + ntile - 1) / std::max(ntile, 1);
+        for (int v0 = 0; v0 < V; v0 += per) {
+            const int v1 = std::min(V, v0 + per), n_own = v1 - v0;
+            // equal degrees side by side: the rows of entries have no holes
+            std::stable_sort(order.begin() + v0, order.begin() + v1, [&](auto &x, auto &y) {
+                return hc.soff[x.second + 1] - hc.soff[x.second] > hc.soff[y.second + 1] - hc.soff[y.second];
+            });
+            SolveTile tl{};
+            tl.cloth = c; tl.n_own = n_own; tl.pos = (int)vert.size(); tl.row = (int)rows.size();
+            tl.s0 = (int)ts.size(); tl.b0 = (int)tb.size();
+            int S = 0;
+            for (int i = 0; i < n_own; i += 32) {
+                int deg = 0;
+                for (int k = i; k < std::min(n_own, i + 32); ++k) {
+                    const int v = order[v0 + k].second;
+                    deg = std::max(deg, hc.soff[v + 1] - hc.soff[v]);
+                }
+                rows.push_back(S);
+                S += 32 * deg;
+            }
+            rows.push_back(S);
+            for (int i = 0; i < n_own; ++i) {
+                vpos[order[v0 + i].second] = i;
+                vert.push_back(order[v0 + i].second + (int)cd.v_off);
+            }
+            std::vector<int> halo;
+            auto local_of = [&](int v) {
+                if (vpos[v] < 0) {
+                    vpos[v] = n_own + (int)halo.size();
+                    halo.push_back(v);
+                    vert.push_back(v + (int)cd.v_off);
+                }
+                return (uint32_t)vpos[v];
+            };
+            const bool tri = cd.tri_bend;
+            for (int i = 0; i < n_own; ++i) {
+                const int v = order[v0 + i].second, at0 = rows[tl.row + i / 32] + i % 32;
+                for (int e = hc.soff[v]; e < hc.soff[v + 1]; ++e) {
+                    const uint32_t ent = hc.sent[e], k = ent & 0x1FFFFFFFu, role = (ent >> 29) & 3u;
+                    const uint32_t at = (uint32_t)(at0 + 32 * (e - hc.soff[v]));
+                    const uint32_t place = (at << (16 * (role & 1u))) | (0xffffu << (16 * (~role & 1u)));
+                    if (ent >> 31) {
+                        if (rec_b[k] < tl.b0) {
+                            const int4 id = hc.b_ids[k];
+                            const uint32_t a = local_of(id.x), b = local_of(id.y), p = local_of(id.z);
+                            rec_b[k] = (int)tb.size();
+                            tb.push_back(make_uint4(a | (b << 16), p | ((tri ? p : local_of(id.w)) << 16), ~0u, ~0u));
+                            bk.push_back((int)k + (int)cd.b_off);
+                        }
+                        uint4 &r = tb[rec_b[k]];
+                        (role < 2 ? r.z : r.w) &= place;
+                    } else {
+                        if (rec_s[k] < tl.s0) {
+                            const int2 id = hc.s_ids[k];
+                            const uint32_t a = local_of(id.x), b = local_of(id.y);
+                            rec_s[k] = (int)ts.size();
+                            ts.push_back(make_uint2(a | (b << 16), ~0u));
+                            sk.push_back((int)k + (int)cd.s_off);
+                        }
+                        ts[rec_s[k]].y &= place;
+                    }
+                }
+            }
+            tl.n_pos = n_own + (int)halo.size();
+            tl.s1 = (int)ts.size(); tl.b1 = (int)tb.size();
+            const size_t bytes = sizeof(float4) * (size_t)tl.n_pos + 3 * sizeof(float) * (size_t)S;
+            if (S >= 0xffff || tl.n_pos >= 0xffff || bytes > kSolveTileSmem) return LC_OK;
+            smem = std::max(smem, bytes);
+            tiles.push_back(tl);
+            for (int i = 0; i < n_own; ++i) vpos[order[v0 + i].second] = -1;
+            for (int v : halo) vpos[v] = -1;
+        }
+    }
+    if (tiles.empty() || !tiles_supported()) {
+        cudaGetLastError();
+        return LC_OK;
+    }
+    SolveTile *dt;
+    int *dv, *dr, *dsk, *dbk;
+    uint2 *dts;
+    uint4 *dtb;
+    LC_TRY(arena.alloc(dt, tiles.size(), "tiles")); LC_TRY(arena.alloc(dv, vert.size(), "tile vertices"));
+    LC_TRY(arena.alloc(dr, rows.size(), "tile rows"));
+    LC_TRY(arena.alloc(dts, ts.size() + 1, "tile stretch")); LC_TRY(arena.alloc(dtb, tb.size() + 1, "tile bends"));
+    LC_TRY(arena.alloc(dsk, sk.size() + 1, "tile stretch ids")); LC_TRY(arena.alloc(dbk, bk.size() + 1, "tile bend ids"));
+    LC_TRY(upload(dt, tiles)); LC_TRY(upload(dv, vert)); LC_TRY(upload(dr, rows));
+    LC_TRY(upload(dts, ts)); LC_TRY(upload(dtb, tb)); LC_TRY(upload(dsk, sk)); LC_TRY(upload(dbk, bk));
+    d.tile = dt; d.tile_vert = dv; d.tile_row = dr; d.tile_s = dts; d.tile_b = dtb; d.tile_sk = dsk; d.tile_bk = dbk;
+    d.ntiles = (int)tiles.size();
+    tile_smem = smem;
+    fit = true;
     return LC_OK;
 }
 

@@ -102,6 +102,19 @@ struct ClothState {
 };
 
 // Everything a step kernel may need, passed by value.
+// Global-memory solver: a tile of one cloth's vertices and the constraints that
+// touch them.  Local vertices: the tile's own first, then the others its
+// constraints read; own vertex i's correction entry j is rows[i / 32] + 32 j +
+// i % 32.
+struct SolveTile {
+    int cloth, n_own, n_pos;
+    int pos;            // tile_vert: global ids of the local vertices
+    int row;            // tile_row: first entry of each 32 own vertices
+    int s0, s1, b0, b1; // tile_s / tile_b records
+};
+constexpr int kSolveTileThreads = 512;
+constexpr size_t kSolveTileSmem = 112 * 1024;  // positions and entries: two tiles on an SM
+
 struct DevPtrs {
     int C;                 // cloths
     int Vtot, Ttot, Ntot, Itot;
@@ -178,6 +191,13 @@ struct DevPtrs {
     // global-memory solver, one iteration: a row of Etot for the stretch
     // constraints and four of Btot for the bends (see k_constraints)
     float4 *corr;
+    // or, tile by tile (ntiles != 0)
+    int ntiles;
+    const SolveTile *tile;
+    const int *tile_vert, *tile_row;
+    const uint2 *tile_s;    // local vertices, entries (16 bits each; 0xffff: another tile's)
+    const uint4 *tile_b;
+    const int *tile_sk, *tile_bk;  // the constraints
     int Etot, Btot;
     // LRA / ground
     const int *fixed;      // global ids of pinned vertices, per cloth at f_off

@@ -321,17 +321,20 @@ __global__ void k_sphere(DevPtrs d) {
 }
 
 // ---------------------------------------------------------------------------
-// Jacobi iteration (Physics/CudaPBD.cu:648-659) in two launches.
-// k_constraints evaluates every stretch and bend constraint once on the
-// positions of the previous iteration (xa) and stores what the corrections of
-// its vertices share, constraint by constraint; k_jacobi scales and sums a
-// vertex's corrections in order, adds the terms that are its own and the
-// contacts, and writes its update to xb.  Bound by the L2: 64 bytes written
-// and 128 read per edge with its bend, which stay there for 512 x 512 vertices
-// (105 MB with the constraints' own data).  An iteration of that cloth takes
-// JACOBI_US; 72 us when each vertex evaluated its 18 constraints itself (a chain of
-// three loads per evaluation), 67 us when every correction was stored at its
-// vertex's place (scattered half-sector writes).  The sum is
+// Jacobi iteration (Physics/CudaPBD.cu:648-659), one launch, a block per tile of
+// a cloth's vertices (k_jacobi_tile): every constraint that touches the tile is
+// evaluated once on the positions of the previous iteration (xa), and its
+// corrections for the tile's own vertices go to their entries in shared memory;
+// a vertex sums its entries in order, adds the terms that are its own and the
+// contacts, and writes its update to xb.  Bound by instructions, two thirds of
+// them the bends', and by the wait for positions and records at a block's
+// start.  Us per iteration, 32, 128, 256, 512 and 724 squared vertices:
+//   18 constraints evaluated at each vertex           26, 26, 33, 76, 147
+//   once each, shared through memory (two launches)   17, 18, 25, 61, 122
+//   tiles                                             10, 12, 15, 35, 70
+// The second (k_constraints, k_jacobi) writes and reads 160 bytes per edge and
+// its bend, 120 MB at 512 squared, which the L2 does not hold; it remains for
+// cloths whose entries do not fit tiles.  In all three the sum is
 // associated like the reference's accumulator: ((ground + LRA) + static) +
 // dynamic, then x += acc / count.
 // ---------------------------------------------------------------------------
@@ -382,18 +385,12 @@ __global__ void __launch_bounds__(kThreads) k_constraints(DevPtrs d, const float
 }
 
 constexpr int kEntryBatch = 6;
-__global__ void k_jacobi(DevPtrs d, const float4 *__restrict__ xa, float4 *__restrict__ xb, int it,
-                         const uint32_t *__restrict__ nvf_dev) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= d.Vtot) return;
-    const int c = d.vcloth[i];
-    const ClothDev &cd = d.cloth[c];
-    const float4 xi4 = xa[i];
-    if (it >= cd.iters) {
-        xb[i] = xi4;
-        if (d.coll_act) d.coll_act[(size_t)(it + 1) * d.Vtot + i] = 0;
-        return;
-    }
+// One vertex's update.  static_sum(): its stretch and bend corrections, summed
+// in entry order.
+template <class Sum>
+__device__ __forceinline__ void jacobi_vertex(const DevPtrs &d, const ClothDev &cd, const float4 *__restrict__ xa,
+                                              float4 *__restrict__ xb, int it, const uint32_t *__restrict__ nvf_dev,
+                                              int i, float4 xi4, int n_static, Sum static_sum) {
     const float3 xi = xyz(xi4);
     float3 acc = f3(0.f, 0.f, 0.f);
     int cnt = 0;
@@ -427,29 +424,8 @@ __global__ void k_jacobi(DevPtrs d, const float4 *__restrict__ xa, float4 *__res
         cnt += lc;
     }
     // static stretch + bend, Physics/CudaPBD.cu:942-1147, 1417-1446
-    {
-        float3 sa = f3(0.f, 0.f, 0.f);
-        const int s0 = d.soff[i], s1 = d.soff[i + 1];
-        for (int e = s0; e < s1; e += kEntryBatch) {  // the loads of a batch in flight together
-            uint32_t ent[kEntryBatch];
-            float4 r[kEntryBatch];
-#pragma unroll
-            for (int j = 0; j < kEntryBatch; ++j) ent[j] = __ldg(&d.sent[min(e + j, s1 - 1)]);
-#pragma unroll
-            for (int j = 0; j < kEntryBatch; ++j) {
-                const uint32_t k = ent[j] & 0x1FFFFFFFu, role = (ent[j] >> 29) & 3u;
-                r[j] = d.corr[(ent[j] >> 31) ? (size_t)d.Etot + role * (size_t)d.Btot + k : (size_t)k];
-            }
-#pragma unroll
-            for (int j = 0; j < kEntryBatch; ++j) {
-                if (e + j >= s1) break;
-                const float f = xi4.w * r[j].w;
-                sa = add(sa, mul(xyz(r[j]), (ent[j] >> 29) == 1u ? f : -f));
-            }
-        }
-        acc = add(acc, sa);
-        cnt += s1 - s0;
-    }
+    acc = add(acc, static_sum());
+    cnt += n_static;
     // dynamic VF / EE, Physics/CudaPBD.cu:1190-1415, 1448-1475
     {
         const uint32_t e0 = d.dyn_off[i], e1 = d.dyn_off[i + 1];
@@ -476,6 +452,108 @@ __global__ void k_jacobi(DevPtrs d, const float4 *__restrict__ xa, float4 *__res
         else if (act) *act = 0;
     }
     xb[i] = f4(xn, xi4.w);
+}
+
+__device__ __forceinline__ void jacobi_idle(const DevPtrs &d, float4 *__restrict__ xb, int it, int i, float4 xi4) {
+    xb[i] = xi4;
+    if (d.coll_act) d.coll_act[(size_t)(it + 1) * d.Vtot + i] = 0;
+}
+
+__global__ void k_jacobi(DevPtrs d, const float4 *__restrict__ xa, float4 *__restrict__ xb, int it,
+                         const uint32_t *__restrict__ nvf_dev) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= d.Vtot) return;
+    const ClothDev &cd = d.cloth[d.vcloth[i]];
+    const float4 xi4 = xa[i];
+    if (it >= cd.iters) { jacobi_idle(d, xb, it, i, xi4); return; }
+    const int s0 = d.soff[i], s1 = d.soff[i + 1];
+    jacobi_vertex(d, cd, xa, xb, it, nvf_dev, i, xi4, s1 - s0, [&]() {
+        float3 sa = f3(0.f, 0.f, 0.f);
+        for (int e = s0; e < s1; e += kEntryBatch) {  // the loads of a batch in flight together
+            uint32_t ent[kEntryBatch];
+            float4 r[kEntryBatch];
+#pragma unroll
+            for (int j = 0; j < kEntryBatch; ++j) ent[j] = __ldg(&d.sent[min(e + j, s1 - 1)]);
+#pragma unroll
+            for (int j = 0; j < kEntryBatch; ++j) {
+                const uint32_t k = ent[j] & 0x1FFFFFFFu, role = (ent[j] >> 29) & 3u;
+                r[j] = d.corr[(ent[j] >> 31) ? (size_t)d.Etot + role * (size_t)d.Btot + k : (size_t)k];
+            }
+#pragma unroll
+            for (int j = 0; j < kEntryBatch; ++j) {
+                if (e + j >= s1) break;
+                const float f = xi4.w * r[j].w;
+                sa = add(sa, mul(xyz(r[j]), (ent[j] >> 29) == 1u ? f : -f));
+            }
+        }
+        return sa;
+    });
+}
+
+// 12 bytes per entry: two blocks of 431 vertices of degree 18 on an SM.  Reading
+// the records a turn ahead, or bends and stretches from one list, was 4% slower.
+__global__ void __launch_bounds__(kSolveTileThreads, 2) k_jacobi_tile(DevPtrs d, const float4 *__restrict__ xa,
+                                                                 float4 *__restrict__ xb, int it,
+                                                                 const uint32_t *__restrict__ nvf_dev) {
+    extern __shared__ float4 s_pos[];
+    const SolveTile tl = d.tile[blockIdx.x];
+    const ClothDev &cd = d.cloth[tl.cloth];
+    const int t = threadIdx.x, lane = t & 31;
+    const int *vert = d.tile_vert + tl.pos, *row = d.tile_row + tl.row;
+    if (it >= cd.iters) {
+        for (int i = t; i < tl.n_own; i += kSolveTileThreads) jacobi_idle(d, xb, it, vert[i], xa[vert[i]]);
+        return;
+    }
+    const int rows = (tl.n_own + 31) / 32, S = row[rows];
+    float *cx = reinterpret_cast<float *>(s_pos + tl.n_pos), *cy = cx + S, *cz = cy + S;
+    auto put = [&](uint32_t at, float3 v) {
+        if (at == 0xffffu) return;
+        cx[at] = v.x; cy[at] = v.y; cz[at] = v.z;
+    };
+    for (int i = t; i < tl.n_pos; i += kSolveTileThreads) s_pos[i] = xa[vert[i]];
+    __syncthreads();
+    for (int r = tl.s0 + t; r < tl.s1; r += kSolveTileThreads) {
+        const uint2 rec = __ldg(&d.tile_s[r]);
+        const float2 par = __ldg(&d.s_par[__ldg(&d.tile_sk[r])]);
+        float3 out[2];
+        if (!stretch_all_pos(s_pos[rec.x & 0xffffu], s_pos[rec.x >> 16], par.x, par.y, out)) out[0] = out[1] = f3(0.f, 0.f, 0.f);
+        put(rec.y & 0xffffu, out[0]);
+        put(rec.y >> 16, out[1]);
+    }
+    const bool tri = cd.tri_bend;
+    for (int r = tl.b0 + t; r < tl.b1; r += kSolveTileThreads) {
+        const uint4 rec = __ldg(&d.tile_b[r]);
+        const int k = __ldg(&d.tile_bk[r]);
+        const float kp = __ldg(&d.b_kp[k]);
+        const float4 p0 = s_pos[rec.x & 0xffffu], p1 = s_pos[rec.x >> 16], p2 = s_pos[rec.y & 0xffffu];
+        if (tri) {
+            const float3 tv = tri_bend_vec_pos(p0, p1, p2, kp, __int_as_float(d.b_ids[k].w));
+            put(rec.z & 0xffffu, mul(tv, 2.f * p0.w));
+            put(rec.z >> 16, mul(tv, 2.f * p1.w));
+            put(rec.w & 0xffffu, mul(tv, -4.f * p2.w));
+            continue;
+        }
+        const float4 p3 = s_pos[rec.y >> 16];
+        float3 q[4];
+        float s;
+        if (!bend_all_pos(p0, p1, p2, p3, kp, d.kpi_gap, q, s)) {
+            q[0] = q[1] = q[2] = q[3] = f3(0.f, 0.f, 0.f);
+            s = 0.f;
+        }
+        put(rec.z & 0xffffu, mul(q[0], -(p0.w * s)));
+        put(rec.z >> 16, mul(q[1], -(p1.w * s)));
+        put(rec.w & 0xffffu, mul(q[2], -(p2.w * s)));
+        put(rec.w >> 16, mul(q[3], -(p3.w * s)));
+    }
+    __syncthreads();
+    for (int i = t; i < tl.n_own; i += kSolveTileThreads) {
+        const int g = vert[i], n = d.soff[g + 1] - d.soff[g], at = row[i >> 5] + lane;
+        jacobi_vertex(d, cd, xa, xb, it, nvf_dev, g, s_pos[i], n, [&]() {
+            float3 sa = f3(0.f, 0.f, 0.f);
+            for (int j = 0; j < n; ++j) sa = add(sa, f3(cx[at + 32 * j], cy[at + 32 * j], cz[at + 32 * j]));
+            return sa;
+        });
+    }
 }
 
 // _FinalUpdate (Physics/CudaPBD.cu:1916-1932) then _WorldConstraints
@@ -528,8 +606,15 @@ void launch_solver_setup(const DevPtrs &d, bool sphere, cudaStream_t st) {
     k_solver_setup<<<nblk(d.Vtot), kThreads, 0, st>>>(d);
     if (sphere) k_sphere<<<nblk(d.Vtot), kThreads, 0, st>>>(d);
 }
+bool tiles_supported() {
+    return cudaFuncSetAttribute(k_jacobi_tile, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSolveTileSmem) == cudaSuccess;
+}
 void launch_jacobi(const DevPtrs &d, const float4 *xa, float4 *xb, int it, const uint32_t *nvf, int block,
-                   cudaStream_t st) {
+                   size_t tile_smem, cudaStream_t st) {
+    if (d.ntiles) {
+        k_jacobi_tile<<<d.ntiles, kSolveTileThreads, tile_smem, st>>>(d, xa, xb, it, nvf);
+        return;
+    }
     const int nbs = nblk(d.Etot), nbb = nblk(d.Btot);
     if (nbs + nbb) k_constraints<<<nbs + nbb, kThreads, 0, st>>>(d, xa, nbs);
     if (d.Vtot) k_jacobi<<<nblk(d.Vtot, block), block, 0, st>>>(d, xa, xb, it, nvf);
