@@ -1703,6 +1703,29 @@ __device__ __forceinline__ bool ee_far(float3 a, float3 b, float3 c, float3 d, f
            fminf(a.z, b.z) - fmaxf(c.z, d.z) > m || fminf(c.z, d.z) - fmaxf(a.z, b.z) > m;
 }
 
+// Whether two edges moving with constant velocities are further apart than a
+// test_ee hit allows at every advance T of [lo, hi]: their projections on one
+// axis, the line through their midpoints halfway, are apart by more than th
+// plus the margin at both ends (the gap, a minimum of linear functions of T less
+// a maximum of such, is concave, so nowhere between the ends is it smaller).  The margin
+// also covers what the roundings of the advances, and of this, add at the
+// coordinates' size.  NaN anywhere: not apart.
+__device__ __forceinline__ bool ee_apart(float3 x1, float3 x2, float3 x3, float3 x4, float3 v1, float3 v2, float3 v3,
+                                         float3 v4, float lo, float hi, float th) {
+    const float3 u = sub(x2, x1), v = sub(x3, x1), w = sub(x4, x1);
+    const float3 du = sub(v2, v1), dv = sub(v3, v1), dw = sub(v4, v1);
+    const float mid = 0.5f * (lo + hi);
+    const float3 m = add(sub(add(v, w), u), mul(sub(add(dv, dw), du), mid));
+    const float pu = dot(u, m), pv = dot(v, m), pw = dot(w, m);
+    const float qu = dot(du, m), qv = dot(dv, m), qw = dot(dw, m);
+    const float gl = fminf(pv + qv * lo, pw + qw * lo) - fmaxf(pu + qu * lo, 0.f);
+    const float gh = fminf(pv + qv * hi, pw + qw * hi) - fmaxf(pu + qu * hi, 0.f);
+    const float size = fabsf(x1.x) + fabsf(x1.y) + fabsf(x1.z) +
+                       fmaxf(fabsf(lo), fabsf(hi)) * (fabsf(v1.x) + fabsf(v1.y) + fabsf(v1.z));
+    const float t = 1.001f * th + 1e-5f + 4e-6f * size;
+    return fminf(gl, gh) > 0.f && gl * gl > t * t * dot(m, m) && gh * gh > t * t * dot(m, m);
+}
+
 // Particle swept box of Collision/FeatureList.cu:134-148, recomputed from
 // x and x_prev (min/max are exact, so this equals the stored boxes).
 struct Box { float3 lo, hi; };
@@ -1910,23 +1933,79 @@ __global__ void k_narrow_expand(DevPtrs d, const uint32_t *__restrict__ npairs) 
 // until one test hits.  Here each warp takes 32 candidates at a time:
 // (1) every lane sets up its candidate's cubic, evaluates f at the interval
 // ends and queues the intervals that need a secant solve; (2) the warp runs
-// the queued solves, one per lane; (3) every lane tests its times in the
-// reference's order with the cumulative advance and stops at the first hit.
+// the queued solves, one per lane; (3) VF: the tests of all candidates and
+// times are spread over the lanes; EE: a candidate whose edges stay apart at all
+// of its times (ee_apart: 19 in 20 of those of a batch in contact) is done, and
+// the others are queued until 32 are together, whose tests one call runs.
 // The operands and operations of every piece are the reference's, so the
-// decisions are the same bits; only the assignment of work to lanes differs.
+// decisions are the same bits; only the assignment of work to lanes, and
+// which tests that cannot hit are run, differs.  Bound by issue slots, for EE 30%
+// set-up and 45% secant solves, with half of the lanes on (22 of 32 have a
+// solve, and they end after 7 iterations on average and 16 at the latest).
+// 17 million candidates of 24 cloths up to 160 squared, half of them: EE 199 us
+// with the tests spread as for VF (47% of the time), 134 so; VF 80.
 constexpr int kCcdWarps = 8;
-struct CcdJob { float a, b, fa, fb; };
+constexpr int kNearCap = 64;  // 31 left over and 32 more
 
-// At most 64 registers, for 4 resident blocks per SM instead of 3 (a few
-// words spill to L1): measured 0.83 -> 0.80 ms per step for VF, EE unchanged.
+// A hit: its contact's weights, placed at their final index by k_ccd_emit.
 template <bool VF>
-__global__ void __launch_bounds__(kCcdWarps * 32, 4) k_ccd_warp(DevPtrs d, const uint32_t *__restrict__ ncand) {
-    __shared__ float geom[kCcdWarps][24][33];     // x1..x4 then v1..v4 (test order) per lane (padded)
-    __shared__ CcdJob jobs[kCcdWarps][96];
-    __shared__ uint8_t job_owner[kCcdWarps][96];  // lane << 2 | interval
-    __shared__ float roots[kCcdWarps][3][32];
-    __shared__ float tq[kCcdWarps][6][32];        // each lane's times to test, in the reference's order
-    __shared__ int best[kCcdWarps][32];           // each lane's first hitting test (6: none)
+__device__ __forceinline__ void record_hit(const DevPtrs &d, uint32_t q, const Wts &wt) {
+    const uint64_t cap = VF ? d.vf_cap : d.ee_cap;
+    const uint32_t slot = atomicAdd(&d.hit_n[VF ? 0 : 1], 1u);
+    if (slot < cap) {
+        d.hit_q[VF ? 0 : 1][slot] = q;
+        d.hit_w[VF ? 0 : 1][slot] = make_float4(wt.w0, wt.w1, wt.w2, wt.w3);
+        if (VF && d.hit_nrm) d.hit_nrm[slot] = make_float4(wt.n.x, wt.n.y, wt.n.z, 0.f);
+        if (d.hit_tn[VF ? 0 : 1]) d.hit_tn[VF ? 0 : 1][slot] = make_float4(wt.n.x, wt.n.y, wt.n.z, wt.t);
+    } else {
+        atomicOr(d.err, VF ? ERR_VF_OVERFLOW : ERR_EE_OVERFLOW);
+    }
+}
+
+// The ordered tests of queued EE candidate q, whose times are t[kNearCap k]:
+// the same advances and tests, up to a hit.  A call, not inlined: the loop over
+// the candidates then fits the instruction cache (EE 190 -> 171 us).
+__device__ __noinline__ void test_near(const DevPtrs &d, uint32_t q, int nt, const float *t) {
+    const int4 ids = d.cand_e[q];
+    const ClothDev &cd = d.cloth[d.vcloth[ids.x]];
+    const float h = cd.h, dt = cd.dt;
+    float3 x1 = xyz(d.xp[ids.x]), x2 = xyz(d.xp[ids.y]), x3 = xyz(d.xp[ids.z]), x4 = xyz(d.xp[ids.w]);
+    const float3 v1 = xyz(d.v[ids.x]), v2 = xyz(d.v[ids.y]), v3 = xyz(d.v[ids.z]), v4 = xyz(d.v[ids.w]);
+    for (int k = 0; k < nt; ++k) {
+        const float tt = t[k * kNearCap] * dt;
+        x1 = add(x1, mul(v1, tt));
+        x2 = add(x2, mul(v2, tt));
+        x3 = add(x3, mul(v3, tt));
+        x4 = add(x4, mul(v4, tt));
+        Wts wt;
+        if (ee_far(x1, x2, x3, x4, h) || !test_ee(x1, x2, x3, x4, h, wt)) continue;
+        wt.t = tt;  // the contact's time (Collision/CudaPrimitiveTests.cu:174, 228)
+        record_hit<false>(d, q, wt);
+        atomicOr(&d.hitg_mask[1][q / 32], 1u << (q & 31u));
+        atomicAdd(&d.hitg_cnt[1][q / 32], 1u);
+        return;
+    }
+}
+
+// At most 64 registers, for 4 resident blocks per SM instead of 3: EE 134 us
+// against 150.
+template <bool VF>
+__global__ void __launch_bounds__(kCcdWarps * 32, 4) k_ccd_warp(const __grid_constant__ DevPtrs d,
+                                                                const uint32_t *__restrict__ ncand) {
+    __shared__ float4 geom[kCcdWarps][6][32];     // x1..x4 then v1..v4 (test order) per lane
+    __shared__ float fval[kCcdWarps][4][32];      // f at the interval ends
+    __shared__ float ends[kCcdWarps][2][32];      // the inner ends
+    __shared__ uint8_t job_owner[kCcdWarps][96];  // queued secant solves: lane << 2 | interval
+    // each lane's times to test, in the reference's order: interval i's start
+    // (if f is 0 there) at 2 i, its root at 2 i + 1
+    __shared__ float tq[kCcdWarps][6][32];
+    __shared__ int cloth_of[kCcdWarps][32];
+    __shared__ int best[VF ? kCcdWarps : 1][32];     // VF: each lane's first hitting test (6: none)
+    // EE: candidates not apart, until 32 are together
+    __shared__ uint32_t near_q[VF ? 1 : kCcdWarps][kNearCap];
+    __shared__ uint8_t near_n[VF ? 1 : kCcdWarps][kNearCap];
+    __shared__ float near_t[VF ? 1 : kCcdWarps][6][kNearCap];
+    int nnear = 0;
     const uint32_t n = (uint32_t)min((uint64_t)*ncand, d.cand_cap);
     const int4 *list = VF ? d.cand : d.cand_e;
     // hit bits per group of 32 candidates (one warp iteration: base is a
@@ -1943,19 +2022,21 @@ __global__ void __launch_bounds__(kCcdWarps * 32, 4) k_ccd_warp(DevPtrs d, const
         int ncp = -1;
         float e1 = 1.f, e2 = 1.f;
         unsigned imm = 0, sec = 0;
-        float fv[4] = {0.f, 0.f, 0.f, 0.f};
         if (valid) {
             ids = list[q];
             // VF: face ids.y ids.z ids.w, vertex ids.x (x4); EE: x1..x4 = ids
             const int i1 = VF ? ids.y : ids.x, i2 = VF ? ids.z : ids.y, i3 = VF ? ids.w : ids.z, i4 = VF ? ids.x : ids.w;
+            cloth_of[w][lane] = d.vcloth[ids.x];
             const float3 x1 = xyz(d.xp[i1]), x2 = xyz(d.xp[i2]), x3 = xyz(d.xp[i3]), x4 = xyz(d.xp[i4]);
             const float3 v1 = xyz(d.v[i1]), v2 = xyz(d.v[i2]), v3 = xyz(d.v[i3]), v4 = xyz(d.v[i4]);
             const float3 x21 = sub(x2, x1), x31 = sub(x3, x1), x41 = sub(x4, x1);
             const float3 v21 = sub(v2, v1), v31 = sub(v3, v1), v41 = sub(v4, v1);
-            const float g[24] = {x1.x, x1.y, x1.z, x2.x, x2.y, x2.z, x3.x, x3.y, x3.z, x4.x, x4.y, x4.z,
-                                 v1.x, v1.y, v1.z, v2.x, v2.y, v2.z, v3.x, v3.y, v3.z, v4.x, v4.y, v4.z};
-#pragma unroll
-            for (int k = 0; k < 24; ++k) geom[w][k][lane] = g[k];
+            geom[w][0][lane] = make_float4(x1.x, x1.y, x1.z, x2.x);
+            geom[w][1][lane] = make_float4(x2.y, x2.z, x3.x, x3.y);
+            geom[w][2][lane] = make_float4(x3.z, x4.x, x4.y, x4.z);
+            geom[w][3][lane] = make_float4(v1.x, v1.y, v1.z, v2.x);
+            geom[w][4][lane] = make_float4(v2.y, v2.z, v3.x, v3.y);
+            geom[w][5][lane] = make_float4(v3.z, v4.x, v4.y, v4.z);
             const float3 v21v31 = cross(v21, v31), x21v31 = cross(x21, v31), v21x31 = cross(v21, x31),
                          x21x31 = cross(x21, x31);
             const float v1v2v3 = dot(v21v31, v41), x1v2v3 = dot(x21v31, v41), v1x2v3 = dot(v21x31, v41),
@@ -1976,16 +2057,31 @@ __global__ void __launch_bounds__(kCcdWarps * 32, 4) k_ccd_warp(DevPtrs d, const
             }
             e1 = ncp >= 1 ? t1 : 1.f;
             e2 = ncp == 2 ? t2 : 1.f;
-            fv[0] = triple(x21, x31, x41, v21, v31, v41, 0.f);
-#pragma unroll
-            for (int i = 0; i <= 2; ++i) {
-                if (i > ncp) break;
-                const float b = i == ncp ? 1.f : (i == 0 ? e1 : e2);
-                fv[i + 1] = triple(x21, x31, x41, v21, v31, v41, b);
-                if (fabsf(fv[i]) < kEpsCubic) imm |= 1u << i;
-                if (fv[i] * fv[i + 1] < 0.f) sec |= 1u << i;
+            ends[w][0][lane] = e1;
+            ends[w][1][lane] = e2;
+            tq[w][0][lane] = 0.f;
+            tq[w][2][lane] = e1;
+            tq[w][4][lane] = e2;
+            float fa = triple(x21, x31, x41, v21, v31, v41, 0.f);
+            fval[w][0][lane] = fa;
+#pragma unroll 1
+            for (int i = 0; i <= ncp; ++i) {
+                const float fb = triple(x21, x31, x41, v21, v31, v41, i == ncp ? 1.f : (i == 0 ? e1 : e2));
+                fval[w][i + 1][lane] = fb;
+                if (fabsf(fa) < kEpsCubic) imm |= 1u << i;
+                if (fa * fb < 0.f) sec |= 1u << i;
+                fa = fb;
             }
         }
+        // the four vertices of lane L's candidate in test order (VF: face x1 x2 x3,
+        // vertex x4), as its set-up loaded them
+        auto corners = [&](int L, float3 &x1, float3 &x2, float3 &x3, float3 &x4, float3 &v1, float3 &v2,
+                           float3 &v3, float3 &v4) {
+            const float4(*gm)[32] = geom[w];
+            const float4 a = gm[0][L], b = gm[1][L], c = gm[2][L], e = gm[3][L], f = gm[4][L], g = gm[5][L];
+            x1 = f3(a.x, a.y, a.z); x2 = f3(a.w, b.x, b.y); x3 = f3(b.z, b.w, c.x); x4 = f3(c.y, c.z, c.w);
+            v1 = f3(e.x, e.y, e.z); v2 = f3(e.w, f.x, f.y); v3 = f3(f.z, f.w, g.x); v4 = f3(g.y, g.z, g.w);
+        };
         // queue the secant solves of the warp
         int njobs = 0;
 #pragma unroll
@@ -1994,133 +2090,135 @@ __global__ void __launch_bounds__(kCcdWarps * 32, 4) k_ccd_warp(DevPtrs d, const
             const unsigned m = __ballot_sync(full, want);
             if (want) {
                 const int pos = njobs + __popc(m & ((1u << lane) - 1u));
-                const float a = i == 0 ? 0.f : (i == 1 ? e1 : e2);
-                const float b = i == ncp ? 1.f : (i == 0 ? e1 : e2);
-                jobs[w][pos] = CcdJob{a, b, fv[i], fv[i + 1]};
                 job_owner[w][pos] = (uint8_t)(lane << 2 | i);
             }
             njobs += __popc(m);
         }
         __syncwarp();
         for (int j = lane; j < njobs; j += 32) {
-            const CcdJob jb = jobs[w][j];
             const int own = job_owner[w][j] >> 2, iv = job_owner[w][j] & 3;
-            // the set-up's differences, from the same operands
-            const float3 p1 = f3(geom[w][0][own], geom[w][1][own], geom[w][2][own]);
-            const float3 u1 = f3(geom[w][12][own], geom[w][13][own], geom[w][14][own]);
-            const float3 x21 = sub(f3(geom[w][3][own], geom[w][4][own], geom[w][5][own]), p1);
-            const float3 x31 = sub(f3(geom[w][6][own], geom[w][7][own], geom[w][8][own]), p1);
-            const float3 x41 = sub(f3(geom[w][9][own], geom[w][10][own], geom[w][11][own]), p1);
-            const float3 v21 = sub(f3(geom[w][15][own], geom[w][16][own], geom[w][17][own]), u1);
-            const float3 v31 = sub(f3(geom[w][18][own], geom[w][19][own], geom[w][20][own]), u1);
-            const float3 v41 = sub(f3(geom[w][21][own], geom[w][22][own], geom[w][23][own]), u1);
-            roots[w][iv][own] = secant(x21, x31, x41, v21, v31, v41, jb.a, jb.b, jb.fa, jb.fb);
-        }
-        __syncwarp();
-        // The ordered tests of every candidate (the reference advances the
-        // four positions by v t dt for each time in turn and tests after each
-        // advance, stopping at the first hit).  Every (candidate, time) test
-        // of the warp is a job of its own, spread evenly over the lanes: a
-        // job rebuilds its positions by the same sequence of advances and
-        // runs the same test, so it decides the same bits.  A candidate's
-        // first hit is its smallest hitting test index; its owner lane then
-        // runs that test once more for the weights.
-        int nt = 0;
-        float hq = 0.f, dtq = 0.f;
-        if (valid) {
-            for (int i = 0; i <= ncp; ++i) {
-                const float a = i == 0 ? 0.f : (i == 1 ? e1 : e2);
-                if ((imm >> i) & 1u) tq[w][nt++][lane] = a;
-                if ((sec >> i) & 1u) {
-                    const float t = roots[w][i][lane];
-                    if (t != -15.f) tq[w][nt++][lane] = t;
-                }
-            }
-            const ClothDev &cd = d.cloth[d.vcloth[ids.x]];
-            hq = cd.h;
-            dtq = cd.dt;
-        }
-        best[w][lane] = 6;
-        uint32_t ex = (uint32_t)nt;  // inclusive scan of the test counts
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            const uint32_t t = __shfl_up_sync(full, ex, o);
-            if (lane >= o) ex += t;
-        }
-        const uint32_t ntests = __shfl_sync(full, ex, 31);
-        ex -= (uint32_t)nt;
-        __syncwarp();
-        // the four vertices of lane L's candidate in test order (VF: face x1 x2 x3,
-        // vertex x4), as its set-up loaded them
-        auto corners = [&](int L, float3 &x1, float3 &x2, float3 &x3, float3 &x4, float3 &v1, float3 &v2,
-                           float3 &v3, float3 &v4) {
-            const float(*gm)[33] = geom[w];
-            x1 = f3(gm[0][L], gm[1][L], gm[2][L]); x2 = f3(gm[3][L], gm[4][L], gm[5][L]);
-            x3 = f3(gm[6][L], gm[7][L], gm[8][L]); x4 = f3(gm[9][L], gm[10][L], gm[11][L]);
-            v1 = f3(gm[12][L], gm[13][L], gm[14][L]); v2 = f3(gm[15][L], gm[16][L], gm[17][L]);
-            v3 = f3(gm[18][L], gm[19][L], gm[20][L]); v4 = f3(gm[21][L], gm[22][L], gm[23][L]);
-        };
-        // test m of lane L's candidate: the advances by its times 0..m, then the test
-        auto run_test = [&](int L, int m, float h, float dt, Wts &wt) {
             float3 x1, x2, x3, x4, v1, v2, v3, v4;
-            corners(L, x1, x2, x3, x4, v1, v2, v3, v4);
-            float tt = 0.f;
-            for (int k = 0; k <= m; ++k) {
-                tt = tq[w][k][L] * dt;
-                x1 = add(x1, mul(v1, tt));
-                x2 = add(x2, mul(v2, tt));
-                x3 = add(x3, mul(v3, tt));
-                x4 = add(x4, mul(v4, tt));
-            }
-            if (!VF && ee_far(x1, x2, x3, x4, h)) return false;
-            const bool r = VF ? test_vf(x4, x1, x2, x3, h, wt) : test_ee(x1, x2, x3, x4, h, wt);
-            wt.t = tt;  // the contact's time (Collision/CudaPrimitiveTests.cu:174, 228)
-            return r;
-        };
-        for (uint32_t j0 = 0; j0 < ntests; j0 += 32) {
-            const uint32_t j = j0 + lane;
-            int L = 0;  // owner: the last lane whose first test is <= j
-#pragma unroll
-            for (int step = 16; step > 0; step >>= 1) {
-                const int cand = L + step;
-                const uint32_t e = __shfl_sync(full, ex, cand & 31);
-                if (cand < 32 && e <= j) L = cand;
-            }
-            const uint32_t exL = __shfl_sync(full, ex, L);
-            const float h = __shfl_sync(full, hq, L), dt = __shfl_sync(full, dtq, L);
-            if (j < ntests) {
-                const int m = (int)(j - exL);
-                Wts wt;
-                if (run_test(L, m, h, dt, wt)) atomicMin(&best[w][L], m);
-            }
+            corners(own, x1, x2, x3, x4, v1, v2, v3, v4);
+            // (an outer end's place holds 1 where there are fewer intervals)
+            const float a = iv == 0 ? 0.f : ends[w][iv - 1][own], b = iv == 2 ? 1.f : ends[w][iv][own];
+            // the set-up's differences, from the same operands
+            tq[w][2 * iv + 1][own] = secant(sub(x2, x1), sub(x3, x1), sub(x4, x1), sub(v2, v1), sub(v3, v1), sub(v4, v1), a, b,
+                                          fval[w][iv][own], fval[w][iv + 1][own]);
         }
         __syncwarp();
-        bool found = false;
-        Wts wt;
-        if (valid && best[w][lane] < 6) found = run_test(lane, best[w][lane], hq, dtq, wt);
-        if (valid) {
-            if (found) {
-                // the contact's weights, placed at its final index by k_ccd_emit
-                const uint64_t cap = VF ? d.vf_cap : d.ee_cap;
-                const uint32_t slot = atomicAdd(&d.hit_n[VF ? 0 : 1], 1u);
-                if (slot < cap) {
-                    d.hit_q[VF ? 0 : 1][slot] = q;
-                    d.hit_w[VF ? 0 : 1][slot] = make_float4(wt.w0, wt.w1, wt.w2, wt.w3);
-                    if (VF && d.hit_nrm) d.hit_nrm[slot] = make_float4(wt.n.x, wt.n.y, wt.n.z, 0.f);
-                    if (d.hit_tn[VF ? 0 : 1]) d.hit_tn[VF ? 0 : 1][slot] = make_float4(wt.n.x, wt.n.y, wt.n.z, wt.t);
-                } else {
-                    atomicOr(d.err, VF ? ERR_VF_OVERFLOW : ERR_EE_OVERFLOW);
+        unsigned times = (imm & 1u) | (imm & 2u) << 1 | (imm & 4u) << 2;
+#pragma unroll
+        for (int i = 0; i <= 2; ++i)
+            if (((sec >> i) & 1u) && tq[w][2 * i + 1][lane] != -15.f) times |= 2u << (2 * i);
+        if constexpr (VF) {
+            // The ordered tests of every candidate (the reference advances the
+            // four positions by v t dt for each time in turn and tests after each
+            // advance, stopping at the first hit).  Every (candidate, time) test
+            // of the warp is a job of its own, spread evenly over the lanes: a
+            // job rebuilds its positions by the same sequence of advances and
+            // runs the same test, so it decides the same bits.  A candidate's
+            // first hit is its smallest hitting test index; its owner lane then
+            // runs that test once more for the weights.
+            int nt = 0;
+            float hq = 0.f, dtq = 0.f;
+            if (valid) {
+                for (; times; times &= times - 1u) tq[w][nt++][lane] = tq[w][__ffs(times) - 1][lane];
+                hq = d.cloth[cloth_of[w][lane]].h;
+                dtq = d.cloth[cloth_of[w][lane]].dt;
+            }
+            best[w][lane] = 6;
+            uint32_t ex = (uint32_t)nt;  // inclusive scan of the test counts
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const uint32_t t = __shfl_up_sync(full, ex, o);
+                if (lane >= o) ex += t;
+            }
+            const uint32_t ntests = __shfl_sync(full, ex, 31);
+            ex -= (uint32_t)nt;
+            __syncwarp();
+            // test m of lane L's candidate: the advances by its times 0..m, then the test
+            auto run_test = [&](int L, int m, float h, float dt, Wts &wt) {
+                float3 x1, x2, x3, x4, v1, v2, v3, v4;
+                corners(L, x1, x2, x3, x4, v1, v2, v3, v4);
+                float tt = 0.f;
+                for (int k = 0; k <= m; ++k) {
+                    tt = tq[w][k][L] * dt;
+                    x1 = add(x1, mul(v1, tt));
+                    x2 = add(x2, mul(v2, tt));
+                    x3 = add(x3, mul(v3, tt));
+                    x4 = add(x4, mul(v4, tt));
+                }
+                const bool r = test_vf(x4, x1, x2, x3, h, wt);
+                wt.t = tt;  // the contact's time (Collision/CudaPrimitiveTests.cu:174, 228)
+                return r;
+            };
+            for (uint32_t j0 = 0; j0 < ntests; j0 += 32) {
+                const uint32_t j = j0 + lane;
+                int L = 0;  // owner: the last lane whose first test is <= j
+#pragma unroll
+                for (int step = 16; step > 0; step >>= 1) {
+                    const int cand = L + step;
+                    const uint32_t e = __shfl_sync(full, ex, cand & 31);
+                    if (cand < 32 && e <= j) L = cand;
+                }
+                const uint32_t exL = __shfl_sync(full, ex, L);
+                const float h = __shfl_sync(full, hq, L), dt = __shfl_sync(full, dtq, L);
+                if (j < ntests) {
+                    const int m = (int)(j - exL);
+                    Wts wt;
+                    if (run_test(L, m, h, dt, wt)) atomicMin(&best[w][L], m);
                 }
             }
+            __syncwarp();
+            bool found = false;
+            Wts wt;
+            if (valid && best[w][lane] < 6) found = run_test(lane, best[w][lane], hq, dtq, wt);
+            if (found) record_hit<VF>(d, q, wt);
+            const unsigned hb = __ballot_sync(full, found);
+            if (lane == 0) {
+                hmask[base / 32] = hb;
+                hcnt[base / 32] = (uint32_t)__popc(hb);
+            }
+            __syncwarp();
+            continue;
         }
-        const unsigned hb = __ballot_sync(full, found);
-        if (lane == 0) {
-            hmask[base / 32] = hb;
-            hcnt[base / 32] = (uint32_t)__popc(hb);
+        // EE: the few candidates whose edges are not apart throughout their
+        // times' advances go on to the tests, 32 of them at a time.
+        bool is_near = false;
+        if (valid && times) {
+            const float h = d.cloth[cloth_of[w][lane]].h, dt = d.cloth[cloth_of[w][lane]].dt;
+            float T = 0.f, lo = 3.4e38f, hi = -3.4e38f;
+            for (unsigned m = times; m; m &= m - 1u) {
+                T += tq[w][__ffs(m) - 1][lane] * dt;
+                lo = fminf(lo, T);
+                hi = fmaxf(hi, T);
+            }
+            float3 x1, x2, x3, x4, v1, v2, v3, v4;
+            corners(lane, x1, x2, x3, x4, v1, v2, v3, v4);
+            is_near = !(T == T && ee_apart(x1, x2, x3, x4, v1, v2, v3, v4, lo, hi, h));  // (NaN times: T is NaN)
         }
+        const unsigned nb = __ballot_sync(full, is_near);
+        if (is_near) {
+            const int at = nnear + __popc(nb & ((1u << lane) - 1u));
+            near_q[w][at] = q;
+            near_n[w][at] = (uint8_t)__popc(times);
+            int k = 0;
+            for (unsigned m = times; m; m &= m - 1u) near_t[w][k++][at] = tq[w][__ffs(m) - 1][lane];
+        }
+        nnear += __popc(nb);
+        if (lane == 0) hmask[base / 32] = hcnt[base / 32] = 0u;
         __syncwarp();
+        if (nnear >= 32) {
+            nnear -= 32;
+            const int at = nnear + lane;
+            test_near(d, near_q[w][at], near_n[w][at], &near_t[w][0][at]);
+            __syncwarp();
+        }
     }
+    if (!VF && lane < nnear)
+        test_near(d, near_q[w][lane], near_n[w][lane], &near_t[w][0][lane]);
 }
+
 
 // The discrete tests (CudaPrimitiveTests::DCDTriangleTests,
 // Collision/CudaPrimitiveTests.cu:21-94): one TestVF / TestEE of every
