@@ -46,7 +46,8 @@ void launch_adj_rescale(const DevPtrs &d, float *gx, float *gxp, float *gv, floa
 void launch_adjoint(const DevPtrs &d, const AdjPtrs &A, float4 *a, float4 *g, const uint32_t *nvf, const uint32_t *nee,
                     int grid, int nfixed, float *gk_stretch, float *gk_bend, cudaStream_t st);
 void launch_vertex_normals(const DevPtrs &d, cudaStream_t st);
-void launch_dyn(const DevPtrs &d, const uint32_t *nvf, const uint32_t *nee, int grid, int phase, cudaStream_t st);
+void launch_dyn(const DevPtrs &d, const uint32_t *nvf, const uint32_t *nee, int grid, int phase, bool sorted,
+                cudaStream_t st);
 void launch_solver_setup(const DevPtrs &d, bool sphere, cudaStream_t st);
 bool tiles_supported();
 void launch_jacobi(const DevPtrs &d, const float4 *xa, float4 *xb, int it, const uint32_t *nvf, int block,
@@ -445,8 +446,7 @@ static lc_status enqueue_cluster_solver(lc_batch *b, cudaStream_t st);
 lc_status lc_batch::enqueue_step(cudaStream_t st) {
     const bool dbg = opt.debug_capture != 0;
     LC_PHASE(0);
-    LC_CUDA(cudaMemsetAsync(d.counters, 0, sizeof(unsigned long long) * 4, st));
-    // 1. PBD External
+    // 1. PBD External (and the step's counters cleared)
     if (any_wind) launch_wind(d, st);
     launch_external(d, st, recording ? tape_xin : nullptr, recording ? tape_vb : nullptr);
     if (dbg) {
@@ -490,8 +490,7 @@ lc_status lc_batch::enqueue_step(cudaStream_t st) {
     const uint32_t hcap = (uint32_t)(d.cand_cap / 32 + 1);
     const ScanJob hits_ee{d.hitg_cnt[1], d.hitg_off[1], d.hitg_n + 1, 0, hcap, nee, &d.counters[2]};
     scan_u32({d.hitg_cnt[0], d.hitg_off[0], d.hitg_n, 0, hcap, nvf, &d.counters[1]}, &hits_ee, d.scan_tmp, d.err, st);
-    launch_narrow(d, npairs, ncand, ncand_e, narrow_grid, 3, st);  // write contacts
-    launch_narrow(d, npairs, ncand, ncand_e, narrow_grid, 4, st);  // per-cloth ranges
+    launch_narrow(d, npairs, ncand, ncand_e, narrow_grid, 4, st);  // write contacts and per-cloth ranges
     launch_collider(d, narrow_grid, st);                            // static colliders (lc_batch_set_collider)
     LC_PHASE(5);
     // 6. PBD Solver (+ 7. integration fused on the cluster path).  The
@@ -503,12 +502,12 @@ lc_status lc_batch::enqueue_step(cudaStream_t st) {
     const bool on_chip = use_cluster;
     const bool ordered = !(on_chip && cluster_scatter) || d.friction_any;  // float sums in entry order
     if (ordered || recording || (on_chip && cluster_scatter && ca.contact_gather)) {
-        LC_CUDA(cudaMemsetAsync(d.dyn_cnt, 0, sizeof(uint32_t) * (size_t)d.Vtot, st));
-        LC_CUDA(cudaMemsetAsync(d.dyn_cur, 0, sizeof(uint32_t) * (size_t)d.Vtot, st));
-        launch_dyn(d, nvf, nee, narrow_grid, 0, st);
+        LC_CUDA(cudaMemsetAsync(d.dyn_cnt, 0, 2 * sizeof(uint32_t) * (size_t)d.Vtot, st));  // dyn_cur too
+        const bool sorted = ordered || recording;
+        launch_dyn(d, nvf, nee, narrow_grid, 0, sorted, st);
         scan_u32({d.dyn_cnt, d.dyn_off, nullptr, V, V, nullptr, nullptr}, nullptr, d.scan_tmp, d.err, st);
-        launch_dyn(d, nvf, nee, narrow_grid, 1, st);
-        if (ordered || recording) launch_dyn(d, nvf, nee, narrow_grid, 2, st);
+        launch_dyn(d, nvf, nee, narrow_grid, 1, sorted, st);
+        if (sorted) launch_dyn(d, nvf, nee, narrow_grid, 2, sorted, st);
     }
     if (on_chip) {
         LC_KEV(0);
@@ -1005,8 +1004,9 @@ static lc_status batch_build(lc_batch *b, const lc_cloth_desc *descs, int n, con
         LC_TRY(A.alloc(d.vf_n, vf_cap, "vf_n"));
         LC_TRY(A.alloc(d.hit_nrm, vf_cap, "hit_nrm_vf"));
     }
-    LC_TRY(A.alloc(d.dyn_cnt, V, "dyn_cnt")); LC_TRY(A.alloc(d.dyn_off, V + 1, "dyn_off"));
-    LC_TRY(A.alloc(d.dyn_cur, V, "dyn_cur")); LC_TRY(A.alloc(d.dyn_ent, d.dyn_cap, "dyn_ent"));
+    LC_TRY(A.alloc(d.dyn_cnt, 2 * V, "dyn_cnt")); LC_TRY(A.alloc(d.dyn_off, V + 1, "dyn_off"));
+    d.dyn_cur = d.dyn_cnt + V;
+    LC_TRY(A.alloc(d.dyn_ent, d.dyn_cap, "dyn_ent"));
     int *soff; uint32_t *sent; int2 *sids; float2 *spar; int4 *bids; float *bkp;
     LC_TRY(A.alloc(soff, V + 1, "soff")); LC_TRY(A.alloc(sent, S, "sent"));
     LC_TRY(A.alloc(sids, E, "s_ids")); LC_TRY(A.alloc(spar, E, "s_par"));
@@ -1031,6 +1031,9 @@ static lc_status batch_build(lc_batch *b, const lc_cloth_desc *descs, int n, con
     LC_TRY(A.alloc(vbf, vb_first.size(), "vb_first"));
     d.vblk_cloth = vbc; d.vblk_start = vbs; d.vb_first = vbf;
     LC_TRY(A.alloc(d.damp_part, 16 * vblk_cloth.size(), "damp_part"));
+    LC_TRY(A.alloc(d.damp_f, 12 * (size_t)n, "damp_f"));
+    LC_TRY(A.alloc(d.damp_done, n, "damp_done"));
+    LC_CUDA(cudaMemset(d.damp_done, 0, sizeof(unsigned) * (size_t)n));
     LC_TRY(A.alloc(d.vbox, 2 * std::max<int64_t>(V, 1), "vertex swept boxes"));
     LC_TRY(A.alloc(b->npairs, 1, "npairs")); LC_TRY(A.alloc(b->nvf, 1, "nvf")); LC_TRY(A.alloc(b->nee, 1, "nee"));
     LC_TRY(A.alloc(b->ncand, 1, "ncand")); LC_TRY(A.alloc(b->ncand_e, 1, "ncand_e"));

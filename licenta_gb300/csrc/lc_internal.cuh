@@ -221,6 +221,8 @@ struct DevPtrs {
     const int *vblk_cloth, *vblk_start;  // vertex blocks never straddle cloths
     const int *vb_first;                 // per cloth: first vertex block (C+1 entries)
     double *damp_part;                   // 16 partial sums per vertex block
+    float *damp_f;                       // 12 per cloth: angular velocity, mass centre, its velocity
+    unsigned *damp_done;                 // per cloth: its blocks that have written theirs
     int nvblk;
     // discrete decisions of the last step, recorded only for parity checks
     uint32_t *dbg_ground_it;  // per vertex: bit it = ground term counted in iteration it

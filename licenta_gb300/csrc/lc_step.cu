@@ -53,31 +53,52 @@ __device__ __forceinline__ void block_partials(float (&v)[N], double *dst) {
     }
 }
 
-// Cloth totals of the block partials [k0, k0+N), one block per cloth, summed
-// in a fixed order (deterministic) into d.damp[c*16 + k].
-__global__ void k_cloth_totals(DevPtrs d, int k0, int N) {
-    const int c = blockIdx.x;
+// Cloth totals of the block partials [K0, K0 + N) of cloth c, summed by the last
+// of its blocks to arrive, in a fixed order (deterministic), into
+// d.damp[c * 16 + k].  In a launch of its own this took 4 us of every step,
+// twice.  done: the cloth's counter, left at zero.
+// Returns whether this block was the last.
+template <int K0, int N>
+__device__ __forceinline__ bool cloth_totals(const DevPtrs &d, int c, unsigned *done) {
+    __shared__ bool last;
     const int b0 = d.vb_first[c], b1 = d.vb_first[c + 1];
-    __shared__ double red[16][kThreads / 32];
+    __threadfence();
+    __syncthreads();
+    if (threadIdx.x == 0) last = atomicAdd(done, 1u) + 1u == (unsigned)(b1 - b0);
+    __syncthreads();
+    if (!last) return false;
+    __threadfence();
+    __shared__ double red[N][kThreads / 32];
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-    for (int k = 0; k < N; ++k) {
-        double s = 0;
-        for (int b = b0 + threadIdx.x; b < b1; b += blockDim.x) s += d.damp_part[(size_t)b * 16 + k0 + k];
+    double s[N];
 #pragma unroll
-        for (int o = 16; o > 0; o >>= 1) s += __shfl_down_sync(0xffffffffu, s, o);
-        if (lane == 0) red[k][wid] = s;
+    for (int k = 0; k < N; ++k) s[k] = 0;
+    for (int b = b0 + threadIdx.x; b < b1; b += blockDim.x) {
+#pragma unroll
+        for (int k = 0; k < N; ++k) s[k] += __ldcg(&d.damp_part[(size_t)b * 16 + K0 + k]);
+    }
+#pragma unroll
+    for (int k = 0; k < N; ++k) {
+        double t = s[k];
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) t += __shfl_down_sync(0xffffffffu, t, o);
+        if (lane == 0) red[k][wid] = t;
     }
     __syncthreads();
     if (threadIdx.x < N) {
         double t = 0;
         for (int w = 0; w < (int)(blockDim.x / 32); ++w) t += red[threadIdx.x][w];
-        d.damp[(size_t)c * 16 + k0 + threadIdx.x] = t;
+        d.damp[(size_t)c * 16 + K0 + threadIdx.x] = t;
     }
+    if (threadIdx.x == 0) *done = 0u;
+    __syncthreads();
+    return true;
 }
 
 // ApplyExternalForces (Physics/CudaPBD.cu:1992-2003), GlobalVelDamp (:1934-1941)
 // and the mass / first-moment sums of DampVelocities (:419-435).
-__global__ void k_external(DevPtrs d) {
+__global__ void __launch_bounds__(kThreads) k_external(DevPtrs d) {
+    if (blockIdx.x == 0 && threadIdx.x < 4) d.counters[threadIdx.x] = 0;
     const int c = d.vblk_cloth[blockIdx.x];
     const ClothDev &cd = d.cloth[c];
     const int i = d.vblk_start[blockIdx.x] + threadIdx.x;
@@ -104,20 +125,22 @@ __global__ void k_external(DevPtrs d) {
         s[4] = vel.x * m; s[5] = vel.y * m; s[6] = vel.z * m;
     }
     block_partials<7>(s, d.damp_part + (size_t)blockIdx.x * 16);
+    // mass centre and its velocity, once per cloth and a thread per quotient: FP64
+    // division is slow on this part
+    if (cloth_totals<0, 7>(d, c, d.damp_done + c) && threadIdx.x < 6) {
+        const double *t = d.damp + (size_t)c * 16;
+        d.damp_f[(size_t)c * 12 + 3 + threadIdx.x] = (float)(t[1 + threadIdx.x] / t[0]);
+    }
 }
 
 // ComputeL / ComputeIs (Physics/CudaPBD.cu:1955-1976): angular momentum and
 // inertia about the mass centre.
-__global__ void k_damp_moments(DevPtrs d) {
+__global__ void __launch_bounds__(kThreads) k_damp_moments(DevPtrs d) {
     const int c = d.vblk_cloth[blockIdx.x];
     const ClothDev &cd = d.cloth[c];
-    const double *t = d.damp + (size_t)c * 16;
     const int i = d.vblk_start[blockIdx.x] + threadIdx.x;
     const bool valid = i < cd.v_off + cd.V;
-    // the mass centre once per block: FP64 division is slow on this part
-    __shared__ float cm[3];
-    if (threadIdx.x < 3) cm[threadIdx.x] = (float)(t[1 + threadIdx.x] / t[0]);
-    __syncthreads();
+    const float *cm = d.damp_f + (size_t)c * 12 + 3;
     float s[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0};
     if (valid) {
         const float3 xcm = f3(cm[0], cm[1], cm[2]);
@@ -129,17 +152,10 @@ __global__ void k_damp_moments(DevPtrs d) {
         s[6] = -(r.x * r.y) * m; s[7] = -(r.x * r.z) * m; s[8] = -(r.y * r.z) * m;
     }
     block_partials<9>(s, d.damp_part + (size_t)blockIdx.x * 16 + 7);
-}
-
-// omega = I^-1 L (the host glm::inverse of Physics/CudaPBD.cu:447-454, here in
-// double on the device), UpdateVels (:1978-1990) and ExplicitEuler (:2005-2012).
-__global__ void k_damp_apply(DevPtrs d) {
-    const int c = d.vblk_cloth[blockIdx.x];
-    const ClothDev &cd = d.cloth[c];
-    const double *a = d.damp + (size_t)c * 16;
-    __shared__ float sh[9];
-    if (threadIdx.x == 0) {
-        const double ms = a[0];
+    // omega = I^-1 L (the host glm::inverse of Physics/CudaPBD.cu:447-454, here in
+    // double on the device)
+    if (cloth_totals<7, 9>(d, c, d.damp_done + c) && threadIdx.x < 3) {
+        const double *a = d.damp + (size_t)c * 16;
         const double L0 = a[7], L1 = a[8], L2 = a[9];
         const double i1x = a[10], i1y = a[11], i1z = a[12], i2x = a[13], i2y = a[14], i2z = a[15];
         const double A = i1y + i1z, B = i2x, C = i2y, D = i1x + i1z, E = i2z, F = i1x + i1y;
@@ -147,13 +163,18 @@ __global__ void k_damp_apply(DevPtrs d) {
         const double c00 = D * F - E * E, c01 = -(B * F - E * C), c02 = B * E - D * C;
         const double c11 = A * F - C * C, c12 = -(A * E - B * C), c22 = A * D - B * B;
         const double det = A * c00 + B * c01 + C * c02;
-        sh[0] = (float)((c00 * L0 + c01 * L1 + c02 * L2) / det);
-        sh[1] = (float)((c01 * L0 + c11 * L1 + c12 * L2) / det);
-        sh[2] = (float)((c02 * L0 + c12 * L1 + c22 * L2) / det);
-        sh[3] = (float)(a[1] / ms); sh[4] = (float)(a[2] / ms); sh[5] = (float)(a[3] / ms);
-        sh[6] = (float)(a[4] / ms); sh[7] = (float)(a[5] / ms); sh[8] = (float)(a[6] / ms);
+        const double r0 = threadIdx.x == 0 ? c00 : threadIdx.x == 1 ? c01 : c02;
+        const double r1 = threadIdx.x == 0 ? c01 : threadIdx.x == 1 ? c11 : c12;
+        const double r2 = threadIdx.x == 0 ? c02 : threadIdx.x == 1 ? c12 : c22;
+        d.damp_f[(size_t)c * 12 + threadIdx.x] = (float)((r0 * L0 + r1 * L1 + r2 * L2) / det);
     }
-    __syncthreads();
+}
+
+// UpdateVels (:1978-1990) and ExplicitEuler (:2005-2012).
+__global__ void k_damp_apply(DevPtrs d) {
+    const int c = d.vblk_cloth[blockIdx.x];
+    const ClothDev &cd = d.cloth[c];
+    const float *sh = d.damp_f + (size_t)c * 12;
     const int i = d.vblk_start[blockIdx.x] + threadIdx.x;
     if (i >= cd.v_off + cd.V) return;
     const float3 omega = f3(sh[0], sh[1], sh[2]);
@@ -215,7 +236,13 @@ __global__ void k_dyn_count(DevPtrs d, const uint32_t *nvf_dev, const uint32_t *
     }
 }
 
-__global__ void k_dyn_fill(DevPtrs d, const uint32_t *nvf_dev, const uint32_t *nee_dev) {
+// Entry k of the unsorted lists: in the hits' weights, dead by now, 16 bytes
+// per contact as the lists take.
+__device__ __forceinline__ uint32_t *dyn_unsorted(const DevPtrs &d, uint32_t k) {
+    const uint64_t first = 4 * d.vf_cap;
+    return k < first ? reinterpret_cast<uint32_t *>(d.hit_w[0]) + k : reinterpret_cast<uint32_t *>(d.hit_w[1]) + (k - first);
+}
+__global__ void k_dyn_fill(DevPtrs d, const uint32_t *nvf_dev, const uint32_t *nee_dev, bool sorted) {
     uint32_t nvf, nee;
     contact_counts(d, nvf_dev, nee_dev, nvf, nee);
     const uint32_t n = nvf + nee;
@@ -225,23 +252,26 @@ __global__ void k_dyn_fill(DevPtrs d, const uint32_t *nvf_dev, const uint32_t *n
 #pragma unroll
         for (int s = 0; s < 4; ++s) {
             const uint32_t pos = d.dyn_off[vs[s]] + atomicAdd(&d.dyn_cur[vs[s]], 1u);
-            d.dyn_ent[pos] = c * 4u + (uint32_t)s;
+            *(sorted ? dyn_unsorted(d, pos) : d.dyn_ent + pos) = c * 4u + (uint32_t)s;
         }
     }
 }
 
-__global__ void k_dyn_sort(DevPtrs d) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= d.Vtot) return;
-    const uint32_t a = d.dyn_off[i], b = d.dyn_off[i + 1];
-    for (uint32_t k = a + 1; k < b; ++k) {
-        const uint32_t key = d.dyn_ent[k];
-        uint32_t j = k;
-        while (j > a && d.dyn_ent[j - 1] > key) {
-            d.dyn_ent[j] = d.dyn_ent[j - 1];
-            --j;
-        }
-        d.dyn_ent[j] = key;
+// Every entry to its rank in its vertex's list, a thread per contact.  (A thread
+// per vertex sorting by insertion waited for its longest list: 34 us for one folded
+// cloth of 101 squared, 5.5 so; 152 and 10 for 24 draped ones.)
+__global__ void k_dyn_sort(DevPtrs d, const uint32_t *nvf_dev, const uint32_t *nee_dev) {
+    uint32_t nvf, nee;
+    contact_counts(d, nvf_dev, nee_dev, nvf, nee);
+    const uint32_t n = 4u * (nvf + nee);
+    for (uint32_t e = blockIdx.x * blockDim.x + threadIdx.x; e < n; e += gridDim.x * blockDim.x) {
+        const uint32_t c = e >> 2;
+        const int4 *v4 = c < nvf ? &d.vf_v[c] : &d.ee_v[c - nvf];
+        const int v = reinterpret_cast<const int *>(v4)[e & 3u];
+        const uint32_t a = d.dyn_off[v], b = d.dyn_off[v + 1];
+        uint32_t r = a;
+        for (uint32_t k = a; k < b; ++k) r += *dyn_unsorted(d, k) < e;
+        d.dyn_ent[r] = e;
     }
 }
 
@@ -585,9 +615,7 @@ void launch_wind(const DevPtrs &d, cudaStream_t st) { k_wind<<<nblk(d.C, 128), 1
 void launch_external(const DevPtrs &d, cudaStream_t st, float4 *save_x, float4 *save_v) {
     if (d.nvblk) {
         k_external<<<d.nvblk, kThreads, 0, st>>>(d);
-        k_cloth_totals<<<d.C, kThreads, 0, st>>>(d, 0, 7);
         k_damp_moments<<<d.nvblk, kThreads, 0, st>>>(d);
-        k_cloth_totals<<<d.C, kThreads, 0, st>>>(d, 7, 9);
         if (save_x) cudaMemcpyAsync(save_x, d.x, sizeof(float4) * (size_t)d.Vtot, cudaMemcpyDeviceToDevice, st);
         if (save_v) cudaMemcpyAsync(save_v, d.v, sizeof(float4) * (size_t)d.Vtot, cudaMemcpyDeviceToDevice, st);
         k_damp_apply<<<d.nvblk, kThreads, 0, st>>>(d);
@@ -596,10 +624,11 @@ void launch_external(const DevPtrs &d, cudaStream_t st, float4 *save_x, float4 *
 void launch_vertex_normals(const DevPtrs &d, cudaStream_t st) {
     if (d.Vtot) k_vertex_normals<<<nblk(d.Vtot), kThreads, 0, st>>>(d);
 }
-void launch_dyn(const DevPtrs &d, const uint32_t *nvf, const uint32_t *nee, int grid, int phase, cudaStream_t st) {
+void launch_dyn(const DevPtrs &d, const uint32_t *nvf, const uint32_t *nee, int grid, int phase, bool sorted,
+                cudaStream_t st) {
     if (phase == 0) k_dyn_count<<<grid, kThreads, 0, st>>>(d, nvf, nee);
-    else if (phase == 1) k_dyn_fill<<<grid, kThreads, 0, st>>>(d, nvf, nee);
-    else if (d.Vtot) k_dyn_sort<<<nblk(d.Vtot), kThreads, 0, st>>>(d);
+    else if (phase == 1) k_dyn_fill<<<grid, kThreads, 0, st>>>(d, nvf, nee, sorted);
+    else k_dyn_sort<<<grid, kThreads, 0, st>>>(d, nvf, nee);
 }
 void launch_solver_setup(const DevPtrs &d, bool sphere, cudaStream_t st) {
     if (!d.Vtot) return;
