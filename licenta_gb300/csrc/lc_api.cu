@@ -482,11 +482,15 @@ lc_status lc_batch::enqueue_step(cudaStream_t st) {
     const ScanJob groups_ee{d.grp_ee_cnt, d.grp_ee_off, d.ngroups, 0, gcap, ncand_e, nullptr};
     scan_u32({d.grp_vf_cnt, d.grp_vf_off, d.ngroups, 0, gcap, ncand, nullptr}, &groups_ee, d.scan_tmp, d.err, st);
     launch_narrow(d, npairs, ncand, ncand_e, narrow_grid, 1, st);  // expand
-    LC_KEV(8);
-    launch_narrow(d, npairs, ncand, ncand_e, narrow_grid, 2, st);  // VF CCD
-    LC_KEV(9);
-    launch_narrow(d, npairs, ncand, ncand_e, narrow_grid, 5, st);  // EE CCD
-    LC_KEV(10);
+    if (kern_ev || d.Ttot > kBothCcdLeaves) {  // (profiles time them one by one)
+        LC_KEV(8);
+        launch_narrow(d, npairs, ncand, ncand_e, narrow_grid, 2, st);  // VF CCD
+        LC_KEV(9);
+        launch_narrow(d, npairs, ncand, ncand_e, narrow_grid, 5, st);  // EE CCD
+        LC_KEV(10);
+    } else {
+        launch_narrow(d, npairs, ncand, ncand_e, narrow_grid, 9, st);  // VF and EE CCD
+    }
     const uint32_t hcap = (uint32_t)(d.cand_cap / 32 + 1);
     const ScanJob hits_ee{d.hitg_cnt[1], d.hitg_off[1], d.hitg_n + 1, 0, hcap, nee, &d.counters[2]};
     scan_u32({d.hitg_cnt[0], d.hitg_off[0], d.hitg_n, 0, hcap, nvf, &d.counters[1]}, &hits_ee, d.scan_tmp, d.err, st);

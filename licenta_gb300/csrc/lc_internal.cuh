@@ -18,6 +18,8 @@ constexpr int kSortTile = 2048;          // keys per sort tile (256 threads x 8)
 constexpr int kSortPassesMax = 8;        // 8-bit digits of a 63-bit key
 constexpr int kRangePad = 32;            // range-tree entries of a cloth of T leaves: at most T + kRangePad
 constexpr int kTraverseStack = 64;       // Collision/CudaBVH.cu:38
+constexpr int kBothCcdLeaves = 48 << 10;    // leaves up to which the VF and the EE CCD share a launch
+constexpr uint64_t kBothCcdPairs = 10ull * kBothCcdLeaves;  // the same for the narrowphase entry (ten pairs a leaf)
 constexpr int kPacketLeaves = 1 << 20;   // leaves above which a batch's traversal walks 32 of them together
 constexpr int kTraverseBlockMax = 256;   // largest traversal block (the packet kernel is bounded for 6 of them per SM)
 constexpr uint32_t kScanBlocks = 304;    // largest grid of the device-count scans

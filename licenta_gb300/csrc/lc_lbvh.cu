@@ -1957,35 +1957,47 @@ __device__ __noinline__ void test_near(const DevPtrs &d, uint32_t q, int nt, con
     }
 }
 
-// At most 64 registers, for 4 resident blocks per SM instead of 3: EE 134 us
-// against 150.
 template <bool VF>
-__global__ void __launch_bounds__(kCcdWarps * 32, 4) k_ccd_warp(const __grid_constant__ DevPtrs d,
-                                                                const uint32_t *__restrict__ ncand) {
-    __shared__ float4 geom[kCcdWarps][6][32];     // x1..x4 then v1..v4 (test order) per lane
-    __shared__ float fval[kCcdWarps][4][32];      // f at the interval ends
-    __shared__ float ends[kCcdWarps][2][32];      // the inner ends
-    __shared__ uint8_t job_owner[kCcdWarps][96];  // queued secant solves: lane << 2 | interval
+struct CcdShared {
+    float4 geom[kCcdWarps][6][32];     // x1..x4 then v1..v4 (test order) per lane
+    float fval[kCcdWarps][4][32];      // f at the interval ends
+    float ends[kCcdWarps][2][32];      // the inner ends
     // each lane's times to test, in the reference's order: interval i's start
     // (if f is 0 there) at 2 i, its root at 2 i + 1
-    __shared__ float tq[kCcdWarps][6][32];
-    __shared__ int cloth_of[kCcdWarps][32];
-    __shared__ int best[VF ? kCcdWarps : 1][32];     // VF: each lane's first hitting test (6: none)
+    float tq[kCcdWarps][6][32];
+    int cloth_of[kCcdWarps][32];
+    int best[VF ? kCcdWarps : 1][32];  // VF: each lane's first hitting test (6: none)
     // EE: candidates not apart, until 32 are together
-    __shared__ uint32_t near_q[VF ? 1 : kCcdWarps][kNearCap];
-    __shared__ uint8_t near_n[VF ? 1 : kCcdWarps][kNearCap];
-    __shared__ float near_t[VF ? 1 : kCcdWarps][6][kNearCap];
+    uint32_t near_q[VF ? 1 : kCcdWarps][kNearCap];
+    float near_t[VF ? 1 : kCcdWarps][6][kNearCap];
+    uint8_t near_n[VF ? 1 : kCcdWarps][kNearCap];
+    uint8_t job_owner[kCcdWarps][96];  // queued secant solves: lane << 2 | interval
+};
+// Block `block` of nblocks.
+template <bool VF>
+__device__ __forceinline__ void ccd_run(const DevPtrs &d, const uint32_t *__restrict__ ncand, CcdShared<VF> &sh,
+                                        uint32_t block, uint32_t nblocks) {
+    auto &geom = sh.geom;
+    auto &fval = sh.fval;
+    auto &ends = sh.ends;
+    auto &tq = sh.tq;
+    auto &cloth_of = sh.cloth_of;
+    auto &best = sh.best;
+    auto &near_q = sh.near_q;
+    auto &near_t = sh.near_t;
+    auto &near_n = sh.near_n;
+    auto &job_owner = sh.job_owner;
     int nnear = 0;
     const uint32_t n = (uint32_t)min((uint64_t)*ncand, d.cand_cap);
     const int4 *list = VF ? d.cand : d.cand_e;
     // hit bits per group of 32 candidates (one warp iteration: base is a
     // multiple of 32); the scan of their counts orders the contacts
     uint32_t *hmask = d.hitg_mask[VF ? 0 : 1], *hcnt = d.hitg_cnt[VF ? 0 : 1];
-    if (blockIdx.x == 0 && threadIdx.x == 0) d.hitg_n[VF ? 0 : 1] = (n + 31) / 32;
+    if (block == 0 && threadIdx.x == 0) d.hitg_n[VF ? 0 : 1] = (n + 31) / 32;
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     const unsigned full = 0xffffffffu;
-    const uint32_t nwarps = gridDim.x * kCcdWarps;
-    for (uint32_t base = (blockIdx.x * kCcdWarps + w) * 32u; base < n; base += nwarps * 32u) {
+    const uint32_t nwarps = nblocks * kCcdWarps;
+    for (uint32_t base = (block * kCcdWarps + w) * 32u; base < n; base += nwarps * 32u) {
         const uint32_t q = base + lane;
         const bool valid = q < n;
         int4 ids = make_int4(0, 0, 0, 0);
@@ -2189,6 +2201,31 @@ __global__ void __launch_bounds__(kCcdWarps * 32, 4) k_ccd_warp(const __grid_con
         test_near(d, near_q[w][lane], near_n[w][lane], &near_t[w][0][lane]);
 }
 
+// One kind, or both in one launch (the first half of the blocks takes the EE
+// candidates): the two wait for nothing of each other, and in a small step
+// each leaves most of the chip idle; in a large one the two codes evict each
+// other from the instruction cache.  Us per step, one by one / both, folded
+// cloths of 16, 32, 64, 101, 140 and 192 squared: 183, 238, 311, 455, 853, 955 /
+// 176, 230, 306, 449, 850, 971; 24 cloths up to 128 squared 1255 / 1271.
+// At most 64 registers, for 4 resident blocks per SM instead of 3: EE 134 us
+// against 150.
+template <bool VF>
+__global__ void __launch_bounds__(kCcdWarps * 32, 4) k_ccd_warp(const __grid_constant__ DevPtrs d,
+                                                                const uint32_t *__restrict__ ncand) {
+    __shared__ CcdShared<VF> sh;
+    ccd_run<VF>(d, ncand, sh, blockIdx.x, gridDim.x);
+}
+__global__ void __launch_bounds__(kCcdWarps * 32, 4) k_ccd_both(const __grid_constant__ DevPtrs d,
+                                                                const uint32_t *__restrict__ ncv,
+                                                                const uint32_t *__restrict__ nce) {
+    __shared__ union {
+        CcdShared<true> vf;
+        CcdShared<false> ee;
+    } sh;
+    const uint32_t half = gridDim.x / 2;
+    if (blockIdx.x < half) ccd_run<false>(d, nce, sh.ee, blockIdx.x, half);
+    else ccd_run<true>(d, ncv, sh.vf, blockIdx.x - half, half);
+}
 
 // The discrete tests (CudaPrimitiveTests::DCDTriangleTests,
 // Collision/CudaPrimitiveTests.cu:21-94): one TestVF / TestEE of every
@@ -2577,6 +2614,8 @@ void launch_narrow(const DevPtrs &d, const uint32_t *npairs, const uint32_t *ncv
     else if (stage == 1) k_narrow_expand<<<grid, kThreads, 0, st>>>(d, npairs);
     else if (stage == 2) {
         k_ccd_warp<true><<<grid, kCcdWarps * 32, 0, st>>>(d, ncv);
+    } else if (stage == 9) {
+        k_ccd_both<<<2 * grid, kCcdWarps * 32, 0, st>>>(d, ncv, nce);
     } else if (stage == 5) {
         k_ccd_warp<false><<<grid, kCcdWarps * 32, 0, st>>>(d, nce);
     } else if (stage == 3) {

@@ -234,8 +234,12 @@ lc_status lc_narrowphase_run(lc_narrowphase *h, int32_t mode, const float *x, co
     launch_narrow(d, h->npairs, h->ncand, h->ncand_e, h->grid, 1, st);
     // Collision/CudaPrimitiveTests.cu:96-238: CCD on x_prev and v; or :21-94,
     // the discrete tests at x_prev
-    launch_narrow(d, h->npairs, h->ncand, h->ncand_e, h->grid, ccd ? 2 : 7, st);
-    launch_narrow(d, h->npairs, h->ncand, h->ncand_e, h->grid, ccd ? 5 : 8, st);
+    if (ccd && num_pairs <= kBothCcdPairs) {
+        launch_narrow(d, h->npairs, h->ncand, h->ncand_e, h->grid, 9, st);
+    } else {
+        launch_narrow(d, h->npairs, h->ncand, h->ncand_e, h->grid, ccd ? 2 : 7, st);
+        launch_narrow(d, h->npairs, h->ncand, h->ncand_e, h->grid, ccd ? 5 : 8, st);
+    }
     const uint32_t hcap = (uint32_t)(d.cand_cap / 32 + 1);
     const ScanJob hits_ee{d.hitg_cnt[1], d.hitg_off[1], d.hitg_n + 1, 0, hcap, h->nee, nullptr};
     scan_u32({d.hitg_cnt[0], d.hitg_off[0], d.hitg_n, 0, hcap, h->nvf, nullptr}, &hits_ee, d.scan_tmp, d.err, st);

@@ -63,3 +63,37 @@ def test_contacts_equal_the_oracle(cuda, pairs, kind, edge, offset, thick, speed
         g, r = got[:cnt].cpu().numpy(), np.ascontiguousarray(ref).view(np.int32).reshape(cnt, 12)
         both_nan = np.isnan(g.view(np.float32)) & np.isnan(r.view(np.float32))  # (a NaN's payload is the processor's)
         assert np.array_equal(g[~both_nan], r[~both_nan])
+
+
+def test_many_pairs_equal_the_same_pairs_few_at_a_time(cuda):
+    """More pairs than the rule gives one launch for both kinds: the contacts
+    of a repeated list are the list's, repeated."""
+    torch = cuda
+    from licenta_gb300 import Narrowphase
+    rng = np.random.default_rng(9)
+    pairs, reps = 700, 710
+    xp, v = _soup(rng, pairs, 0.02, 0.0, 0.5, "free")
+    dt, h = 1 / 64, 0.3 * 0.02
+    dev = lambda a: torch.from_numpy(np.ascontiguousarray(a)).cuda()
+    dx, dxp, dv = dev(xp + v * np.float32(dt)), dev(xp), dev(v)
+    dtr = dev(np.arange(6 * pairs, dtype=np.uint32).reshape(-1, 3))
+    df = dev(np.full(2 * pairs, 0x3F, np.uint8))
+    pr = np.arange(2 * pairs, dtype=np.uint32).reshape(-1, 2)
+
+    def run(p):
+        cap = 2 * len(p)
+        out = [torch.zeros((cap, 12), dtype=torch.int32, device="cuda") for _ in range(2)]
+        n = Narrowphase(len(xp), 2 * pairs, len(p), candidate_capacity=15 * len(p), contact_capacity=cap)
+        try:
+            dp = dev(p)
+            rc, nvf, nee = n.run(dx.data_ptr(), dxp.data_ptr(), dv.data_ptr(), len(xp), dtr.data_ptr(), df.data_ptr(),
+                                 2 * pairs, dp.data_ptr(), len(p), h, dt, out[0].data_ptr(), cap, out[1].data_ptr(), cap)
+        finally:
+            n.close()
+        assert rc == 0
+        return out[0][:nvf].cpu().numpy(), out[1][:nee].cpu().numpy()
+
+    few, many = run(pr), run(np.tile(pr, (reps, 1)))
+    for a, b in zip(few, many):
+        assert len(a) > 50
+        assert np.array_equal(np.tile(a, (reps, 1)), b)
