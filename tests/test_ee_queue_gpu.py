@@ -97,3 +97,38 @@ def test_many_pairs_equal_the_same_pairs_few_at_a_time(cuda):
     for a, b in zip(few, many):
         assert len(a) > 50
         assert np.array_equal(np.tile(a, (reps, 1)), b)
+
+
+@pytest.mark.parametrize("mode", [0, 1])
+@pytest.mark.parametrize("vertices,triangles", [(4, 6), (9, 40), (30, 33)])
+def test_ownership_and_shared_vertices(cuda, mode, vertices, triangles):
+    """Triangles with zero to three vertices in common, every ownership byte."""
+    torch = cuda
+    from licenta_gb300 import Narrowphase, _ffi
+    rng = np.random.default_rng([vertices, mode])
+    xp = rng.uniform(0, 0.05, (vertices, 3)).astype(np.float32)
+    v = rng.normal(0, 1, (vertices, 3)).astype(np.float32)
+    x = xp + v * np.float32(1 / 64)
+    tris = np.stack([rng.permutation(vertices)[:3] for _ in range(triangles)]).astype(np.uint32)
+    feats = rng.integers(0, 64, triangles).astype(np.uint8)
+    a, b = np.triu_indices(triangles, 1)
+    pr = np.stack([a, b], 1).astype(np.uint32)
+    h, dt = 0.01, 1 / 64
+    want = narrow_contacts(mode, x, xp, v, tris, feats, pr, h, dt)
+    dev = lambda q: torch.from_numpy(np.ascontiguousarray(q)).cuda()
+    dx, dxp, dv, dtr, df, dp = dev(x), dev(xp), dev(v), dev(tris), dev(feats), dev(pr)
+    cap = 15 * len(pr)
+    out = [torch.zeros((cap, 12), dtype=torch.int32, device="cuda") for _ in range(2)]
+    n = Narrowphase(vertices, triangles, len(pr), candidate_capacity=cap, contact_capacity=cap)
+    try:
+        rc, nvf, nee = n.run(dx.data_ptr(), dxp.data_ptr(), dv.data_ptr(), vertices, dtr.data_ptr(), df.data_ptr(),
+                             triangles, dp.data_ptr(), len(pr), h, dt, out[0].data_ptr(), cap, out[1].data_ptr(), cap,
+                             mode=_ffi.LC_NARROW_DCD if mode else _ffi.LC_NARROW_CCD)
+    finally:
+        n.close()
+    assert rc == 0 and (vertices == 4 or len(want[1]) > 0)  # (four vertices leave one disjoint edge per edge)
+    for got, cnt, ref in ((out[0], nvf, want[0]), (out[1], nee, want[1])):
+        assert cnt == len(ref)
+        g, r = got[:cnt].cpu().numpy(), np.ascontiguousarray(ref).view(np.int32).reshape(cnt, 12)
+        both_nan = np.isnan(g.view(np.float32)) & np.isnan(r.view(np.float32))
+        assert np.array_equal(g[~both_nan], r[~both_nan])
