@@ -1146,6 +1146,8 @@ static lc_status batch_build(lc_batch *b, const lc_cloth_desc *descs, int n, con
         LC_TRY(A.alloc(J.slot, std::max<int64_t>(S, 1), "adj_slot"));
         LC_TRY(A.alloc(J.dyn, std::max<uint64_t>(d.dyn_cap, 1), "adj_dyn"));
         LC_TRY(A.alloc(J.fixed, 3 * std::max<int64_t>(F, 1), "adj_fixed"));
+        LC_TRY(A.alloc(J.done, 1, "adj_done"));
+        LC_CUDA(cudaMemset(J.done, 0, sizeof(unsigned)));
         LC_CUDA(cudaMemset(J.fixed, 0, sizeof(float) * 3 * std::max<int64_t>(F, 1)));
         LC_TRY(A.alloc(J.red, 8 * (vblk_cloth.size() + (size_t)n), "adj_red"));
         LC_TRY(A.alloc(b->adj_flag, 2 * (size_t)n, "adj_flag"));

@@ -268,6 +268,7 @@ struct AdjPtrs {
     int nvblk_red;           // offset of the cloth totals in red
     int K;                   // solver iterations of the recorded step (max over cloths)
     int E, B;                // stretch / bend constraints of the batch
+    unsigned *done;        // blocks of a gather that have arrived
 };
 
 // ---------------------------------------------------------------------------
