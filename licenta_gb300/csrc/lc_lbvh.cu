@@ -1524,21 +1524,32 @@ __global__ void __launch_bounds__(kTraverseBlockMax, 6) k_traverse_packet(DevPtr
 }
 
 
-// Order-preserving compaction of the per-leaf chunks into the pair list, eight
-// lanes per leaf (a leaf of a cloth at rest has ten pairs): reads and writes
-// are runs, every lane's first copy waits for two loads only, and the writes are
-// the bound for a million leaves.  With a warp per 32 leaves, 18, 34 and 162 us for
-// 1922 and 20 k leaves at rest and a million in contact; 6, 7 and 162 so.
-constexpr int kCompactLanes = 8;
-__global__ void k_pair_compact(DevPtrs d) {
-    const int s = (int)((blockIdx.x * (unsigned)blockDim.x + threadIdx.x) / kCompactLanes);
-    if (s >= d.Ttot) return;
-    const uint32_t n = d.pair_cnt[s], lane = threadIdx.x & (kCompactLanes - 1);
-    if (lane >= n) return;
-    const uint32_t o = d.pair_off[s];
-    const ClothDev &cd = d.cloth[d.tcloth[s]];
-    const uint32_t *src = d.pair_chunk + cd.pc_off + (int64_t)(s - cd.t_off) * cd.chunk;
-    for (uint32_t k = lane; k < n; k += kCompactLanes) d.pairs[o + k] = make_uint2((uint32_t)s, (uint32_t)cd.t_off + src[k]);
+// Order-preserving compaction of the per-leaf chunks into the pair list: a
+// warp takes `per` leaves and copies those with pairs four at a time, eight lanes
+// each (a leaf of a cloth at rest has ten pairs).  Four leaves per warp while the
+// latency of one copy is what a launch takes, 32 when it is the number of
+// warps (us, 4 / 32: 1922 leaves 6 / 16, 20 k 7 / 22, 130 k 12 / 12, 522 k 35 / 24, a million of cloths in
+// contact 166 / 150, a million with a pair in 15 31 / 11; with lanes that look
+// up their leaf for every output 18, 33, -, 181, 11).
+constexpr int kCompactLanes = 8, kCompactManyLeaves = 1 << 17;
+__global__ void k_pair_compact(DevPtrs d, int per) {
+    const int lane = threadIdx.x & 31;
+    const int64_t base = (int64_t)((blockIdx.x * (unsigned)blockDim.x + threadIdx.x) >> 5) * per;
+    const uint32_t n = lane < per && base + lane < d.Ttot ? d.pair_cnt[base + lane] : 0u;
+    const unsigned some = __ballot_sync(0xffffffffu, n != 0u);
+    const int nsome = __popc(some), sub = lane / kCompactLanes;
+    for (int r = 0; r < nsome; r += 32 / kCompactLanes) {
+        const int pick = r + sub;
+        const int L = pick < nsome ? (int)__fns(some, 0, pick + 1) : 0;
+        const uint32_t nL = __shfl_sync(0xffffffffu, n, L);
+        if (pick >= nsome) continue;
+        const int leaf = (int)base + L;
+        const uint32_t o = d.pair_off[leaf];
+        const ClothDev &cd = d.cloth[d.tcloth[leaf]];
+        const uint32_t *src = d.pair_chunk + cd.pc_off + (int64_t)(leaf - cd.t_off) * cd.chunk;
+        for (uint32_t k = lane & (kCompactLanes - 1); k < nL; k += kCompactLanes)
+            d.pairs[o + k] = make_uint2((uint32_t)leaf, (uint32_t)cd.t_off + src[k]);
+    }
 }
 
 // ---------------------------------------------------------------------------
@@ -2604,7 +2615,9 @@ void launch_traverse(const DevPtrs &d, int block, bool packets, cudaStream_t st)
     }
 }
 void launch_pair_compact(const DevPtrs &d, cudaStream_t st) {
-    if (d.Ttot) k_pair_compact<<<nblk((int64_t)d.Ttot * kCompactLanes), kThreads, 0, st>>>(d);
+    if (!d.Ttot) return;
+    const int per = d.Ttot > kCompactManyLeaves ? 32 : 4;
+    k_pair_compact<<<nblk(((int64_t)d.Ttot + per - 1) / per * 32), kThreads, 0, st>>>(d, per);
 }
 void launch_narrow(const DevPtrs &d, const uint32_t *npairs, const uint32_t *ncv, const uint32_t *nce, int grid,
                    int stage, cudaStream_t st) {

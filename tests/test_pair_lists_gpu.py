@@ -38,6 +38,36 @@ def test_leaf_pairs(cuda, n, chunk):
         t.close()
 
 
+@pytest.mark.parametrize("n", [(1 << 17) - 1, 1 << 17, (1 << 17) + 33])
+def test_many_leaves(cuda, n):
+    """Around the size at which a warp takes 32 leaves: a chain of boxes, each
+    overlapping the next one along x, pairs with and without gaps."""
+    torch = cuda
+    k = np.arange(n, dtype=np.float64)
+    lo = np.stack([k / n, np.zeros(n), np.zeros(n)], 1)
+    hi = lo + [[1.4 / n, 1e-3, 1e-3]]
+    hi[::3, 0] = lo[::3, 0] + 0.4 / n  # every third reaches nobody
+    lo, hi = lo.astype(np.float32), hi.astype(np.float32)
+    want = {(i, i + 1) for i in np.flatnonzero(hi[:-1, 0] >= lo[1:, 0]).tolist()}
+    t = Lbvh(n)
+    try:
+        dl, dh = torch.from_numpy(lo).cuda(), torch.from_numpy(hi).cuda()
+        t.build(dl.data_ptr(), dh.data_ptr(), n)
+        out = torch.zeros((4 * n, 2), dtype=torch.int32, device="cuda")
+        got = t.pairs(out.data_ptr(), 4 * n)
+        ids = torch.zeros(n, dtype=torch.int32, device="cuda")
+        t.sorted_ids(ids.data_ptr())
+        ids = ids.cpu().numpy()
+        p = out[:got].cpu().numpy()
+    finally:
+        t.close()
+    assert np.all(np.diff(p[:, 0]) >= 0)
+    pairs = np.sort(ids[p], axis=1)
+    overlap = hi[pairs[:, 0], 0] >= lo[pairs[:, 1], 0]
+    assert overlap.all() and len({tuple(q) for q in pairs.tolist()}) == got
+    assert want <= {tuple(q) for q in pairs.tolist()}
+
+
 @pytest.mark.parametrize("variant", [1, 2])
 @pytest.mark.parametrize("friction", [0, 1])
 def test_contact_lists_are_ordered(cuda, variant, friction):
