@@ -30,7 +30,7 @@ void launch_leaves_from_boxes(const DevPtrs &d, const float *bmin, const float *
                               cudaStream_t st);
 void launch_morton_sort(const DevPtrs &d, const int *tile_first, int mode, int max_T, cudaStream_t st);
 void launch_hierarchy(const DevPtrs &d, int max_T, cudaStream_t st);
-void launch_traverse(const DevPtrs &d, int block, bool packets, cudaStream_t st);
+void launch_traverse(const DevPtrs &d, int block, cudaStream_t st);
 void launch_pair_compact(const DevPtrs &d, cudaStream_t st);
 void launch_narrow(const DevPtrs &d, const uint32_t *npairs, const uint32_t *ncv, const uint32_t *nce, int grid,
                    int stage, cudaStream_t st);
@@ -468,7 +468,7 @@ lc_status lc_batch::enqueue_step(cudaStream_t st) {
     LC_PHASE(3);
     // 4. Create Triangle Tests
     LC_KEV(2);
-    launch_traverse(d, traverse_block, d.Ttot > kPacketLeaves, st);
+    launch_traverse(d, traverse_block, st);
     LC_KEV(3);
     const uint32_t T = (uint32_t)d.Ttot, V = (uint32_t)d.Vtot;
     scan_u32({d.pair_cnt, d.pair_off, nullptr, T, T, npairs, &d.counters[0]}, nullptr, d.scan_tmp, d.err, st);
@@ -2465,7 +2465,7 @@ lc_status lc_lbvh_pairs(lc_lbvh *h, uint32_t *out_pairs, uint64_t cap, uint64_t 
     cudaStream_t st = (cudaStream_t)stream;
     lc_batch &b = h->b;
     DevPtrs &d = b.d;
-    launch_traverse(d, b.traverse_block, false, st);
+    launch_traverse(d, b.traverse_block, st);
     scan_u32({d.pair_cnt, d.pair_off, nullptr, (uint32_t)d.Ttot, (uint32_t)d.Ttot, b.npairs, &d.counters[0]}, nullptr,
              d.scan_tmp, d.err, st);
     launch_pair_compact(d, st);

@@ -357,7 +357,9 @@ __global__ void k_bp_bvh(BvhPtrs B, const float *lo, const float *hi, const uint
                 leaf(node - I);
             } else {
                 const float4 *r = B.rec + 4 * (size_t)node;
-                const float4 l0 = __ldg(r), l1 = __ldg(r + 1), r0 = __ldg(r + 2), r1 = __ldg(r + 3);
+                float4 l0, l1, r0, r1;
+                ld_pair(r, l0, l1);
+                ld_pair(r + 2, r0, r1);
                 const int chx = __float_as_int(l0.w), chy = __float_as_int(r0.w);
                 bool ol = __float_as_int(l1.w) > s && overlap(alo, ahi, xyz(l0), xyz(l1));
                 bool orr = __float_as_int(r1.w) > s && overlap(alo, ahi, xyz(r0), xyz(r1));

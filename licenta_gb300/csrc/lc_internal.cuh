@@ -20,8 +20,7 @@ constexpr int kRangePad = 32;            // range-tree entries of a cloth of T l
 constexpr int kTraverseStack = 64;       // Collision/CudaBVH.cu:38
 constexpr int kBothCcdLeaves = 48 << 10;    // leaves up to which the VF and the EE CCD share a launch
 constexpr uint64_t kBothCcdPairs = 10ull * kBothCcdLeaves;  // the same for the narrowphase entry (ten pairs a leaf)
-constexpr int kPacketLeaves = 1 << 20;   // leaves above which a batch's traversal walks 32 of them together
-constexpr int kTraverseBlockMax = 256;   // largest traversal block (the packet kernel is bounded for 6 of them per SM)
+constexpr int kTraverseBlockMax = 256;   // largest traversal block
 constexpr uint32_t kScanBlocks = 304;    // largest grid of the device-count scans
 constexpr uint32_t kScanScratch = 2 * (2 * kScanBlocks + 2);  // u32 words of scratch of two scans in one launch
 constexpr int kPairGroup = 32;           // consecutive pairs per narrowphase expansion warp (one per lane)
@@ -303,6 +302,11 @@ __host__ __device__ __forceinline__ bool overlap(float3 amin, float3 amax, float
     bool b = amax.y < bmin.y || amin.y > bmax.y;
     bool c = amax.z < bmin.z || amin.z > bmax.z;
     return !(a || b || c);
+}
+// 32 bytes at a 32-byte boundary in one load.
+__device__ __forceinline__ void ld_pair(const float4 *p, float4 &a, float4 &b) {
+    asm("ld.global.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+        : "=f"(a.x), "=f"(a.y), "=f"(a.z), "=f"(a.w), "=f"(b.x), "=f"(b.y), "=f"(b.z), "=f"(b.w) : "l"(p));
 }
 __host__ __device__ __forceinline__ float4 f4(float3 a, float w) { return make_float4(a.x, a.y, a.z, w); }
 

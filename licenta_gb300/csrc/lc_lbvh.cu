@@ -1381,7 +1381,13 @@ __global__ void k_traverse(DevPtrs d) {
     if (dropped) atomicAdd(&d.counters[3], (unsigned long long)dropped);
 }
 
-// The single-leaf traversal over the records, one thread per leaf.
+// The single-leaf traversal over the records, one thread per leaf; a record is
+// two 32-byte loads.  Bound by the latency of the walk in a small batch, by the
+// records' L1 traffic in a large one.  A walk per 32 leaves, which read each
+// record once for all, was slower from the smallest batch (43 us against 24 for
+// 1922 leaves) to the largest (987 against 917 for 1.92 million, 1568 against
+// 1509 for 3.3 million): every leaf then waits for the records of all.  With
+// four 16-byte loads 442 us for 619 k leaves, 383 so; a million random boxes 95.
 __global__ void __launch_bounds__(kTraverseBlockMax) k_traverse_leaf(DevPtrs d) {
     const int s = blockIdx.x * blockDim.x + threadIdx.x;
     if (s >= d.Ttot) return;
@@ -1400,7 +1406,9 @@ __global__ void __launch_bounds__(kTraverseBlockMax) k_traverse_leaf(DevPtrs d) 
     const int guard_max = 4 * cd.T + 64;
     for (int guard = 0; guard < guard_max; ++guard) {
         const float4 *r = W + 4 * (size_t)node;
-        const float4 l0 = __ldg(r), l1 = __ldg(r + 1), r0 = __ldg(r + 2), r1 = __ldg(r + 3);
+        float4 l0, l1, r0, r1;
+        ld_pair(r, l0, l1);
+        ld_pair(r + 2, r0, r1);
         const int chx = __float_as_int(l0.w), rmx = __float_as_int(l1.w);
         const int chy = __float_as_int(r0.w), rmy = __float_as_int(r1.w);
         const bool ol = rmx > me && overlap(amin, amax, xyz(l0), xyz(l1));
@@ -1430,99 +1438,6 @@ __global__ void __launch_bounds__(kTraverseBlockMax) k_traverse_leaf(DevPtrs d) 
     d.pair_cnt[s] = (uint32_t)got;
     if (dropped) atomicAdd(&d.counters[3], (unsigned long long)dropped);
 }
-
-// The traversal as a packet: a left-first depth-first walk of a Karras tree
-// meets the leaves in increasing index order, so leaf i's result is the
-// increasing list of leaves j > i whose boxes overlap its own, cut at the
-// chunk size.  A warp walks the tree once for its 32 consecutive leaves
-// (spatially close in Morton order): every node record is read once for the
-// warp, each lane tests its own box (and rightmost-leaf bound) against the
-// two children, and the warp descends into a child when any lane needs it.
-// Each lane keeps exactly the leaves it overlaps, in the walk's order, so
-// every chunk is the single-leaf traversal's.  A warp whose leaves span two
-// cloths walks each cloth's tree for its own lanes.
-// At most 40 registers (6 blocks of 256, or 12 of 128, per SM): the walk
-// waits on dependent node fetches, and 12 resident 4-warp blocks hide more of
-// that latency than the 10 that 41 registers allowed.
-__global__ void __launch_bounds__(kTraverseBlockMax, 6) k_traverse_packet(DevPtrs d) {
-    static_assert(kTraverseStack == 64, "two stack slots per lane");
-    const unsigned full = 0xffffffffu;
-    const int lane = threadIdx.x & 31;
-    // the warp's stack in registers: slot k in lane k % 32, register k / 32
-    int stk0 = 0, stk1 = 0;
-    const int s = ((blockIdx.x * blockDim.x + threadIdx.x) >> 5) * 32 + lane;
-    const bool valid = s < d.Ttot;
-    int c = -1, me = 0, got = 0, chunk = 0;
-    uint32_t dropped = 0;
-    uint32_t *out = nullptr;
-    float3 amin = f3(0.f, 0.f, 0.f), amax = amin;
-    bool has_tree = false;
-    if (valid) {
-        c = d.tcloth[s];
-        const ClothDev &cd = d.cloth[c];
-        const int id = s - cd.t_off, In = cd.T - 1;
-        has_tree = In > 0;
-        me = In + id;
-        chunk = cd.chunk;
-        out = d.pair_chunk + cd.pc_off + (int64_t)id * chunk;
-        if (has_tree) {
-            amin = xyz(d.nmin[cd.n_off + me]);
-            amax = xyz(d.nmax[cd.n_off + me]);
-        }
-    }
-    unsigned pending = __ballot_sync(full, has_tree);
-    bool overflow = false;
-    while (pending) {
-        const int leader = __ffs(pending) - 1;
-        const int cc = __shfl_sync(full, c, leader);
-        const bool mine = ((pending >> lane) & 1u) && c == cc;
-        pending &= ~__ballot_sync(full, mine);
-        const ClothDev &cd = d.cloth[cc];
-        const int In = cd.T - 1;
-        const float4 *W = d.wnode + 4 * (size_t)cd.i_off;
-        int top = 1, node = 0;
-        if (lane == 0) stk0 = -1;
-        const int guard_max = 4 * cd.T + 64;
-        for (int guard = 0; guard < guard_max; ++guard) {
-            const float4 *r = W + 4 * (size_t)node;
-            const float4 l0 = __ldg(r), l1 = __ldg(r + 1), r0 = __ldg(r + 2), r1 = __ldg(r + 3);
-            const int chx = __float_as_int(l0.w), rmx = __float_as_int(l1.w);
-            const int chy = __float_as_int(r0.w), rmy = __float_as_int(r1.w);
-            const bool ol = mine && rmx > me && overlap(amin, amax, xyz(l0), xyz(l1));
-            const bool orr = mine && rmy > me && overlap(amin, amax, xyz(r0), xyz(r1));
-            if (ol && chx >= In) {
-                if (got < chunk) out[got++] = (uint32_t)(chx - In);
-                else ++dropped;
-            }
-            if (orr && chy >= In) {
-                if (got < chunk) out[got++] = (uint32_t)(chy - In);
-                else ++dropped;
-            }
-            const bool tl = chx < In && __any_sync(full, ol), tr = chy < In && __any_sync(full, orr);
-            if (!tl && !tr) {
-                --top;
-                const int a = __shfl_sync(full, stk0, top & 31), b = __shfl_sync(full, stk1, top & 31);
-                node = top < 32 ? a : b;
-            } else {
-                node = tl ? chx : chy;
-                if (tl && tr) {
-                    if (top >= kTraverseStack) { overflow = true; break; }
-                    if (lane == (top & 31)) {
-                        if (top < 32) stk0 = chy;
-                        else stk1 = chy;
-                    }
-                    ++top;
-                }
-            }
-            if (top == 0) break;
-        }
-        __syncwarp();
-    }
-    if (overflow && lane == 0) atomicOr(d.err, ERR_STACK);
-    if (valid) d.pair_cnt[s] = (uint32_t)got;
-    if (dropped) atomicAdd(&d.counters[3], (unsigned long long)dropped);
-}
-
 
 // Order-preserving compaction of the per-leaf chunks into the pair list: a
 // warp takes `per` leaves and copies those with pairs four at a time, eight lanes
@@ -1708,13 +1623,10 @@ __device__ __forceinline__ bool ee_apart(float3 x1, float3 x2, float3 x3, float3
 // x and x_prev (min/max are exact, so this equals the stored boxes).
 struct Box { float3 lo, hi; };
 __device__ __forceinline__ Box pbox(const DevPtrs &d, int v, float h) {
-    if (d.vbox) {  // the same operations, once per vertex: one 32-byte load
-        Box b;
-        float pad0, pad1;
-        asm("ld.global.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
-            : "=f"(b.lo.x), "=f"(b.lo.y), "=f"(b.lo.z), "=f"(pad0), "=f"(b.hi.x), "=f"(b.hi.y), "=f"(b.hi.z), "=f"(pad1)
-            : "l"(d.vbox + 2 * (size_t)v));
-        return b;
+    if (d.vbox) {  // the same operations, once per vertex
+        float4 lo, hi;
+        ld_pair(d.vbox + 2 * (size_t)v, lo, hi);
+        return Box{xyz(lo), xyz(hi)};
     }
     const float3 p = xyz(d.x[v]), q = xyz(d.xp[v]);
     return Box{subc(vmin(p, q), h), addc(vmax(p, q), h)};
@@ -2599,17 +2511,10 @@ void launch_hierarchy(const DevPtrs &d, int max_T, cudaStream_t st) {
     k_refit_upper<<<std::min(nblk(2 * (int64_t)std::max(d.Itot, 1)), 1024), kThreads, 0, st>>>(d);
     k_pack_nodes<<<nblk(d.Ttot), kThreads, 0, st>>>(d);
 }
-// packets: one walk per 32 leaves, else one per leaf (us, cloths of 1922, 20 k,
-// 102 k, 522 k, 619 k and 1.92 million leaves 43, 68, 131, 137, 443 and 983
-// against 24, 37, 98, 110, 414 and 1038; a million random boxes 181 against 95).
-// One walk per leaf has less to do and waits for fewer loads; the packet reads
-// a record once for 32 leaves, which pays where swept boxes of a large batch
-// overlap dozens of neighbours and the record reads bind.
-void launch_traverse(const DevPtrs &d, int block, bool packets, cudaStream_t st) {
+void launch_traverse(const DevPtrs &d, int block, cudaStream_t st) {
     if (!d.Ttot) return;
     if (d.wnode) {
-        if (packets) k_traverse_packet<<<nblk(d.Ttot, block), block, 0, st>>>(d);
-        else k_traverse_leaf<<<nblk(d.Ttot, block), block, 0, st>>>(d);
+        k_traverse_leaf<<<nblk(d.Ttot, block), block, 0, st>>>(d);
     } else {
         k_traverse<<<nblk(d.Ttot, block), block, 0, st>>>(d);
     }

@@ -31,7 +31,7 @@ void launch_leaves_from_boxes(const DevPtrs &d, const float *bmin, const float *
                               cudaStream_t st);
 void launch_morton_sort(const DevPtrs &d, const int *tile_first, int mode, int max_T, cudaStream_t st);
 void launch_hierarchy(const DevPtrs &d, int max_T, cudaStream_t st);
-void launch_traverse(const DevPtrs &d, int block, bool packets, cudaStream_t st);
+void launch_traverse(const DevPtrs &d, int block, cudaStream_t st);
 
 namespace {
 
@@ -239,7 +239,7 @@ extern "C" lc_status lc_lbvh_pairs_static(const float *tri_min, const float *tri
     launch_leaves_from_boxes(d, tri_min, tri_max, T, morton_mode, st);
     launch_morton_sort(d, tile_first, morton_mode, T, st);
     launch_hierarchy(d, T, st);
-    launch_traverse(d, 128, false, st);
+    launch_traverse(d, 128, st);
     scan_u32({d.pair_cnt, d.pair_off, nullptr, (uint32_t)T, (uint32_t)T, npairs, &d.counters[0]}, nullptr, d.scan_tmp,
              d.err, st);
     const int nwb = (T * 32 + kThreads - 1) / kThreads;  // one warp per leaf

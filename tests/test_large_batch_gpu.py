@@ -1,6 +1,6 @@
-"""Batches of more leaves than the traversal's rule sends to single-leaf walks
-take the packet walk: the same cloths give the same bits on both sides of it,
-also where the pair chunk of a triangle is full."""
+"""Batches of more than a million leaves: every cloth's pairs and state are the
+bits of the same cloth alone, also where the pair chunk of a triangle is
+full."""
 from __future__ import annotations
 
 import numpy as np
@@ -13,7 +13,7 @@ pytestmark = pytest.mark.gpu
 
 @pytest.mark.parametrize("chunk", [64, 10])
 @pytest.mark.parametrize("side,copies", [(191, 15), (190, 15), (64, 133)])
-def test_packets_equal_single_walks(cuda, side, copies, chunk):
+def test_a_cloth_in_a_large_batch_equals_the_cloth_alone(cuda, side, copies, chunk):
     spec = scenes.small_cloth(seed=side, n=side, thickness=0.6 / side)
     spec.params.BVHChunkSize = chunk
     assert copies * spec.indices.size // 3 > 1 << 20
