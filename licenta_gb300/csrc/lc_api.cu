@@ -2085,7 +2085,7 @@ lc_status lc_batch_counters(lc_batch *b, uint64_t out[4]) {
 lc_status lc_batch::cloth_contacts(int c, bool vf, std::vector<uint64_t> &gidx, std::vector<int4> &iv,
                                    std::vector<float4> &wv) {
     // a cloth's contacts of each kind are one contiguous range of the batch's
-    // list (k_contact_ranges writes it every step)
+    // list (k_ccd_emit writes it every step)
     const ClothDev &cd = cds[c];
     uint4 cr;
     LC_CUDA(cudaMemcpy(&cr, d.crange + c, sizeof(uint4), cudaMemcpyDeviceToHost));
