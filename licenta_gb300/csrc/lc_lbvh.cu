@@ -1047,8 +1047,11 @@ __global__ void __launch_bounds__(BS) k_karras(DevPtrs d) {
         s_key[0] = B0 > 0 ? d.keys[B0 - 1] : 0ull;
         s_key[B1 - B0 + 1] = B1 < d.Ttot ? d.keys[B1] : 0ull;
     }
-    // (block-uniform: flagged cloths take their boxes from the climb)
-    const bool tree = d.eq3 && !(d.eq3[d.tcloth[B0]] && d.eq3[d.tcloth[B1 - 1]]);
+    // (block-uniform: flagged cloths take their boxes from the climb, so the
+    // leaves are of no use only where every cloth of the block is flagged)
+    bool tree = false;
+    if (d.eq3)
+        for (int c = d.tcloth[B0], c1 = d.tcloth[B1 - 1]; c <= c1 && !tree; ++c) tree = !d.eq3[c];
 #pragma unroll
     for (int q = 0; q < SPAN / BS; ++q) {
         const int k = q * BS + t;
