@@ -503,7 +503,7 @@ lc_status lc_broadphase_create(const lc_broadphase_desc *desc, lc_broadphase **o
 lc_status lc_broadphase_update(lc_broadphase *b, const float *box_min, const float *box_max, int32_t num_objects,
                                void *stream);
 /* The boxes from host memory, copied into the handle's own device buffers
- * (which the following test reads). */
+ * (which the following test reads) by the time the call returns. */
 lc_status lc_broadphase_update_host(lc_broadphase *b, const float *box_min, const float *box_max,
                                     int32_t num_objects, void *stream);
 lc_status lc_broadphase_test(lc_broadphase *b, uint32_t *pairs, uint64_t cap, uint64_t *count, void *stream);

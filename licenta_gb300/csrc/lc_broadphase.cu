@@ -653,6 +653,7 @@ lc_status lc_broadphase_update_host(lc_broadphase *b, const float *box_min, cons
     if (n > 0) {
         LC_BP_CUDA(cudaMemcpyAsync(b->hlo, box_min, sizeof(float) * 3 * (size_t)n, cudaMemcpyHostToDevice, st));
         LC_BP_CUDA(cudaMemcpyAsync(b->hhi, box_max, sizeof(float) * 3 * (size_t)n, cudaMemcpyHostToDevice, st));
+        LC_BP_CUDA(cudaStreamSynchronize(st));  // page-locked arrays are the caller's again on return
     }
     return lc_broadphase_update(b, b->hlo, b->hhi, n, stream);
 }
