@@ -1604,8 +1604,11 @@ __device__ __forceinline__ bool ee_far(float3 a, float3 b, float3 c, float3 d, f
 // axis, the line through their midpoints halfway, are apart by more than th
 // plus the margin at both ends (the gap, a minimum of linear functions of T less
 // a maximum of such, is concave, so nowhere between the ends is it smaller).  The margin
-// also covers what the roundings of the advances, and of this, add at the
-// coordinates' size.  NaN anywhere: not apart.
+// also covers what roundings add at the size S of the coordinates, the largest
+// over the vertices of |x| + T |v|: a vertex advanced six times at most is off
+// by 13 u S (u = 2^-24, half a spacing), so two edges by 26 u S; the gap as
+// computed here by 53 u S; the test's closest points by less than 20 u S:
+// below 6e-6 S = 100 u S together.  NaN anywhere: not apart.
 __device__ __forceinline__ bool ee_apart(float3 x1, float3 x2, float3 x3, float3 x4, float3 v1, float3 v2, float3 v3,
                                          float3 v4, float lo, float hi, float th) {
     const float3 u = sub(x2, x1), v = sub(x3, x1), w = sub(x4, x1);
@@ -1616,9 +1619,12 @@ __device__ __forceinline__ bool ee_apart(float3 x1, float3 x2, float3 x3, float3
     const float qu = dot(du, m), qv = dot(dv, m), qw = dot(dw, m);
     const float gl = fminf(pv + qv * lo, pw + qw * lo) - fmaxf(pu + qu * lo, 0.f);
     const float gh = fminf(pv + qv * hi, pw + qw * hi) - fmaxf(pu + qu * hi, 0.f);
-    const float size = fabsf(x1.x) + fabsf(x1.y) + fabsf(x1.z) +
-                       fmaxf(fabsf(lo), fabsf(hi)) * (fabsf(v1.x) + fabsf(v1.y) + fabsf(v1.z));
-    const float t = 1.001f * th + 1e-5f + 4e-6f * size;
+    const float T = fmaxf(fabsf(lo), fabsf(hi));
+    auto reach = [&](float3 x, float3 vel) {
+        return fabsf(x.x) + fabsf(x.y) + fabsf(x.z) + T * (fabsf(vel.x) + fabsf(vel.y) + fabsf(vel.z));
+    };
+    const float size = fmaxf(fmaxf(reach(x1, v1), reach(x2, v2)), fmaxf(reach(x3, v3), reach(x4, v4)));
+    const float t = 1.001f * th + 1e-5f + 6e-6f * size;
     return fminf(gl, gh) > 0.f && gl * gl > t * t * dot(m, m) && gh * gh > t * t * dot(m, m);
 }
 
