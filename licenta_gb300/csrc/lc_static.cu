@@ -253,6 +253,10 @@ extern "C" lc_status lc_lbvh_pairs_static(const float *tri_min, const float *tri
     LC_STATIC_CUDA(cudaMemcpyAsync(&err, d.err, sizeof(err), cudaMemcpyDeviceToHost, st));
     LC_STATIC_CUDA(cudaStreamSynchronize(st));
     *count = n;
+    if (err & ERR_SORT) {
+        lc::set_last_error("lc_lbvh_pairs_static: sort or scan wait exceeded its bound");
+        return LC_ERR_TIMEOUT;
+    }
     if (err & ERR_STACK) {
         lc::set_last_error("lc_lbvh_pairs_static: BVH traversal stack (64) exceeded");
         return LC_ERR_STACK_OVERFLOW;
