@@ -539,7 +539,8 @@ typedef struct lc_primitive_contact {
  * lc_narrowphase_run writes them; VF first in the impulse order).  Stiffness
  * is the reference's kStretch, vertex_mass objectMass / vertex count.
  * Allocates its scratch in stream order (cudaMallocAsync) and, when there are
- * contacts, waits for the stream once to validate their vertex ids. */
+ * contacts, waits for the stream once before x and v are written, to validate
+ * their vertex ids and that the lists were built (else LC_ERR_TIMEOUT). */
 lc_status lc_solve_collisions(float *x, const float *x_prev, float *v, const uint8_t *fixed, int32_t num_vertices,
                               const lc_primitive_contact *vf, uint64_t num_vf, const lc_primitive_contact *ee,
                               uint64_t num_ee, float stiffness, float vertex_mass, float timestep, float thickness,

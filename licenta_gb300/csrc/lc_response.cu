@@ -38,13 +38,14 @@ __global__ void k_imp_check(const lc_primitive_contact *__restrict__ vf, uint64_
 
 // _CreateImpulses / _CreateImpulseVF / _CreateImpulseEE / _CreateImpulse
 // (Collision/CudaCollisionResponse.cu:142-254): the contact's four impulses,
-// and the per-vertex impulse counts.
+// and the per-vertex impulse counts.  Nothing when k_imp_check found a bad id.
 __global__ void k_imp_create(const float *__restrict__ pos, const float *__restrict__ vel,
                              const lc_primitive_contact *__restrict__ vf, uint64_t nvf,
                              const lc_primitive_contact *__restrict__ ee, uint64_t nee, float stiffness, float mass,
-                             float dt, float h, float4 *__restrict__ vals, uint32_t *__restrict__ cnt) {
+                             float dt, float h, const uint32_t *__restrict__ bad, float4 *__restrict__ vals,
+                             uint32_t *__restrict__ cnt) {
     const uint64_t id = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
-    if (id >= nvf + nee) return;
+    if (id >= nvf + nee || *bad) return;
     const bool isvf = id < nvf;
     const lc_primitive_contact c = isvf ? vf[id] : ee[id - nvf];
     float3 vr;
@@ -166,38 +167,44 @@ extern "C" lc_status lc_solve_collisions(float *x, const float *x_prev, float *v
     uint32_t *cnt = nullptr, *off = nullptr, *cur = nullptr, *slots = nullptr, *flag = nullptr, *rank = nullptr,
              *part = nullptr, *bad = nullptr;
     float4 *vals = nullptr;
-    uint32_t hbad = 0;
+    uint32_t seen[2] = {0, 0};  // bad ids, error word
     // scratch in stream order from the device's default pool
     LC_R_CUDA(cudaMallocAsync((void **)&cnt, 2 * sizeof(uint32_t) * V, st));
     cur = cnt + V;
     LC_R_CUDA(cudaMallocAsync((void **)&off, sizeof(uint32_t) * (V + 1), st));
     LC_R_CUDA(cudaMallocAsync((void **)&flag, sizeof(uint32_t) * V, st));
     LC_R_CUDA(cudaMallocAsync((void **)&rank, sizeof(uint32_t) * (V + 1), st));
-    LC_R_CUDA(cudaMallocAsync((void **)&part, sizeof(uint32_t) * (kScanScratch + 1), st));
+    LC_R_CUDA(cudaMallocAsync((void **)&part, sizeof(uint32_t) * (kScanScratch + 2), st));
     bad = part + kScanScratch;
     LC_R_CUDA(cudaMallocAsync((void **)&slots, 2 * sizeof(uint32_t) * std::max<uint64_t>(S, 1), st));
     LC_R_CUDA(cudaMallocAsync((void **)&vals, sizeof(float4) * std::max<uint64_t>(S, 1), st));
     LC_R_CUDA(cudaMemsetAsync(cnt, 0, 2 * sizeof(uint32_t) * V, st));
-    LC_R_CUDA(cudaMemsetAsync(part, 0, sizeof(uint32_t) * (kScanScratch + 1), st));
+    LC_R_CUDA(cudaMemsetAsync(part, 0, sizeof(uint32_t) * (kScanScratch + 2), st));
     if (C) {
         k_imp_check<<<cblk, nb, 0, st>>>(vf, num_vf, ee, num_ee, V, bad);
-        LC_R_CUDA(cudaMemcpyAsync(&hbad, bad, sizeof(uint32_t), cudaMemcpyDeviceToHost, st));
+        k_imp_create<<<cblk, nb, 0, st>>>(x_prev, v, vf, num_vf, ee, num_ee, stiffness, vertex_mass, timestep,
+                                          thickness, bad, vals, cnt);
+    }
+    scan_u32({cnt, off, nullptr, (uint32_t)V, (uint32_t)V, nullptr, nullptr}, nullptr, part, bad + 1, st);
+    k_imp_flag<<<vblk, nb, 0, st>>>(cnt, flag, V);
+    scan_u32({flag, rank, nullptr, (uint32_t)V, (uint32_t)V, nullptr, nullptr}, nullptr, part, bad + 1, st);
+    if (C) {  // (without contacts every sum is zero, seen or not)
+        // the lists below hold only with the ids checked and the scans complete
+        LC_R_CUDA(cudaMemcpyAsync(seen, bad, sizeof(seen), cudaMemcpyDeviceToHost, st));
         LC_R_CUDA(cudaStreamSynchronize(st));
-        if (hbad) {
+        if (seen[0]) {
             lc::set_last_error("lc_solve_collisions: a contact vertex id is out of range");
             status = LC_ERR_INVALID_ARG;
             goto done;
         }
-        k_imp_create<<<cblk, nb, 0, st>>>(x_prev, v, vf, num_vf, ee, num_ee, stiffness, vertex_mass, timestep,
-                                          thickness, vals, cnt);
-    }
-    scan_u32({cnt, off, nullptr, (uint32_t)V, (uint32_t)V, nullptr, nullptr}, nullptr, part, nullptr, st);
-    if (C) {
+        if (seen[1] & ERR_SORT) {
+            lc::set_last_error("lc_solve_collisions: scan wait exceeded its bound");
+            status = LC_ERR_TIMEOUT;
+            goto done;
+        }
         k_imp_fill<<<cblk, nb, 0, st>>>(vf, num_vf, ee, num_ee, off, cur, slots + S);
         k_imp_sort<<<(unsigned)((S + nb - 1) / nb), nb, 0, st>>>(vf, num_vf, ee, num_ee, off, slots + S, slots);
     }
-    k_imp_flag<<<vblk, nb, 0, st>>>(cnt, flag, V);
-    scan_u32({flag, rank, nullptr, (uint32_t)V, (uint32_t)V, nullptr, nullptr}, nullptr, part, nullptr, st);
     k_imp_apply<<<vblk, nb, 0, st>>>(x, x_prev, v, fixed, V, off, slots, rank, vals, (C + 255) / 256 * 256,
                                      vertex_mass, timestep);
     LC_R_CUDA(cudaGetLastError());
