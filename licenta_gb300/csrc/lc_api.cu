@@ -877,6 +877,26 @@ static lc_status alloc_range_tree(lc_batch *b, int64_t T, int C) {
     return LC_OK;
 }
 
+// The sort's scratch for C segments of T keys in all, cut into `tiles` tiles.
+static lc_status alloc_sort(lc_batch *b, int64_t T, int C, int64_t tiles) {
+    DevPtrs &d = b->d;
+    DeviceArena &A = b->arena;
+    LC_TRY(A.alloc(d.sseg, kSortHead + (size_t)C * kSortPassesMax * kSortBuckets, "sort segment totals"));
+    int64_t words = tiles;
+    if (b->morton_mode != LC_MORTON_K30) {
+        // at most so many runs of more than kTieRun keys, of more than a tile,
+        // and tiles of the latter
+        const int64_t small = T / (kTieRun + 1) + 1, tiled = T / (kSortTile + 1) + 1, run_tiles = 2 * T / (kSortTile + 1) + 1;
+        words = std::max(words, run_tiles);
+        LC_TRY(A.alloc(d.run_tiled, tiled, "long runs"));
+        LC_TRY(A.alloc(d.run_total, tiled * 4 * kSortBuckets + 2 * small + run_tiles, "long run totals"));
+        d.run_small = reinterpret_cast<int2 *>(d.run_total + tiled * 4 * kSortBuckets);
+        d.run_of_tile = reinterpret_cast<int *>(d.run_small + small);
+    }
+    LC_TRY(A.alloc(d.sstat, (size_t)kSortPassesMax * words * kSortBuckets, "sort look-back status"));
+    return LC_OK;
+}
+
 static lc_status batch_build(lc_batch *b, const lc_cloth_desc *descs, int n, const lc_batch_options &opt_in) {
     lc_batch_options opt = opt_in;
     // adjoint batches: the reverse pass replays the global-memory Jacobi
@@ -1028,9 +1048,7 @@ static lc_status batch_build(lc_batch *b, const lc_cloth_desc *descs, int n, con
     int *stc, *sts, *tf; LC_TRY(A.alloc(stc, stile_cloth.size(), "stile_cloth"));
     LC_TRY(A.alloc(sts, stile_start.size(), "stile_start")); LC_TRY(A.alloc(tf, n + 1, "tile_first"));
     d.stile_cloth = stc; d.stile_start = sts; b->tile_first = tf;
-    LC_TRY(A.alloc(d.shist, (size_t)stile_cloth.size() * kSortBuckets, "shist"));
-    LC_TRY(A.alloc(d.sseg, kSortPassesMax + (size_t)n * kSortPassesMax * kSortBuckets, "sort segment totals"));
-    LC_TRY(A.alloc(d.sstat, (size_t)kSortPassesMax * stile_cloth.size() * kSortBuckets, "sort look-back status"));
+    LC_TRY(alloc_sort(b, T, n, (int64_t)stile_cloth.size()));
     int *vbc, *vbs, *vbf; LC_TRY(A.alloc(vbc, vblk_cloth.size(), "vblk_cloth")); LC_TRY(A.alloc(vbs, vblk_start.size(), "vblk_start"));
     LC_TRY(A.alloc(vbf, vb_first.size(), "vb_first"));
     d.vblk_cloth = vbc; d.vblk_start = vbs; d.vb_first = vbf;
@@ -2416,9 +2434,7 @@ lc_status lc_lbvh_create(int32_t max_triangles, int32_t chunk_size, int32_t mort
     int *stc, *sts, *tf;
     LC_TRY(A.alloc(stc, tiles, "stile_cloth")); LC_TRY(A.alloc(sts, tiles, "stile_start")); LC_TRY(A.alloc(tf, 2, "tile_first"));
     d.stile_cloth = stc; d.stile_start = sts; b.tile_first = tf;
-    LC_TRY(A.alloc(d.shist, tiles * kSortBuckets, "shist"));
-    LC_TRY(A.alloc(d.sseg, kSortPassesMax + (size_t)kSortPassesMax * kSortBuckets, "sort segment totals"));
-    LC_TRY(A.alloc(d.sstat, (size_t)kSortPassesMax * tiles * kSortBuckets, "sort look-back status"));
+    LC_TRY(alloc_sort(&b, T, 1, tiles));
     LC_TRY(A.alloc(b.npairs, 1, "npairs"));
     d.pair_cap = (uint64_t)PC;
     LC_CUDA(cudaMemset(d.err, 0, sizeof(uint32_t)));

@@ -564,7 +564,7 @@ lc_status lc_broadphase_create(const lc_broadphase_desc *desc, lc_broadphase **o
         d.stile_cloth = stc;
         d.stile_start = sts;
         LC_TRY_BP(b.alloc(d.shist, tiles * kSortBuckets, "sort histograms"));
-        LC_TRY_BP(b.alloc(d.sseg, kSortPassesMax + (size_t)kSortPassesMax * kSortBuckets, "sort segment totals"));
+        LC_TRY_BP(b.alloc(d.sseg, kSortHead + (size_t)kSortPassesMax * kSortBuckets, "sort segment totals"));
         LC_TRY_BP(b.alloc(d.sstat, (size_t)kSortPassesMax * tiles * kSortBuckets, "sort look-back status"));
         d.err = b.err;
         LC_TRY_BP(b.alloc(d.keys, keys, "keys"));

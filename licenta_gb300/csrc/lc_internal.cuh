@@ -15,7 +15,11 @@ constexpr int kThreads = 256;
 constexpr int kSortBits = 8;
 constexpr int kSortBuckets = 1 << kSortBits;
 constexpr int kSortTile = 2048;          // keys per sort tile (256 threads x 8)
-constexpr int kSortPassesMax = 8;        // 8-bit digits of a 63-bit key
+constexpr int kSortPassesMax = 4;        // one-sweep passes: 8-bit digits of half a key
+// First words of sseg: a tile ticket per pass, then the long runs' counts (of
+// one tile, of more, the latter's tiles), ticket and finished items.
+enum { kRunsSmall = kSortPassesMax, kRunsTiled, kRunsTiles, kRunsTicket, kRunsDone, kSortHead };
+constexpr int kTieRun = 64;              // longest run of equal top halves that the post-sort ranks
 constexpr int kRangePad = 32;            // range-tree entries of a cloth of T leaves: at most T + kRangePad
 constexpr int kTraverseStack = 64;       // Collision/CudaBVH.cu:38
 constexpr int kBothCcdLeaves = 48 << 10;    // leaves up to which the VF and the EE CCD share a launch
@@ -216,9 +220,17 @@ struct DevPtrs {
     int nstiles;
     uint32_t *shist;          // per tile x bucket counts / offsets
     // one-sweep scratch (both null: per-pass histograms and k_sort_offsets):
-    // sseg = kSortPassesMax tile tickets, then per segment x pass x digit the
-    // segment's digit totals; sstat = per pass x tile x digit look-back status
+    // sseg = kSortHead words, then per segment x pass x digit the segment's
+    // digit totals; sstat = per pass x tile x digit look-back status
     uint32_t *sseg, *sstat;
+    // runs of more than kTieRun equal top halves: those of one sort tile, and
+    // the others (first, end, first tile, whether out of order) with the run
+    // of each of their tiles and four passes' digit totals (null: keys are
+    // sorted whole)
+    int2 *run_small;
+    int4 *run_tiled;
+    int *run_of_tile;
+    uint32_t *run_total;
     const int *vblk_cloth, *vblk_start;  // vertex blocks never straddle cloths
     const int *vb_first;                 // per cloth: first vertex block (C+1 entries)
     double *damp_part;                   // 16 partial sums per vertex block

@@ -180,8 +180,9 @@ __global__ void __launch_bounds__(kSortBuckets * kOffsetsSplit) k_sort_offsets(D
     }
 }
 
-// One-sweep offsets (every sort with look-back scratch; the allocation-free
-// entry keeps the per-pass histogram above).  k_sort_hist_all reads each
+// One-sweep offsets (every sort of up to 2^30 keys; beyond, which only the
+// object broadphase's grid and hash entries can reach, the per-pass histogram
+// above).  k_sort_hist_all reads each
 // tile's keys once and adds the digit counts of every pass to its segment's
 // totals, so the digits' first positions in the segment are known before
 // the first pass; the scatter of a pass then finds a tile's place among its
@@ -226,7 +227,7 @@ __global__ void __launch_bounds__(kThreads) k_sort_hist_all(DevPtrs d, const uns
         }
     }
     __syncthreads();
-    uint32_t *seg = d.sseg + kSortPassesMax + (size_t)c * kSortPassesMax * kSortBuckets;
+    uint32_t *seg = d.sseg + kSortHead + (size_t)c * kSortPassesMax * kSortBuckets;
     for (int p = 0; p < passes; ++p)
         if (h[p][t]) atomicAdd(&seg[p * kSortBuckets + t], h[p][t]);
 }
@@ -252,39 +253,41 @@ __device__ __forceinline__ uint32_t digit_peers(uint32_t dig) {
 // barrier); one scan per digit over the warps then gives every key its slot
 // in the tile sorted by digit, stable because index order is (warp, step,
 // lane).  The sorted tile is staged in shared memory and written out with
-// consecutive threads on consecutive slots of each digit's run.  With
-// kLookback the tile's global slots come from the one-sweep look-back
-// (tiles in ticket order), otherwise from k_sort_offsets.
-template <bool kLookback>
-__global__ void __launch_bounds__(kThreads, 4) k_sort_scatter(DevPtrs d, const unsigned long long *__restrict__ kin,
-                                                           const uint32_t *__restrict__ pin,
-                                                           unsigned long long *__restrict__ kout,
-                                                           uint32_t *__restrict__ pout, int shift, int pass,
-                                                           const int *__restrict__ tile_first) {
+// consecutive threads on consecutive slots of each digit's run.
+struct SortTile {
+    int start, n;           // the tile's first key and number of keys
+    uint32_t lo, hi;        // its segment
+    int tile, first;        // the tile and its segment's first one, numbered as their status words
+    uint32_t *stat;         // kLookback: the pass's status words
+    const uint32_t *total;  // kLookback: the segment's digit totals in this pass
+};
+struct SortShared {
+    unsigned long long key[kSortTile];
+    uint32_t pay[kSortTile];
+    uint32_t wcnt[kThreads / 32][kSortBuckets];  // per warp: keys of each digit (then: first tile slot)
+    uint32_t lbase[kSortBuckets];                // first tile slot per digit
+    uint32_t gbase[kSortBuckets];                // first global slot per digit
+    uint32_t wsum[kThreads / 32], wseg[kThreads / 32];
+    int bad;
+};
+enum SortPlace {
+    kOffsets,   // a tile's global slots are in d.shist (k_sort_offsets)
+    kLookback,  // they come from the one-sweep look-back (tiles in ticket order)
+    kAlone,     // the tile is its segment
+};
+// False: a wait ran past its bound.  kFresh: the keys were written in this launch.
+template <SortPlace kPlace, bool kFresh>
+__device__ __forceinline__ bool sort_tile(const DevPtrs &d, SortShared &sh, const SortTile &T,
+                                          const unsigned long long *__restrict__ kin, const uint32_t *__restrict__ pin,
+                                          unsigned long long *__restrict__ kout, uint32_t *__restrict__ pout, int shift) {
     constexpr int W = kThreads / 32;
     constexpr int R = kSortTile / kThreads;  // keys per lane
     static_assert(kThreads == kSortBuckets && kSortTile == W * 32 * R, "one thread per digit, 32 R keys per warp");
-    __shared__ uint32_t wcnt[W][kSortBuckets];  // per warp: keys of each digit (then: first tile slot)
-    __shared__ uint32_t lbase[kSortBuckets];    // first tile slot per digit
-    __shared__ uint32_t gbase[kSortBuckets];    // first global slot per digit
-    __shared__ uint32_t wsum[W], wseg[W];
-    __shared__ unsigned long long skey[kSortTile];
-    __shared__ uint32_t spay[kSortTile];
-    __shared__ int s_tile, s_bad;
     const int t = threadIdx.x, lane = t & 31, wid = t >> 5;
-    if (kLookback) {
-        if (t == 0) {
-            s_tile = (int)atomicAdd(&d.sseg[pass], 1u);
-            s_bad = 0;
-        }
-        __syncthreads();
-    }
-    const int tile = kLookback ? s_tile : (int)blockIdx.x;
-    const int c = d.stile_cloth[tile];
-    const int start = d.stile_start[tile];
-    const ClothDev &cd = d.cloth[c];
-    const int n = min(kSortTile, cd.t_off + cd.T - start);
-    if (!kLookback) gbase[t] = d.shist[(size_t)tile * kSortBuckets + t];
+    const int n = T.n, start = T.start;
+    auto &wcnt = sh.wcnt;
+    if (kPlace == kOffsets) sh.gbase[t] = d.shist[(size_t)T.tile * kSortBuckets + t];
+    if (kPlace == kLookback && t == 0) sh.bad = 0;
 #pragma unroll
     for (int w = 0; w < W; ++w) wcnt[w][t] = 0;
     __syncthreads();
@@ -295,8 +298,8 @@ __global__ void __launch_bounds__(kThreads, 4) k_sort_scatter(DevPtrs d, const u
     for (int r = 0; r < R; ++r) {
         const int li = wid * 32 * R + r * 32 + lane;
         const bool valid = li < n;
-        kr[r] = valid ? kin[start + li] : 0ull;
-        pr[r] = valid ? pin[start + li] : 0u;
+        kr[r] = valid ? (kFresh ? __ldcg(&kin[start + li]) : kin[start + li]) : 0ull;
+        pr[r] = valid ? (kFresh ? __ldcg(&pin[start + li]) : pin[start + li]) : 0u;
         const uint32_t dig = (uint32_t)(kr[r] >> shift) & (kSortBuckets - 1);
         const uint32_t peers = digit_peers(dig) & __ballot_sync(0xffffffffu, valid);
         const uint32_t before = valid ? wcnt[wid][dig] : 0u;
@@ -313,34 +316,31 @@ __global__ void __launch_bounds__(kThreads, 4) k_sort_scatter(DevPtrs d, const u
     for (int w = 0; w < W; ++w) tot += wcnt[w][t];
     // one-sweep: publish the tile's count of digit t, and scan the segment's
     // digit totals (the digits' first positions in the segment)
-    uint32_t *stat = nullptr;
-    int first = 0;
     uint32_t segtot = 0, segincl = 0;
-    if (kLookback) {
-        first = tile_first[c];
-        stat = d.sstat + (size_t)pass * d.nstiles * kSortBuckets;
-        cuda::atomic_ref<uint32_t, cuda::thread_scope_device>(stat[(size_t)tile * kSortBuckets + t])
-            .store((tile == first ? kStatPre : kStatAgg) | tot, cuda::memory_order_relaxed);
-        segtot = segincl = d.sseg[kSortPassesMax + ((size_t)c * kSortPassesMax + pass) * kSortBuckets + t];
+    if (kPlace == kLookback) {
+        cuda::atomic_ref<uint32_t, cuda::thread_scope_device>(T.stat[(size_t)T.tile * kSortBuckets + t])
+            .store((T.tile == T.first ? kStatPre : kStatAgg) | tot, cuda::memory_order_relaxed);
+        segtot = segincl = kFresh ? __ldcg(&T.total[t]) : T.total[t];
     }
     uint32_t incl = tot;
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
         const uint32_t v = __shfl_up_sync(0xffffffffu, incl, o);
         if (lane >= o) incl += v;
-        if (kLookback) {
+        if (kPlace == kLookback) {
             const uint32_t u = __shfl_up_sync(0xffffffffu, segincl, o);
             if (lane >= o) segincl += u;
         }
     }
     if (lane == 31) {
-        wsum[wid] = incl;
-        if (kLookback) wseg[wid] = segincl;
+        sh.wsum[wid] = incl;
+        if (kPlace == kLookback) sh.wseg[wid] = segincl;
     }
     __syncthreads();
     uint32_t run = incl - tot;
-    for (int w = 0; w < wid; ++w) run += wsum[w];
-    lbase[t] = run;
+    for (int w = 0; w < wid; ++w) run += sh.wsum[w];
+    sh.lbase[t] = run;
+    if (kPlace == kAlone) sh.gbase[t] = T.lo + run;
 #pragma unroll
     for (int w = 0; w < W; ++w) {
         const uint32_t v = wcnt[w][t];
@@ -354,11 +354,11 @@ __global__ void __launch_bounds__(kThreads, 4) k_sort_scatter(DevPtrs d, const u
         if (li < n) {
             const uint32_t dig = (uint32_t)(kr[r] >> shift) & (kSortBuckets - 1);
             const uint32_t pos = wcnt[wid][dig] + rk[r];
-            skey[pos] = kr[r];
-            spay[pos] = pr[r];
+            sh.key[pos] = kr[r];
+            sh.pay[pos] = pr[r];
         }
     }
-    if (kLookback) {
+    if (kPlace == kLookback) {
         // the tile's place among the segment's earlier tiles, digit t: sum
         // the aggregates back to the first inclusive prefix
         // A window of kLookbackWindow earlier tiles is read at once (the
@@ -366,22 +366,22 @@ __global__ void __launch_bounds__(kThreads, 4) k_sort_scatter(DevPtrs d, const u
         // walk never passes it); a window that meets an unpublished tile
         // resumes there.
         uint32_t excl = 0;
-        if (tile != first) {
+        if (T.tile != T.first) {
             uint32_t spins = 0;
-            for (int j = tile - 1;;) {
+            for (int j = T.tile - 1;;) {
                 uint32_t sv[kLookbackWindow];
 #pragma unroll
                 for (int k = 0; k < kLookbackWindow; ++k)
-                    sv[k] = j - k >= first ? cuda::atomic_ref<uint32_t, cuda::thread_scope_device>(
-                                                 stat[(size_t)(j - k) * kSortBuckets + t])
-                                                 .load(cuda::memory_order_relaxed)
-                                           : kStatPre;
+                    sv[k] = j - k >= T.first ? cuda::atomic_ref<uint32_t, cuda::thread_scope_device>(
+                                                   T.stat[(size_t)(j - k) * kSortBuckets + t])
+                                                   .load(cuda::memory_order_relaxed)
+                                             : kStatPre;
                 bool done = false;
                 int k = 0;
                 for (; k < kLookbackWindow; ++k) {
                     if (sv[k] == 0) break;  // not published yet
                     excl += sv[k] & kStatCount;
-                    if ((sv[k] & ~kStatCount) == kStatPre || j - k == first) {
+                    if ((sv[k] & ~kStatCount) == kStatPre || j - k == T.first) {
                         done = true;
                         break;
                     }
@@ -390,7 +390,7 @@ __global__ void __launch_bounds__(kThreads, 4) k_sort_scatter(DevPtrs d, const u
                 j -= k;
                 if (k == 0) {
                     if (++spins > kLookbackSpins) {
-                        s_bad = 1;
+                        sh.bad = 1;
                         atomicOr(d.err, ERR_SORT);
                         break;
                     }
@@ -398,27 +398,55 @@ __global__ void __launch_bounds__(kThreads, 4) k_sort_scatter(DevPtrs d, const u
                 }
             }
             // published even after a failed wait, so that later tiles end
-            cuda::atomic_ref<uint32_t, cuda::thread_scope_device>(stat[(size_t)tile * kSortBuckets + t])
+            cuda::atomic_ref<uint32_t, cuda::thread_scope_device>(T.stat[(size_t)T.tile * kSortBuckets + t])
                 .store(kStatPre | (excl + tot), cuda::memory_order_relaxed);
         }
         uint32_t dbase = segincl - segtot;
-        for (int w = 0; w < wid; ++w) dbase += wseg[w];
-        gbase[t] = (uint32_t)cd.t_off + dbase + excl;
+        for (int w = 0; w < wid; ++w) dbase += sh.wseg[w];
+        sh.gbase[t] = T.lo + dbase + excl;
     }
     __syncthreads();
-    if (kLookback && s_bad) return;
-    const uint32_t lo = (uint32_t)cd.t_off, hi = (uint32_t)(cd.t_off + cd.T);
+    if (kPlace == kLookback && sh.bad) return false;
     for (int i = t; i < n; i += kThreads) {
-        const unsigned long long key = skey[i];
+        const unsigned long long key = sh.key[i];
         const uint32_t dig = (uint32_t)(key >> shift) & (kSortBuckets - 1);
-        const uint32_t g = gbase[dig] + (uint32_t)i - lbase[dig];
-        if (kLookback && (g < lo || g >= hi)) {  // only after a failed wait elsewhere
+        const uint32_t g = sh.gbase[dig] + (uint32_t)i - sh.lbase[dig];
+        if (kPlace == kLookback && (g < T.lo || g >= T.hi)) {  // only after a failed wait elsewhere
             atomicOr(d.err, ERR_SORT);
             continue;
         }
         kout[g] = key;
-        pout[g] = spay[i];
+        pout[g] = sh.pay[i];
     }
+    return true;
+}
+
+template <SortPlace kPlace>
+__global__ void __launch_bounds__(kThreads, 4) k_sort_scatter(DevPtrs d, const unsigned long long *__restrict__ kin,
+                                                           const uint32_t *__restrict__ pin,
+                                                           unsigned long long *__restrict__ kout,
+                                                           uint32_t *__restrict__ pout, int shift, int pass,
+                                                           const int *__restrict__ tile_first) {
+    __shared__ SortShared sh;
+    __shared__ int s_tile;
+    if (kPlace == kLookback) {
+        if (threadIdx.x == 0) s_tile = (int)atomicAdd(&d.sseg[pass], 1u);
+        __syncthreads();
+    }
+    SortTile T;
+    T.tile = kPlace == kLookback ? s_tile : (int)blockIdx.x;
+    const int c = d.stile_cloth[T.tile];
+    const ClothDev &cd = d.cloth[c];
+    T.start = d.stile_start[T.tile];
+    T.n = min(kSortTile, cd.t_off + cd.T - T.start);
+    T.lo = (uint32_t)cd.t_off;
+    T.hi = (uint32_t)(cd.t_off + cd.T);
+    if (kPlace == kLookback) {
+        T.first = tile_first[c];
+        T.stat = d.sstat + (size_t)pass * d.nstiles * kSortBuckets;
+        T.total = d.sseg + kSortHead + ((size_t)c * kSortPassesMax + pass) * kSortBuckets;
+    }
+    sort_tile<kPlace, false>(d, sh, T, kin, pin, kout, pout, shift);
 }
 
 // ---------------------------------------------------------------------------
@@ -427,104 +455,12 @@ __global__ void __launch_bounds__(kThreads, 4) k_sort_scatter(DevPtrs d, const u
 // passes.  Keys that share it stay in their order before the sort, in runs
 // that are almost always of one or two keys; the post-sort ranks the keys of
 // a run of at most kTieRun by (low half, position), which completes the stable
-// sort, and longer runs are radix-sorted in place by one block each before it.
-// A sort of a million keys: 8 passes and the histogram 178 us, 4 passes, the
-// long-run search and the ranks 100 us.
+// sort, and longer runs (codes clamped at the frame's faces, scenes of about a
+// millimetre) are sorted in place after it.
+// A sort of a million keys: 8 passes and the histogram 178 us, 4 passes and the
+// ranks 100 us.
 // ---------------------------------------------------------------------------
-constexpr int kTieRun = 64;
 __device__ __forceinline__ uint32_t top_half(unsigned long long k) { return (uint32_t)(k >> 32); }
-
-// Stable sort of the keys [a, e) (with payload) by their low half, one block,
-// 8-bit digits, through the other buffer; the result is where it started.
-__device__ void sort_run(unsigned long long *k0, uint32_t *p0, unsigned long long *k1, uint32_t *p1, int a, int e) {
-    __shared__ uint32_t hist[kSortBuckets], base[kSortBuckets], wcnt[kThreads / 32][kSortBuckets], wsum[kThreads / 32];
-    static_assert(kThreads == kSortBuckets, "one thread per digit");
-    const int t = threadIdx.x, lane = t & 31, wid = t >> 5;
-    for (int p = 0; p < 4; ++p) {
-        const int shift = p * kSortBits;
-        __syncthreads();
-        hist[t] = 0;
-        __syncthreads();
-        for (int i = a + t; i < e; i += kThreads) atomicAdd(&hist[(uint32_t)(k0[i] >> shift) & (kSortBuckets - 1)], 1u);
-        __syncthreads();
-        uint32_t incl = hist[t];
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            const uint32_t v = __shfl_up_sync(0xffffffffu, incl, o);
-            if (lane >= o) incl += v;
-        }
-        if (lane == 31) wsum[wid] = incl;
-        __syncthreads();
-        uint32_t run = (uint32_t)a + incl - hist[t];
-        for (int w = 0; w < wid; ++w) run += wsum[w];
-        base[t] = run;
-        for (int i0 = a; i0 < e; i0 += kThreads) {  // tiles in order: index order is (warp, lane)
-#pragma unroll
-            for (int w = 0; w < kThreads / 32; ++w) wcnt[w][t] = 0;
-            __syncthreads();
-            const int i = i0 + t;
-            const bool valid = i < e;
-            const unsigned long long key = valid ? k0[i] : 0ull;
-            const uint32_t dig = valid ? (uint32_t)(key >> shift) & (kSortBuckets - 1) : kSortBuckets;
-            const uint32_t peers = __match_any_sync(0xffffffffu, dig);
-            const uint32_t rank = __popc(peers & ((1u << lane) - 1u));
-            if (valid && rank == 0) wcnt[wid][dig] = __popc(peers);
-            __syncthreads();
-            uint32_t b = base[t];
-#pragma unroll
-            for (int w = 0; w < kThreads / 32; ++w) {
-                const uint32_t c = wcnt[w][t];
-                wcnt[w][t] = b;
-                b += c;
-            }
-            base[t] = b;
-            __syncthreads();
-            if (valid) {
-                const uint32_t o = wcnt[wid][dig] + rank;
-                k1[o] = key;
-                p1[o] = p0[i];
-            }
-            __syncthreads();
-        }
-        unsigned long long *tk = k0; k0 = k1; k1 = tk;
-        uint32_t *tp = p0; p0 = p1; p1 = tp;
-    }
-    __syncthreads();
-}
-
-// Runs longer than kTieRun: the thread of a run's first slot finds it, its
-// block sorts it unless it is in order already (equal codes are).
-__global__ void __launch_bounds__(kThreads) k_sort_long_runs(DevPtrs d) {
-    __shared__ int q_first[kThreads], q_end[kThreads], s_n;
-    const int s = blockIdx.x * kThreads + threadIdx.x;
-    if (threadIdx.x == 0) s_n = 0;
-    __syncthreads();
-    if (s < d.Ttot) {
-        const ClothDev &cd = d.cloth[d.tcloth[s]];
-        const int end = cd.t_off + cd.T;
-        if (s + kTieRun < end) {
-            const uint32_t top = top_half(d.keys_alt[s]);
-            if (top_half(d.keys_alt[s + kTieRun]) == top && (s == cd.t_off || top_half(d.keys_alt[s - 1]) != top)) {
-                int lo = s + kTieRun, hi = end;  // keys [s, lo] have this top half, hi has not (or is the end)
-                while (hi - lo > 1) {
-                    const int m = lo + (hi - lo) / 2;
-                    if (top_half(d.keys_alt[m]) == top) lo = m;
-                    else hi = m;
-                }
-                const int k = atomicAdd(&s_n, 1);
-                q_first[k] = s;
-                q_end[k] = hi;
-            }
-        }
-    }
-    __syncthreads();
-    for (int k = 0; k < s_n; ++k) {
-        const int a = q_first[k], e = q_end[k];
-        bool wrong = false;
-        for (int i = a + threadIdx.x; i + 1 < e; i += kThreads) wrong = wrong || d.keys_alt[i] > d.keys_alt[i + 1];
-        if (__syncthreads_or(wrong)) sort_run(d.keys_alt, d.payload_alt, d.keys, d.payload, a, e);
-    }
-}
 
 // A sorted slot's outputs: key, triangle order and record, (fixed mode) the
 // leaf box, and no parents yet.
@@ -543,18 +479,19 @@ __device__ __forceinline__ void put_slot(const DevPtrs &d, const ClothDev &cd, i
 }
 
 // The final place of slot s's key in its run of equal top halves (keys in
-// [first, end), sorted by top half), and whether three equal keys meet in it.
+// [first, end), sorted by top half), and whether three equal keys meet in it;
+// -1 in a run of more than kTieRun.
 template <class Keys>
 __device__ __forceinline__ int tie_place(const Keys &keys, int s, int first, int end, unsigned long long key,
                                          bool &three) {
     const uint32_t top = top_half(key);
+    if ((s + kTieRun < end && top_half(keys[s + kTieRun]) == top) ||
+        (s - kTieRun >= first && top_half(keys[s - kTieRun]) == top))
+        return -1;
     int a = s, e = s + 1;
     while (a > first && s - a < kTieRun && top_half(keys[a - 1]) == top) --a;
     while (e < end && e - s <= kTieRun && top_half(keys[e]) == top) ++e;
-    if (e - a > kTieRun) {  // sorted in place already
-        three = s > first && s + 1 < end && keys[s - 1] == key && keys[s + 1] == key;
-        return s;
-    }
+    if (e - a > kTieRun) return -1;
     int r = a, same = 0;
     for (int j = a; j < e; ++j) {
         const unsigned long long q = keys[j];
@@ -567,20 +504,231 @@ __device__ __forceinline__ int tie_place(const Keys &keys, int s, int first, int
 
 // After the sort: the low halves (halves != 0), the new triangle order and the
 // cloths in which three equal codes meet (their hierarchy may be malformed).
-__global__ void k_post_sort(DevPtrs d, int halves) {
-    const int s = blockIdx.x * blockDim.x + threadIdx.x;
-    if (s >= d.Ttot) return;
-    const int c = d.tcloth[s];
+// Runs longer than kTieRun are left, by the thread of their first slot, to
+// k_sort_long_runs.
+__global__ void __launch_bounds__(kThreads) k_post_sort(DevPtrs d, int halves) {
+    __shared__ int q_first[kThreads / kTieRun + 1], q_end[kThreads / kTieRun + 1], s_n, s_at, s_tile;
+    const int s = blockIdx.x * kThreads + threadIdx.x;
+    bool starts = false;  // a longer run
+    int end = 0;
+    uint32_t top = 0;
+    if (s < d.Ttot) {
+        const int c = d.tcloth[s];
+        const ClothDev &cd = d.cloth[c];
+        const int first = cd.t_off;
+        end = cd.t_off + cd.T;
+        const unsigned long long key = d.keys_alt[s];
+        const unsigned long long prev = s > first ? d.keys_alt[s - 1] : ~key, next = s + 1 < end ? d.keys_alt[s + 1] : ~key;
+        int place = s;
+        bool three = prev == key && next == key;
+        top = top_half(key);
+        if (halves && (top_half(prev) == top || top_half(next) == top))
+            place = tie_place(d.keys_alt, s, first, end, key, three);
+        if (place >= 0) {
+            if (three && d.eq3) d.eq3[c] = 1;
+            put_slot(d, cd, place, key, d.payload_alt[s]);
+        } else {
+            starts = top_half(prev) != top;
+        }
+    }
+    if (threadIdx.x == 0) s_n = 0;
+    if (!halves || !__syncthreads_or(starts)) return;
+    if (starts) {
+        int lo = s + kTieRun, hi = end;  // keys [s, lo] have this top half, hi has not (or is the end)
+        while (hi - lo > 1) {
+            const int m = lo + (hi - lo) / 2;
+            if (top_half(d.keys_alt[m]) == top) lo = m;
+            else hi = m;
+        }
+        const int k = atomicAdd(&s_n, 1);
+        q_first[k] = s;
+        q_end[k] = hi;
+    }
+    __syncthreads();
+    for (int k = 0; k < s_n; ++k) {
+        const int n = q_end[k] - q_first[k], nt = (n + kSortTile - 1) / kSortTile;
+        if (threadIdx.x == 0) {
+            s_at = (int)atomicAdd(&d.sseg[nt > 1 ? kRunsTiled : kRunsSmall], 1u);
+            if (nt > 1) s_tile = (int)atomicAdd(&d.sseg[kRunsTiles], (uint32_t)nt);
+        }
+        __syncthreads();
+        if (nt == 1) {
+            if (threadIdx.x == 0) d.run_small[s_at] = make_int2(q_first[k], q_end[k]);
+        } else {
+            if (threadIdx.x == 0) d.run_tiled[s_at] = make_int4(q_first[k], q_end[k], s_tile, 0);
+            for (int i = threadIdx.x; i < nt; i += kThreads) d.run_of_tile[s_tile + i] = s_at;
+            for (int i = threadIdx.x; i < 4 * kSortBuckets; i += kThreads)
+                d.run_total[(size_t)s_at * 4 * kSortBuckets + i] = 0;
+        }
+        __syncthreads();
+    }
+}
+
+// The outputs of the sorted run r's slots [a, e), by one block.
+__device__ __forceinline__ void put_run(const DevPtrs &d, int first, int end, int a, int e) {
+    const int c = d.tcloth[first];
     const ClothDev &cd = d.cloth[c];
-    const int first = cd.t_off, end = cd.t_off + cd.T;
-    const unsigned long long key = d.keys_alt[s];
-    const unsigned long long prev = s > first ? d.keys_alt[s - 1] : ~key, next = s + 1 < end ? d.keys_alt[s + 1] : ~key;
-    int place = s;
-    bool three = prev == key && next == key;
-    if (halves && (top_half(prev) == top_half(key) || top_half(next) == top_half(key)))
-        place = tie_place(d.keys_alt, s, first, end, key, three);
-    if (three && d.eq3) d.eq3[c] = 1;
-    put_slot(d, cd, place, key, d.payload_alt[s]);
+    for (int s = a + threadIdx.x; s < e; s += kThreads) {
+        const unsigned long long key = __ldcg(&d.keys_alt[s]);
+        if (s > first && s + 1 < end && __ldcg(&d.keys_alt[s - 1]) == key && __ldcg(&d.keys_alt[s + 1]) == key && d.eq3)
+            d.eq3[c] = 1;
+        put_slot(d, cd, s, key, __ldcg(&d.payload_alt[s]));
+    }
+}
+
+// The long runs sorted by their low halves, in place.  Work items are taken by
+// ticket: every tile's digit counts of the runs of several tiles (and whether
+// the run is in order already, as equal codes are); their four passes, tile by
+// tile, with the one-sweep's look-back within the run; their outputs; then the
+// runs of one tile.  An item of a pass waits until every item before it is done.
+// It waits on smaller tickets only, which blocks that run hold, and the
+// smallest one in work waits for nothing: the wait ends without the blocks
+// having to be resident together, and it is bounded all the same.
+// Runs of up to kRankRun keys are ranked by counting in shared memory.
+// So the sort's time is bounded by its passes, whatever the codes.  Bound by the
+// passes, as they are by ranking; with few runs, by the chain of items.  A
+// million boxes' build (ms) with one block per run / so: spread over the cube
+// 0.271 / 0.271, in one cell of the top half 17.3 / 0.36, two codes in turn
+// 10.1 / 0.40, half of each axis clamped 1.83 / 0.42, runs of 300 0.40 / 0.35,
+// a 1 m cloth around the origin 0.44 / 0.40.
+constexpr int kRankRun = 512;
+constexpr int kRunBlocks = 608;  // four on each of 152 SMs
+__global__ void __launch_bounds__(kThreads, 4) k_sort_long_runs(DevPtrs d) {
+    __shared__ SortShared sh;
+    __shared__ uint32_t s_item;
+    __shared__ int s_ok;
+    const uint32_t nsmall = d.sseg[kRunsSmall], ntiles = d.sseg[kRunsTiles], total = nsmall + 6 * ntiles;
+    const int t = threadIdx.x, lane = t & 31;
+    bool gave_up = false;  // block-uniform: it waits no more, and its passes are left out
+    if (total == 0) return;
+    for (;;) {
+        if (t == 0) s_item = atomicAdd(&d.sseg[kRunsTicket], 1u);
+        __syncthreads();
+        const uint32_t item = s_item;
+        if (item >= total) return;
+        if (item >= 6 * ntiles) {
+            const int2 r = d.run_small[item - 6 * ntiles];
+            const int n = r.y - r.x;
+            if (n <= kRankRun) {
+                constexpr int R = kRankRun / kThreads;
+                uint32_t *low = sh.pay;
+                const uint4 *low4 = reinterpret_cast<const uint4 *>(sh.pay);
+                unsigned long long key[R];
+                uint32_t pay[R];
+#pragma unroll
+                for (int k = 0; k < R; ++k) {
+                    const int i = k * kThreads + t;
+                    key[k] = i < n ? d.keys_alt[r.x + i] : ~0ull;
+                    pay[k] = i < n ? d.payload_alt[r.x + i] : 0u;
+                    low[i] = (uint32_t)key[k];  // (past the run: above every key, or not below it)
+                }
+                __syncthreads();
+#pragma unroll
+                for (int k = 0; k < R; ++k) {
+                    const int w0 = k * kThreads + (t & ~31);  // the warp's first position
+                    if (w0 >= n) break;
+                    const uint32_t mine = (uint32_t)key[k];
+                    int place = 0, j = 0;
+                    for (; j < w0; j += 4) {  // earlier positions: equal keys come first
+                        const uint4 q = low4[j / 4];
+                        place += (q.x <= mine) + (q.y <= mine) + (q.z <= mine) + (q.w <= mine);
+                    }
+                    for (int o = 0; o < 32; ++o, ++j) place += low[j] < mine || (low[j] == mine && o < lane);
+                    for (; j < n; j += 4) {
+                        const uint4 q = low4[j / 4];
+                        place += (q.x < mine) + (q.y < mine) + (q.z < mine) + (q.w < mine);
+                    }
+                    if (w0 + lane < n) {
+                        d.keys_alt[r.x + place] = key[k];
+                        d.payload_alt[r.x + place] = pay[k];
+                    }
+                }
+            } else {
+                bool wrong = false;
+                for (int i = r.x + t; i + 1 < r.y; i += kThreads) wrong = wrong || d.keys_alt[i] > d.keys_alt[i + 1];
+                if (__syncthreads_or(wrong)) {
+                    const SortTile T{r.x, n, (uint32_t)r.x, (uint32_t)r.y, 0, 0, nullptr, nullptr};
+                    unsigned long long *k0 = d.keys_alt, *k1 = d.keys;
+                    uint32_t *p0 = d.payload_alt, *p1 = d.payload;
+#pragma unroll 1
+                    for (int p = 0; p < 4; ++p) {
+                        sort_tile<kAlone, true>(d, sh, T, k0, p0, k1, p1, p * kSortBits);
+                        __syncthreads();
+                        unsigned long long *tk = k0; k0 = k1; k1 = tk;
+                        uint32_t *tp = p0; p0 = p1; p1 = tp;
+                    }
+                }
+            }
+            __syncthreads();
+            put_run(d, r.x, r.y, r.x, r.y);
+        } else {
+            const uint32_t phase = item / ntiles;
+            const int tile = (int)(item % ntiles), run = d.run_of_tile[tile];
+            const int4 r = __ldcg(&d.run_tiled[run]);
+            const int start = r.x + (tile - r.z) * kSortTile, n = min(kSortTile, r.y - start);
+            if (phase == 0) {
+                for (int p = 0; p < 4; ++p) {
+                    sh.wcnt[p][t] = 0;
+                    d.sstat[((size_t)p * ntiles + tile) * kSortBuckets + t] = 0;
+                }
+                __syncthreads();
+                bool wrong = false;
+                for (int i0 = 0; i0 < n; i0 += kThreads) {
+                    const int i = i0 + t;
+                    const bool valid = i < n;
+                    const unsigned long long key = valid ? d.keys_alt[start + i] : 0ull;
+                    wrong = wrong || (valid && start + i + 1 < r.y && key > d.keys_alt[start + i + 1]);
+#pragma unroll
+                    for (int p = 0; p < 4; ++p) {
+                        const uint32_t dig = valid ? (uint32_t)(key >> (p * kSortBits)) & (kSortBuckets - 1) : kSortBuckets;
+                        const uint32_t d0 = __shfl_sync(0xffffffffu, dig, 0);
+                        if (__all_sync(0xffffffffu, dig == d0)) {
+                            if (lane == 0 && d0 < kSortBuckets) atomicAdd(&sh.wcnt[p][d0], 32u);
+                        } else if (valid) {
+                            atomicAdd(&sh.wcnt[p][dig], 1u);
+                        }
+                    }
+                }
+                if (__syncthreads_or(wrong) && t == 0) d.run_tiled[run].w = 1;
+                for (int p = 0; p < 4; ++p)
+                    if (sh.wcnt[p][t]) atomicAdd(&d.run_total[((size_t)run * 4 + p) * kSortBuckets + t], sh.wcnt[p][t]);
+            } else {
+                if (t == 0 && !gave_up) {
+                    cuda::atomic_ref<uint32_t, cuda::thread_scope_device> done(d.sseg[kRunsDone]);
+                    uint32_t spins = 0;
+                    s_ok = 1;
+                    while (done.load(cuda::memory_order_acquire) < phase * ntiles) {
+                        if (++spins > kLookbackSpins) {
+                            atomicOr(d.err, ERR_SORT);
+                            s_ok = 0;
+                            break;
+                        }
+                        __nanosleep(64);
+                    }
+                }
+                __syncthreads();
+                gave_up = gave_up || !s_ok;
+                if (phase == 5) {
+                    put_run(d, r.x, r.y, start, start + n);  // (also after a failed wait: every slot gets a triangle)
+                } else if (!gave_up && __ldcg(&d.run_tiled[run].w)) {
+                    const int p = (int)phase - 1;
+                    const SortTile T{start, n, (uint32_t)r.x, (uint32_t)r.y, tile, r.z,
+                                     d.sstat + (size_t)p * ntiles * kSortBuckets,
+                                     d.run_total + ((size_t)run * 4 + p) * kSortBuckets};
+                    const bool odd = p & 1;
+                    if (!sort_tile<kLookback, true>(d, sh, T, odd ? d.keys : d.keys_alt, odd ? d.payload : d.payload_alt,
+                                                    odd ? d.keys_alt : d.keys, odd ? d.payload_alt : d.payload,
+                                                    p * kSortBits))
+                        gave_up = true;
+                }
+            }
+        }
+        __syncthreads();
+        if (t == 0 && item < 5 * ntiles && !gave_up) {
+            __threadfence();
+            atomicAdd(&d.sseg[kRunsDone], 1u);
+        }
+    }
 }
 
 // Segments of at most CS R 1024 keys: sort and post-sort in one launch, one
@@ -768,6 +916,7 @@ __global__ void __launch_bounds__(kSmallThreads) k_sort_segment(DevPtrs d, int h
         bool three = prev == key[r] && next == key[r];
         if (halves && (top_half(prev) == top_half(key[r]) || top_half(next) == top_half(key[r])))
             place = tie_place(keys, i, 0, n, key[r], three);
+        if (place < 0) place = i;  // sorted by the whole key above
         if (three && d.eq3) d.eq3[c] = 1;
         put_slot(d, cd, off + place, key[r], pay[r]);
     }
@@ -2424,17 +2573,17 @@ void launch_sort(const DevPtrs &d, const int *tile_first, int shift0, int passes
     // per-pass histogram and per-segment offsets block remain for the rest.
     const bool sweep = d.sstat && d.sseg && d.Ttot <= (int64_t)kStatCount && passes <= kSortPassesMax;
     if (sweep) {
-        cudaMemsetAsync(d.sseg, 0, sizeof(uint32_t) * (kSortPassesMax + (size_t)d.C * kSortPassesMax * kSortBuckets), st);
+        cudaMemsetAsync(d.sseg, 0, sizeof(uint32_t) * (kSortHead + (size_t)d.C * kSortPassesMax * kSortBuckets), st);
         k_sort_hist_all<<<d.nstiles, kThreads, 0, st>>>(d, k0, shift0, passes);
     }
     for (int p = 0; p < passes; ++p) {
         const int shift = shift0 + p * kSortBits;
         if (sweep) {
-            k_sort_scatter<true><<<d.nstiles, kThreads, 0, st>>>(d, k0, p0, k1, p1, shift, p, tile_first);
+            k_sort_scatter<kLookback><<<d.nstiles, kThreads, 0, st>>>(d, k0, p0, k1, p1, shift, p, tile_first);
         } else {
             k_sort_hist<<<d.nstiles, kThreads, 0, st>>>(d, k0, shift);
             k_sort_offsets<<<d.C, kSortBuckets * kOffsetsSplit, 0, st>>>(d, tile_first);
-            k_sort_scatter<false><<<d.nstiles, kThreads, 0, st>>>(d, k0, p0, k1, p1, shift, p, tile_first);
+            k_sort_scatter<kOffsets><<<d.nstiles, kThreads, 0, st>>>(d, k0, p0, k1, p1, shift, p, tile_first);
         }
         std::swap(k0, k1);
         std::swap(p0, p1);
@@ -2484,9 +2633,14 @@ void launch_morton_sort(const DevPtrs &d, const int *tile_first, int mode, int m
     else if (max_T <= 8 * kSmallThreads) e = sort_segments<1, 8>(d, halves, st);
     if (e == cudaSuccess) return;
     cudaGetLastError();
+    if (halves && !d.run_small) {  // (the allocation-free entry, should the launch above fail: the whole key)
+        launch_sort(d, tile_first, 0, 8, true, st);
+        k_post_sort<<<nblk(d.Ttot), kThreads, 0, st>>>(d, 0);
+        return;
+    }
     launch_sort(d, tile_first, shift0, 4, true, st);
-    if (halves) k_sort_long_runs<<<nblk(d.Ttot), kThreads, 0, st>>>(d);
     k_post_sort<<<nblk(d.Ttot), kThreads, 0, st>>>(d, halves);
+    if (halves) k_sort_long_runs<<<kRunBlocks, kThreads, 0, st>>>(d);
 }
 // The hierarchy with its boxes and records.
 void launch_hierarchy(const DevPtrs &d, int max_T, cudaStream_t st) {
