@@ -1119,7 +1119,7 @@ static lc_status batch_build(lc_batch *b, const lc_cloth_desc *descs, int n, con
         }
         for (size_t k = 0; k < hc.b_ids.size(); ++k) {
             const int4 q = hc.b_ids[k];
-            hbids[bo + k] = make_int4(vo + q.x, vo + q.y, vo + q.z, vo + q.w);
+            hbids[bo + k] = make_int4(vo + q.x, vo + q.y, vo + q.z, cd.tri_bend ? q.w : vo + q.w);  // (rest height bits)
             hbkp[bo + k] = kpb;
         }
         for (int j = 0; j < cd.F; ++j) hfixed[cd.f_off + j] = vo + hc.fixed[j];
