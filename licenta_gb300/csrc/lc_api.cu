@@ -11,7 +11,10 @@
 #include <cstring>
 #include <memory>
 #include <numeric>
+#include <new>
 #include <string>
+#include <system_error>
+#include <thread>
 #include <unordered_map>
 #include <unordered_set>
 #include <queue>
@@ -421,7 +424,7 @@ struct lc_batch {
     lc_status setup_cluster();
     lc_status setup_global_solver();
     lc_status setup_tiles();
-    lc_status build_tiles(int target, bool &fit);
+    lc_status build_tiles(int target, std::vector<std::vector<int>> order, bool &fit);
     size_t tile_smem = 0;          // of the global-memory solver's tiles
 
     // profiling: when non-null, events are recorded at phase boundaries
@@ -613,100 +616,83 @@ lc_status lc_batch::setup_global_solver() {
     return LC_OK;
 }
 
-// The cloths cut into tiles for the global-memory solver.  Vertices per tile:
-// two tiles on an SM, as many turns of the chip as the largest tile that fits
-// asks for, evenly filled, and 64 at least (us per iteration with 64 / 128 / 216
-// / 300 / 431 vertices: 64 squared 10 / 12 / 12 / 13 / 14, 256 squared 24 / 18 /
-// 15 / 16 / 17, 512 squared 68 / 45 / 38 / 36 / 35: constraints across tiles are
-// evaluated in each).  Leaves ntiles 0 where tiles of 32 vertices do not fit.
-lc_status lc_batch::setup_tiles() {
-    for (int most = 448; most >= 32; most -= most / 8) {
-        const int slots = 2 * sm_count(), turns = (int)((d.Vtot + (int64_t)slots * most - 1) / ((int64_t)slots * most));
-        const int per = (int)((d.Vtot + (int64_t)slots * turns - 1) / ((int64_t)slots * turns));
-        bool fit = false;
-        LC_TRY(build_tiles(std::min(most, std::max(per, 64)), fit));
-        if (fit) break;
-    }
-    return LC_OK;
+// Whether a tile of n_pos positions and S entries fits half of an SM.
+static bool tile_fits(int64_t n_pos, int64_t S) {
+    return S < 0xffff && n_pos < 0xffff && sizeof(float4) * (size_t)n_pos + 3 * sizeof(float) * (size_t)S <= kSolveTileSmem;
 }
 
-// Tiles of at most `target` vertices, in Morton order of the rest positions.
-// fit: whether each tile's positions and entries fit half of an SM.
-lc_status lc_batch::build_tiles(int target, bool &fit) {
-    fit = false;
+// A cloth's vertices in Morton order of the rest positions.
+static std::vector<int> morton_vertex_order(const HostCloth &hc) {
+    const int V = hc.V;
+    constexpr float kMax = std::numeric_limits<float>::max();
+    float lo[3] = {kMax, kMax, kMax}, hi[3] = {-kMax, -kMax, -kMax};
+    for (int i = 0; i < V; ++i)
+        for (int a = 0; a < 3; ++a) {
+            lo[a] = std::min(lo[a], hc.pos[3 * i + a]);
+            hi[a] = std::max(hi[a], hc.pos[3 * i + a]);
+        }
+    float ext = 0.f;
+    for (int a = 0; a < 3; ++a) ext = std::max(ext, hi[a] - lo[a]);
+    std::vector<std::pair<uint32_t, int>> order(V), buf(V);
+    std::vector<int> digit_count(3 * 1024, 0);
+    for (int i = 0; i < V; ++i) {
+        uint32_t code = 0;
+        for (int a = 0; a < 3; ++a) {
+            const float u = ext > 0.f ? (hc.pos[3 * i + a] - lo[a]) / ext * 1023.f : 0.f;
+            uint32_t q = u > 0.f ? (uint32_t)std::min(u, 1023.f) : 0u;
+            q = (q | (q << 16)) & 0x030000ffu;  // two zeros between its bits
+            q = (q | (q << 8)) & 0x0300f00fu;
+            q = (q | (q << 4)) & 0x030c30c3u;
+            q = (q | (q << 2)) & 0x09249249u;
+            code |= q << a;
+        }
+        order[i] = {code, i};
+        for (int p = 0; p < 3; ++p) ++digit_count[1024 * p + ((code >> (10 * p)) & 1023u)];
+    }
+    for (int p = 0; p < 3; ++p) {  // by code, three passes of ten bits
+        int *at = digit_count.data() + 1024 * p, sum = 0;
+        for (int k = 0; k < 1024; ++k) sum += std::exchange(at[k], sum);
+        for (const auto &o : order) buf[at[(o.first >> (10 * p)) & 1023u]++] = o;
+        order.swap(buf);
+    }
+    std::vector<int> ids(V);
+    for (int i = 0; i < V; ++i) ids[i] = order[i].second;
+    return ids;
+}
+
+// The records of some of the tiles, by one thread; offsets count from its own arrays.
+struct TileShare {
+    struct Plan {
+        int cloth, v0, n, row, entries;  // vertices order[cloth][v0, v0 + n), first row, entries
+    };
     std::vector<SolveTile> tiles;
-    std::vector<int> vert, rows, sk, bk;
+    std::vector<int> vert, sk, bk;
     std::vector<uint2> ts;
     std::vector<uint4> tb;
-    vert.reserve(2 * (size_t)d.Vtot);
-    ts.reserve((size_t)d.Etot + d.Etot / 4);
-    sk.reserve(ts.capacity());
-    tb.reserve((size_t)d.Btot + d.Btot / 3);
-    bk.reserve(tb.capacity());
     size_t smem = 0;
-    for (int c = 0; c < C; ++c) {
-        const HostCloth &hc = hosts[c];
-        const ClothDev &cd = cds[c];
-        const int V = hc.V;
-        constexpr float kMax = std::numeric_limits<float>::max();
-        float lo[3] = {kMax, kMax, kMax}, hi[3] = {-kMax, -kMax, -kMax};
-        for (int i = 0; i < V; ++i)
-            for (int a = 0; a < 3; ++a) {
-                lo[a] = std::min(lo[a], hc.pos[3 * i + a]);
-                hi[a] = std::max(hi[a], hc.pos[3 * i + a]);
-            }
-        float ext = 0.f;
-        for (int a = 0; a < 3; ++a) ext = std::max(ext, hi[a] - lo[a]);
-        std::vector<std::pair<uint32_t, int>> order(V), buf(V);
-        std::vector<int> digit_count(3 * 1024, 0);
-        for (int i = 0; i < V; ++i) {
-            uint32_t code = 0;
-            for (int a = 0; a < 3; ++a) {
-                const float u = ext > 0.f ? (hc.pos[3 * i + a] - lo[a]) / ext * 1023.f : 0.f;
-                uint32_t q = u > 0.f ? (uint32_t)std::min(u, 1023.f) : 0u;
-                q = (q | (q << 16)) & 0x030000ffu;  // two zeros between its bits
-                q = (q | (q << 8)) & 0x0300f00fu;
-                q = (q | (q << 4)) & 0x030c30c3u;
-                q = (q | (q << 2)) & 0x09249249u;
-                code |= q << a;
-            }
-            order[i] = {code, i};
-            for (int p = 0; p < 3; ++p) ++digit_count[1024 * p + ((code >> (10 * p)) & 1023u)];
+    bool fit = true, out_of_memory = false;
+
+    void build(const std::vector<HostCloth> &hosts, const std::vector<ClothDev> &cds,
+               const std::vector<std::vector<int>> &order, const std::vector<int> &rows, const Plan *p, const Plan *end) try {
+        size_t V = 0, E = 0, B = 0;
+        for (const Plan *q = p; q < end; ++q) {
+            const HostCloth &hc = hosts[q->cloth];
+            V = std::max(V, (size_t)hc.V); E = std::max(E, hc.s_ids.size()); B = std::max(B, hc.b_ids.size());
         }
-        for (int p = 0; p < 3; ++p) {  // by code, three passes of ten bits
-            int *at = digit_count.data() + 1024 * p, sum = 0;
-            for (int k = 0; k < 1024; ++k) sum += std::exchange(at[k], sum);
-            for (const auto &o : order) buf[at[(o.first >> (10 * p)) & 1023u]++] = o;
-            order.swap(buf);
-        }
-        std::vector<int> rec_s(hc.s_ids.size(), -1), rec_b(hc.b_ids.size(), -1);  // a constraint's latest record
-        std::vector<int> vpos(V, -1);      // local index in the current tile
-        const int ntile = (V + target - 1) / target, per = (V + ntile - 1) / std::max(ntile, 1);
-        for (int v0 = 0; v0 < V; v0 += per) {
-            const int v1 = std::min(V, v0 + per), n_own = v1 - v0;
-            // equal degrees side by side: the rows of entries have no holes
-            std::stable_sort(order.begin() + v0, order.begin() + v1, [&](auto &x, auto &y) {
-                return hc.soff[x.second + 1] - hc.soff[x.second] > hc.soff[y.second + 1] - hc.soff[y.second];
-            });
+        std::vector<int> rec_s(E, -1), rec_b(B, -1);  // a constraint's latest record: from the current tile if past its first
+        std::vector<int> vpos(V, -1), halo;           // local index in the current tile
+        for (; p < end; ++p) {
+            const HostCloth &hc = hosts[p->cloth];
+            const ClothDev &cd = cds[p->cloth];
+            const int *own = order[p->cloth].data() + p->v0, n_own = p->n;
             SolveTile tl{};
-            tl.cloth = c; tl.n_own = n_own; tl.pos = (int)vert.size(); tl.row = (int)rows.size();
+            tl.cloth = p->cloth; tl.n_own = n_own; tl.pos = (int)vert.size(); tl.row = p->row;
             tl.s0 = (int)ts.size(); tl.b0 = (int)tb.size();
-            int S = 0;
-            for (int i = 0; i < n_own; i += 32) {
-                int deg = 0;
-                for (int k = i; k < std::min(n_own, i + 32); ++k) {
-                    const int v = order[v0 + k].second;
-                    deg = std::max(deg, hc.soff[v + 1] - hc.soff[v]);
-                }
-                rows.push_back(S);
-                S += 32 * deg;
-            }
-            rows.push_back(S);
             for (int i = 0; i < n_own; ++i) {
-                vpos[order[v0 + i].second] = i;
-                vert.push_back(order[v0 + i].second + (int)cd.v_off);
+                vpos[own[i]] = i;
+                vert.push_back(own[i] + (int)cd.v_off);
             }
-            std::vector<int> halo;
+            halo.clear();
             auto local_of = [&](int v) {
                 if (vpos[v] < 0) {
                     vpos[v] = n_own + (int)halo.size();
@@ -717,7 +703,7 @@ lc_status lc_batch::build_tiles(int target, bool &fit) {
             };
             const bool tri = cd.tri_bend;
             for (int i = 0; i < n_own; ++i) {
-                const int v = order[v0 + i].second, at0 = rows[tl.row + i / 32] + i % 32;
+                const int v = own[i], at0 = rows[tl.row + i / 32] + i % 32;
                 for (int e = hc.soff[v]; e < hc.soff[v + 1]; ++e) {
                     const uint32_t ent = hc.sent[e], k = ent & 0x1FFFFFFFu, role = (ent >> 29) & 3u;
                     const uint32_t at = (uint32_t)(at0 + 32 * (e - hc.soff[v]));
@@ -725,9 +711,9 @@ lc_status lc_batch::build_tiles(int target, bool &fit) {
                     if (ent >> 31) {
                         if (rec_b[k] < tl.b0) {
                             const int4 id = hc.b_ids[k];
-                            const uint32_t a = local_of(id.x), b = local_of(id.y), p = local_of(id.z);
+                            const uint32_t a = local_of(id.x), b = local_of(id.y), c = local_of(id.z);
                             rec_b[k] = (int)tb.size();
-                            tb.push_back(make_uint4(a | (b << 16), p | ((tri ? p : local_of(id.w)) << 16), ~0u, ~0u));
+                            tb.push_back(make_uint4(a | (b << 16), c | ((tri ? c : local_of(id.w)) << 16), ~0u, ~0u));
                             bk.push_back((int)k + (int)cd.b_off);
                         }
                         uint4 &r = tb[rec_b[k]];
@@ -746,15 +732,106 @@ lc_status lc_batch::build_tiles(int target, bool &fit) {
             }
             tl.n_pos = n_own + (int)halo.size();
             tl.s1 = (int)ts.size(); tl.b1 = (int)tb.size();
-            const size_t bytes = sizeof(float4) * (size_t)tl.n_pos + 3 * sizeof(float) * (size_t)S;
-            if (S >= 0xffff || tl.n_pos >= 0xffff || bytes > kSolveTileSmem) return LC_OK;
-            smem = std::max(smem, bytes);
+            if (!tile_fits(tl.n_pos, p->entries)) {
+                fit = false;
+                return;
+            }
+            smem = std::max(smem, sizeof(float4) * (size_t)tl.n_pos + 3 * sizeof(float) * (size_t)p->entries);
             tiles.push_back(tl);
-            for (int i = 0; i < n_own; ++i) vpos[order[v0 + i].second] = -1;
+            for (int i = 0; i < n_own; ++i) vpos[own[i]] = -1;
             for (int v : halo) vpos[v] = -1;
         }
+    } catch (const std::bad_alloc &) {
+        out_of_memory = true;
     }
-    if (tiles.empty() || !tiles_supported()) {
+};
+
+// The cloths cut into tiles for the global-memory solver.  Vertices per tile:
+// two tiles on an SM, as many turns of the chip as the largest tile that fits
+// asks for, evenly filled, and 64 at least (us per iteration with 64 / 128 / 216
+// / 300 / 431 vertices: 64 squared 10 / 12 / 12 / 13 / 14, 256 squared 24 / 18 /
+// 15 / 16 / 17, 512 squared 68 / 45 / 38 / 36 / 35: constraints across tiles are
+// evaluated in each).  Leaves ntiles 0 where tiles of 32 vertices do not fit.
+lc_status lc_batch::setup_tiles() {
+    int64_t busiest = 0;  // constraints of a vertex
+    for (const HostCloth &hc : hosts)
+        for (int i = 0; i < hc.V; ++i) busiest = std::max<int64_t>(busiest, hc.soff[i + 1] - hc.soff[i]);
+    // its row of entries alone: no tile holds it (tried at every size, a hub of 600
+    // beside a 512 x 512 cloth took creation from 105 to 805 ms)
+    if (!tile_fits(1, 32 * busiest)) return LC_OK;
+    std::vector<std::vector<int>> order(C);
+    for (int c = 0; c < C; ++c) order[c] = morton_vertex_order(hosts[c]);
+    for (int most = 448; most >= 32; most -= most / 8) {
+        const int slots = 2 * sm_count(), turns = (int)((d.Vtot + (int64_t)slots * most - 1) / ((int64_t)slots * most));
+        const int per = (int)((d.Vtot + (int64_t)slots * turns - 1) / ((int64_t)slots * turns));
+        bool fit = false;
+        LC_TRY(build_tiles(std::min(most, std::max(per, 64)), order, fit));
+        if (fit) break;
+    }
+    return LC_OK;
+}
+
+// Tiles of at most `target` vertices, consecutive in `order`.  fit: whether each
+// tile's positions and entries fit half of an SM.  The records are made by
+// several threads, each a share of the tiles (creating a 512 x 512 cloth 136 ms
+// with one thread, 115 so, 104 without tiles; a 724 x 724 one 279, 226 and 205).
+lc_status lc_batch::build_tiles(int target, std::vector<std::vector<int>> order, bool &fit) {
+    fit = false;
+    std::vector<TileShare::Plan> plan;
+    std::vector<int> rows, sorted, first;
+    for (int c = 0; c < C; ++c) {
+        const HostCloth &hc = hosts[c];
+        const int ntile = (hc.V + target - 1) / target, per = (hc.V + ntile - 1) / std::max(ntile, 1);
+        for (int v0 = 0; v0 < hc.V; v0 += per) {
+            const int n = std::min(hc.V, v0 + per) - v0;
+            int *v = order[c].data() + v0;
+            auto degree = [&](int i) { return hc.soff[v[i] + 1] - hc.soff[v[i]]; };
+            // equal degrees side by side, the largest first: the rows of entries have no holes
+            int most = 0;
+            for (int i = 0; i < n; ++i) most = std::max(most, degree(i));
+            first.assign(most + 2, 0);
+            for (int i = 0; i < n; ++i) ++first[most - degree(i) + 1];
+            for (int k = 0; k <= most; ++k) first[k + 1] += first[k];
+            sorted.resize(n);
+            for (int i = 0; i < n; ++i) sorted[first[most - degree(i)]++] = v[i];
+            std::copy(sorted.begin(), sorted.end(), v);
+            const int row = (int)rows.size();
+            int S = 0;
+            for (int i = 0; i < n; i += 32) {
+                rows.push_back(S);
+                S += 32 * degree(i);
+            }
+            rows.push_back(S);
+            if (!tile_fits(n, S)) return LC_OK;
+            plan.push_back({c, v0, n, row, S});
+        }
+    }
+    if (plan.empty()) return LC_OK;
+    const int most = (int)std::min<size_t>({8, std::max(1u, std::thread::hardware_concurrency()), plan.size() / 64 + 1});
+    std::vector<TileShare> shares(most);
+    std::vector<std::thread> threads;
+    threads.reserve(most);
+    for (int k = 0; k < most; ++k) {
+        const size_t p0 = plan.size() * k / most, p1 = plan.size() * (k + 1) / most;
+        auto work = [&, k, p0, p1] { shares[k].build(hosts, cds, order, rows, plan.data() + p0, plan.data() + p1); };
+        if (k + 1 < most) {
+            try {
+                threads.emplace_back(work);
+                continue;
+            } catch (const std::system_error &) {  // no thread to be had: this one does it
+            }
+        }
+        work();
+    }
+    for (std::thread &t : threads) t.join();
+    size_t nv = 0, ns = 0, nb = 0, nt = 0, smem = 0;
+    for (const TileShare &q : shares) {
+        if (q.out_of_memory) return fail(LC_ERR_OOM, "tiles of the global-memory solver: host memory");
+        if (!q.fit) return LC_OK;
+        nt += q.tiles.size(); nv += q.vert.size(); ns += q.ts.size(); nb += q.tb.size();
+        smem = std::max(smem, q.smem);
+    }
+    if (!tiles_supported()) {
         cudaGetLastError();
         return LC_OK;
     }
@@ -762,14 +839,25 @@ lc_status lc_batch::build_tiles(int target, bool &fit) {
     int *dv, *dr, *dsk, *dbk;
     uint2 *dts;
     uint4 *dtb;
-    LC_TRY(arena.alloc(dt, tiles.size(), "tiles")); LC_TRY(arena.alloc(dv, vert.size(), "tile vertices"));
+    LC_TRY(arena.alloc(dt, nt, "tiles")); LC_TRY(arena.alloc(dv, nv, "tile vertices"));
     LC_TRY(arena.alloc(dr, rows.size(), "tile rows"));
-    LC_TRY(arena.alloc(dts, ts.size() + 1, "tile stretch")); LC_TRY(arena.alloc(dtb, tb.size() + 1, "tile bends"));
-    LC_TRY(arena.alloc(dsk, sk.size() + 1, "tile stretch ids")); LC_TRY(arena.alloc(dbk, bk.size() + 1, "tile bend ids"));
-    LC_TRY(upload(dt, tiles)); LC_TRY(upload(dv, vert)); LC_TRY(upload(dr, rows));
-    LC_TRY(upload(dts, ts)); LC_TRY(upload(dtb, tb)); LC_TRY(upload(dsk, sk)); LC_TRY(upload(dbk, bk));
+    LC_TRY(arena.alloc(dts, ns + 1, "tile stretch")); LC_TRY(arena.alloc(dtb, nb + 1, "tile bends"));
+    LC_TRY(arena.alloc(dsk, ns + 1, "tile stretch ids")); LC_TRY(arena.alloc(dbk, nb + 1, "tile bend ids"));
+    LC_TRY(upload(dr, rows));
+    nt = nv = ns = nb = 0;
+    for (TileShare &q : shares) {
+        for (SolveTile &t : q.tiles) {
+            t.pos += (int)nv;
+            t.s0 += (int)ns; t.s1 += (int)ns;
+            t.b0 += (int)nb; t.b1 += (int)nb;
+        }
+        LC_TRY(upload(dt + nt, q.tiles)); LC_TRY(upload(dv + nv, q.vert));
+        LC_TRY(upload(dts + ns, q.ts)); LC_TRY(upload(dtb + nb, q.tb));
+        LC_TRY(upload(dsk + ns, q.sk)); LC_TRY(upload(dbk + nb, q.bk));
+        nt += q.tiles.size(); nv += q.vert.size(); ns += q.ts.size(); nb += q.tb.size();
+    }
     d.tile = dt; d.tile_vert = dv; d.tile_row = dr; d.tile_s = dts; d.tile_b = dtb; d.tile_sk = dsk; d.tile_bk = dbk;
-    d.ntiles = (int)tiles.size();
+    d.ntiles = (int)nt;
     tile_smem = smem;
     fit = true;
     return LC_OK;
