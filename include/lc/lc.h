@@ -361,8 +361,8 @@ lc_status lc_batch_set_tuning(lc_batch *b, const lc_tuning *t);
  * the batch's current state (saved on entry, restored before every candidate
  * and on return); the fastest is applied.  Combinations that differ only in a
  * value the chosen solver does not read (the Jacobi block of the on-chip
- * solvers, the cluster size of the global-memory one, the contact mode of
- * solvers other than 3) are timed once.  allow_variants = 0 keeps the batch's
+ * solvers and of the global-memory one's tiles, the cluster size of the
+ * global-memory one, the contact mode of solvers other than 3) are timed once.  allow_variants = 0 keeps the batch's
  * solver variant (block, grid and cluster sizes never change results; the
  * variant sums corrections in another order).  NULL space takes
  * lc_default_autotune_space.  The winner goes to *best with its time per

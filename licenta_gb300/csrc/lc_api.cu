@@ -1697,6 +1697,7 @@ lc_status lc_batch_autotune(lc_batch *b, const lc_autotune_space *space_in, int3
     LC_TRY(lc_batch_sync(b));
     LC_TRY(lc_batch_save_state(b, state, st));
     int32_t n = 0;
+    int jacobi_taken = -1;  // the first Jacobi block that the global-memory solver took
     float best_t = 0.f;
     lc_tuning best_cfg = original;
     for (int i0 = 0; i0 < sp.n_traverse_block; ++i0)
@@ -1712,15 +1713,18 @@ lc_status lc_batch_autotune(lc_batch *b, const lc_autotune_space *space_in, int3
         c.solver_variant = sp.solver_variant[i3];
         c.cluster_size = sp.cluster_size[i4];
         c.contact_gather = sp.contact_gather[i5];
-        // the Jacobi block matters only to the global-memory solver, the
-        // cluster size only to the on-chip ones, the contact mode only to the
-        // scatter solver: other combinations would time the same launch twice
+        // the Jacobi block matters only to the global-memory solver without
+        // tiles, the cluster size only to the on-chip ones, the contact mode
+        // only to the scatter solver: other combinations would time the same
+        // launch twice
         if (c.solver_variant != 1 && i1 != 0) continue;
+        if (c.solver_variant == 1 && b->d.ntiles && jacobi_taken >= 0 && i1 != jacobi_taken) continue;
         if (c.solver_variant == 1 && i4 != 0) continue;
         if (c.solver_variant == 1) c.cluster_size = 0;
         if (c.solver_variant != 3 && i5 != 0) continue;
         if (c.solver_variant != 3) c.contact_gather = 0;
         if (lc_batch_set_tuning(b, &c) != LC_OK) continue;  // a shape the batch cannot take
+        if (c.solver_variant == 1 && jacobi_taken < 0) jacobi_taken = i1;
         LC_TRY(lc_batch_load_state(b, state, st));
         LC_TRY(lc_batch_step(b, warmup, st));
         LC_CUDA(cudaEventRecord(e0, st));
