@@ -455,9 +455,11 @@ lc_status lc_lbvh_destroy(lc_lbvh *h);
  * SpatialHashing, Collision/BVH.cpp etc.), which run on the CPU over SceneObjects.
  * Here an object is its axis-aligned box, and lc_broadphase_update (the
  * interface's Update) takes all boxes at once: box_min / box_max, 3 floats per
- * object, in device memory, which must stay valid until the
- * lc_broadphase_test that follows (TestCollision) has returned.  Every method
- * returns the same set, all pairs (a, b), a < b, of objects whose closed boxes
+ * object, in device memory, which must stay valid and as they are until the
+ * lc_broadphase_test that follows (TestCollision) has returned: what a method
+ * keeps of them is from the update (sweep and prune all of them, the BVH its
+ * hierarchy), the others read them at the test.  Every method returns the same
+ * set, all pairs (a, b), a < b, of objects whose closed boxes
  * overlap (BoundingBox::Collides), with nothing dropped; the methods differ in
  * the work they do:
  *   LC_BP_BRUTE every pair;

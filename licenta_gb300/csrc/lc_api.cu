@@ -311,9 +311,9 @@ static lc_status build_host_cloth(const lc_cloth_desc &d, HostCloth &hc) {
         if (s_ != LC_OK) return s_;   \
     } while (0)
 
-// Device arrays of one handle.  Small ones share blocks of 2 MB, which is what
-// the driver maps for any small one by itself: a handle has up to a hundred, at
-// two microseconds or more a call (creating a 32 x 32 cloth 1.16 ms, 1.00 so).
+// Device arrays of one handle.  Small ones share blocks of 2 MB, the size CUDA
+// maps for a small one by itself: a handle has up to a hundred, at two
+// microseconds or more a call (creating a 32 x 32 cloth 1.16 ms, 1.00 so).
 struct DeviceArena {
     static constexpr size_t kBlock = 2 << 20, kSmall = 256 << 10;
     std::vector<void *> ptrs;
@@ -987,6 +987,8 @@ static lc_status alloc_range_tree(lc_batch *b, int64_t T, int C) {
 }
 
 // The sort's scratch for C segments of T keys in all, cut into `tiles` tiles.
+// (No per-pass histograms: a handle of 2^30 keys, from which they would be
+// needed, takes more than the device's memory.)
 static lc_status alloc_sort(lc_batch *b, int64_t T, int C, int64_t tiles) {
     DevPtrs &d = b->d;
     DeviceArena &A = b->arena;

@@ -106,7 +106,6 @@ struct ClothState {
     unsigned long long rng;
 };
 
-// Everything a step kernel may need, passed by value.
 // Global-memory solver: a tile of one cloth's vertices and the constraints that
 // touch them.  Local vertices: the tile's own first, then the others its
 // constraints read; own vertex i's correction entry j is rows[i / 32] + 32 j +
@@ -120,6 +119,7 @@ struct SolveTile {
 constexpr int kSolveTileThreads = 512;
 constexpr size_t kSolveTileSmem = 112 * 1024;  // positions and entries: two tiles on an SM
 
+// Everything a step kernel may need, passed by value.
 struct DevPtrs {
     int C;                 // cloths
     int Vtot, Ttot, Ntot, Itot;

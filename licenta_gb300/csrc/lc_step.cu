@@ -358,7 +358,8 @@ __global__ void k_sphere(DevPtrs d) {
 // a vertex sums its entries in order, adds the terms that are its own and the
 // contacts, and writes its update to xb.  Bound by instructions, two thirds of
 // them the bends', and by the wait for positions and records at a block's
-// start.  Us per iteration, 32, 128, 256, 512 and 724 squared vertices:
+// start.  Us per iteration, launch to launch in a step (a launch of tiles alone
+// takes 32 at 512 squared), 32, 128, 256, 512 and 724 squared vertices:
 //   18 constraints evaluated at each vertex           26, 26, 33, 76, 147
 //   once each, shared through memory (two launches)   17, 18, 25, 61, 122
 //   tiles                                             10, 12, 15, 35, 70
