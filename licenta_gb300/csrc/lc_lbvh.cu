@@ -854,6 +854,7 @@ __global__ void __launch_bounds__(kSmallThreads) k_sort_segment(DevPtrs d, int h
 #pragma unroll
     for (int r = 0; r < R; ++r) w[r] = first + place_of(r) < n ? word(first + place_of(r), halves != 0) : ~0ull;
     for (int p = 0; p < 4; ++p) pass(32 + p * kSortBits);
+    bool any = false;  // the keys are in the order of the whole code
     if (halves) {  // a long run of equal top halves: by low half first, then by top half again
         if (t == 0) s_long = 0;
         __syncthreads();
@@ -863,7 +864,7 @@ __global__ void __launch_bounds__(kSmallThreads) k_sort_segment(DevPtrs d, int h
             if (i + kTieRun / 2 < N && first + i + kTieRun / 2 < n && top_half(s_key[i]) == top_half(s_key[i + kTieRun / 2])) s_long = 1;
         }
         barrier();
-        bool any = s_long != 0;
+        any = s_long != 0;
         if (CS > 1) {
 #pragma unroll
             for (int k = 0; k < CS; ++k) {
@@ -914,9 +915,8 @@ __global__ void __launch_bounds__(kSmallThreads) k_sort_segment(DevPtrs d, int h
         const unsigned long long prev = i > 0 ? keys[i - 1] : ~key[r], next = i + 1 < n ? keys[i + 1] : ~key[r];
         int place = i;
         bool three = prev == key[r] && next == key[r];
-        if (halves && (top_half(prev) == top_half(key[r]) || top_half(next) == top_half(key[r])))
+        if (halves && !any && (top_half(prev) == top_half(key[r]) || top_half(next) == top_half(key[r])))
             place = tie_place(keys, i, 0, n, key[r], three);
-        if (place < 0) place = i;  // sorted by the whole key above
         if (three && d.eq3) d.eq3[c] = 1;
         put_slot(d, cd, off + place, key[r], pay[r]);
     }
