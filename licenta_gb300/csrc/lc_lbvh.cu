@@ -1463,17 +1463,28 @@ __global__ void k_pack_nodes(DevPtrs d) {
               d.rml[cd.i_off + k]);
 }
 
-// Climb and records of flagged cloths, a block per cloth in one launch: for
-// batches of small cloths, where the three launches above cost more than they
-// do.
-__global__ void __launch_bounds__(kRefitBlock) k_refit_block(DevPtrs d) {
-    const int c = blockIdx.x;
+// Climb and records of flagged cloths in one launch, `per` blocks per cloth, the
+// last of which to arrive writes the records: where the three launches above cost
+// more than they do.
+__global__ void __launch_bounds__(kRefitBlock) k_refit_block(DevPtrs d, int per) {
+    __shared__ int s_last;
+    const int c = blockIdx.x / per;
     if (!d.eq3[c]) return;
     const ClothDev &cd = d.cloth[c];
     const int In = cd.T - 1;
-    for (int id = threadIdx.x; id <= In && In > 0; id += kRefitBlock) refit_climb(d, cd, d.parent[cd.n_off + In + id]);
+    for (int id = (blockIdx.x % per) * kRefitBlock + threadIdx.x; id <= In && In > 0; id += per * kRefitBlock)
+        refit_climb(d, cd, d.parent[cd.n_off + In + id]);
     __threadfence();
     __syncthreads();
+    if (per > 1) {
+        if (threadIdx.x == 0) {
+            s_last = atomicAdd(&d.tree_done[c], 1) == per - 1;
+            if (s_last) d.tree_done[c] = 0;
+        }
+        __syncthreads();
+        if (!s_last) return;
+        __threadfence();
+    }
     const float4 *nmin = d.nmin + cd.n_off, *nmax = d.nmax + cd.n_off;
     for (int k = threadIdx.x; k < In; k += kRefitBlock) {
         const int2 ch = d.child[cd.i_off + k];
@@ -2663,9 +2674,13 @@ void launch_hierarchy(const DevPtrs &d, int max_T, cudaStream_t st) {
         k_karras<kThreads, kThreads><<<nblk(d.Ttot), kThreads, Any::kSmem, st>>>(d);
         k_karras_far<<<far_blocks, kThreads, 0, st>>>(d);
     }
-    // cloths in which three equal codes meet
-    if (max_T <= 4 * kSortTile) {
-        k_refit_block<<<d.C, kRefitBlock, 0, st>>>(d);
+    // Cloths in which three equal codes meet: one launch where they are small, or
+    // few of up to 8192 triangles.  A flagged cloth of 8192 (mostly clamped at the
+    // frame's faces): its one block took 180 us, the three launches 54 and 5 more
+    // for every other cloth, eight blocks 58 and none.
+    if (max_T <= kSortTile || (max_T <= 4 * kSortTile && d.C <= kSmallCtas)) {
+        const int per = max_T <= kSortTile ? 1 : 8;
+        k_refit_block<<<per * d.C, kRefitBlock, 0, st>>>(d, per);
         return;
     }
     // the upper pass: a grid-stride loop over the arrivals left, sized to be

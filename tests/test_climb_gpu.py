@@ -94,3 +94,52 @@ def test_more_than_a_million_leaves(cuda, n):
     assert np.array_equal(box[:n - 1, 3:], np.maximum(box[left, 3:], box[right, 3:]))
     ids = np.arange(n - 1)
     assert np.array_equal(par[left], ids) and np.array_equal(par[right], ids) and par[0] == -1
+
+
+@pytest.mark.parametrize("kind", ["triples", "few", "clamped"])
+def test_flagged_segment_of_one_launch(cuda, kind):
+    """Up to 8192 leaves: one block per cloth, or a cluster of eight."""
+    torch = cuda
+    h = Lbvh(8192)
+    try:
+        for n in (8192, 8191, 4097, 2049, 2048, 1025, 1024, 70):
+            lo, hi = _boxes(kind, n)
+            want = lbvh_boxes(lo, hi, chunk=64, mode=_ffi.LC_MORTON_REF63)
+            tl, th = torch.from_numpy(lo).cuda(), torch.from_numpy(hi).cuda()
+            h.build(tl.data_ptr(), th.data_ptr(), n)
+            count = h.pairs(None, 0)
+            for what in ARRAYS:
+                got, exp = h.debug(what), want[what]
+                if what == "NODE_AABB":
+                    got, exp = got.view(np.uint32), exp.view(np.uint32)
+                assert got.shape == exp.shape and np.array_equal(got, exp), (n, what)
+            assert count == len(want["PAIRS"]), n
+    finally:
+        h.close()
+
+
+@pytest.mark.parametrize("count", [3, 9])
+def test_flagged_cloths_of_up_to_8192_triangles(cuda, count):
+    """Few cloths (clusters) and more (three launches), some of them clamped at the frame's faces."""
+    specs = []
+    for k in range(count):
+        s = scenes.small_cloth(seed=k, n=(64, 40, 12)[k % 3], thickness=0.1 / 64)
+        if k % 2 == 0:
+            s.params.worldMin[:] = (-2.0, -2.0, -2.0)
+            s.positions -= np.float32([0.5, 1.0, 0.9])
+        specs.append(s)
+    with ClothBatch(specs, debug_capture=True) as b:
+        for step in range(2):
+            pre = [b.get_state(c)["vn"] for c in range(count)]
+            b.step(1)
+            b.sync()
+            flagged = 0
+            for c, s in enumerate(specs):
+                m = b.debug(c, "MORTON")
+                flagged += bool((m[2:] == m[:-2]).any())
+                o32 = Oracle([s], fp64=False)
+                try:
+                    parity.check_collision(b, c, o32, pre[c], tag=f"step {step}, cloth {c}")
+                finally:
+                    o32.close()
+            assert 0 < flagged < count
